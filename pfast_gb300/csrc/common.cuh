@@ -6,11 +6,11 @@
 #include <cmath>
 
 #include "../../include/pfast_gb300.h"
+#include "exact_arith.h"
 
 namespace pfast {
 
-// The reference's "infinity" for unreached nodes (INF macro, src/T_pfsm3d.h:12-14).
-constexpr double kInf = 9999999.0;
+constexpr double kInf = kUnreached;   // exact_arith.h
 // isconv tolerance (src/T_pfsm3d.h:126, src/RT_pfsm2d.h:112).
 constexpr double kConvTol = 1e-9;
 // Default polish floor: FP64 polish corrections at or below this (seconds, or relative to
@@ -84,6 +84,7 @@ struct Spacing3 {
     // instruction runs in an FP32 kernel: w = 1/d^2, rp[a] = 1/(W - w[a]), rW = 1/W.
     float df[3], wf[3], rpf[3], rWf;
     int iso;         // dx == dy == dz
+    ExactGrid3 ex;   // constants of the plain updates
 };
 
 // Bit-pattern helpers.  For doubles >= +0 (including +inf) the IEEE bit patterns

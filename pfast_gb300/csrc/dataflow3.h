@@ -21,10 +21,12 @@
 // 0 = index - 1, 1 = index + 1.
 #pragma once
 
+#ifndef PFAST_HD
 #ifdef __CUDACC__
 #define PFAST_HD __host__ __device__ __forceinline__
 #else
 #define PFAST_HD inline
+#endif
 #endif
 
 namespace pfast {

@@ -154,6 +154,7 @@ Spacing3 make_spacing(double dx, double dy, double dz) {
     }
     s.rWf = (float)(1.0 / W);
     s.iso = (dx == dy && dy == dz) ? 1 : 0;
+    s.ex = exact_grid3(d);
     return s;
 }
 

@@ -253,6 +253,7 @@ Sweep2Args base2(const pfast_survey2d* sv) {
     a.wxf = (float)a.inv2x;
     a.wzf = (float)a.inv2z;
     a.rsumf = (float)(1.0 / (a.inv2x + a.inv2z));
+    a.ex = exact_grid2(sv->dx, sv->dz);
     a.polish_floor = kPolishFloor;
     a.wpr = (sv->nc + 31) / 32;
     return a;

@@ -1,0 +1,340 @@
+// exact_arith.h -- the plain FP64 node updates with fewer FP64 instructions and the same bits
+// (host and device code; the CPU check tests/native/exact_arith_check.cpp compiles it with g++).
+//
+// What bounds the plain sweeps is the FP64 pipe: on this part an FP64 warp instruction holds its
+// SM sub-partition for 64 cycles (measured: one warp, dependent or independent; 76 with all four
+// sub-partitions busy), and an FP64 division costs 8 to 9 such instructions, a square root 10.
+// The reference's 3D Godunov update (src/T_pfsm3d.h:99-119) holds 13 divisions by constants of the
+// grid and 2 square roots, its adjoint update (src/T_padjoint3d.h:42-71) 12 and one by a variable.
+// So
+//   * a division by a grid constant d multiplies by its reciprocal as an unevaluated sum
+//     rh + rl (rh = 1/d rounded, rl = the remainder, rounded): q = fma(x, rh, x * rl).  That is
+//     within 2^-105 relative of x / d before the last rounding, and x / d is at least
+//     2^-(54+m) relative away from every rounding boundary when the odd part of d's significand
+//     has m bits, so q is x / d correctly rounded whenever m <= 48 (Brisebarre, Muller and Raina,
+//     "Accelerating correctly rounded floating-point division when the divisor is known in
+//     advance", IEEE Trans. Comput. 53(8), 2004).  For other d one more step, r = fma(-d, q, x)
+//     and fma(r, rh, q), is correctly rounded because q is faithful (P. Markstein, "Computation
+//     of elementary functions on the IBM RISC System/6000 processor", 1990).  2 or 4
+//     instructions instead of 8 to 9.
+//   * scalings by powers of two are left out where they commute with rounding, terms the reference
+//     multiplies by +0 are not formed, and POS / NEG are taken from the sign bit.
+//   * the branch of the reference's case analysis that a node takes is predicted from FP32 copies
+//     with a margin far above every rounding error, so that a 3-neighbour node does not evaluate
+//     the 2-neighbour solution first.
+// Arguments outside the exponent range in which these identities hold take the reference's
+// expressions as they stand.
+#pragma once
+
+#include <cmath>
+#include <cstdint>
+#include <cstring>
+
+#ifndef PFAST_HD
+#ifdef __CUDACC__
+#define PFAST_HD __host__ __device__ __forceinline__
+#else
+#define PFAST_HD inline
+#endif
+#endif
+
+namespace pfast {
+
+// The reference's "infinity" for unreached nodes (INF macro, src/T_pfsm3d.h:12-14).
+constexpr double kUnreached = 9999999.0;
+
+PFAST_HD long long bits_of(double x) {
+#ifdef __CUDA_ARCH__
+    return __double_as_longlong(x);
+#else
+    long long b;
+    std::memcpy(&b, &x, sizeof(b));
+    return b;
+#endif
+}
+PFAST_HD double from_bits(long long b) {
+#ifdef __CUDA_ARCH__
+    return __longlong_as_double(b);
+#else
+    double x;
+    std::memcpy(&x, &b, sizeof(x));
+    return x;
+#endif
+}
+PFAST_HD int exponent_of(double x) { return (int)((unsigned long long)bits_of(x) >> 52) & 0x7ff; }
+PFAST_HD bool is_zero(double x) { return ((unsigned long long)bits_of(x) << 1) == 0; }
+
+// An integer that orders like the value (NaNs beyond the infinities).
+PFAST_HD long long ordered(double x) {
+    const long long b = bits_of(x);
+    return b ^ ((b >> 63) & 0x7fffffffffffffffll);
+}
+
+// A divisor known in advance.  short_: the 2-instruction form is correctly rounded.
+struct DivBy {
+    double d, rh, rl;
+    int short_, pad_;
+};
+
+// Host: the constants of a positive normal divisor (exponent well inside the double range).
+inline DivBy div_by(double d) {
+    DivBy k;
+    k.d = d;
+    k.rh = 1.0 / d;
+    k.rl = std::fma(-d, k.rh, 1.0) / d;   // the remainder 1 - d rh is exact
+    unsigned long long m = ((unsigned long long)bits_of(d) & 0xfffffffffffffull) | (1ull << 52);
+    while (!(m & 1)) m >>= 1;
+    k.short_ = m < (1ull << 48);
+    k.pad_ = 0;
+    return k;
+}
+
+// x / k.d for x = +0 or a normal x with |x / d| in the normal range (the callers check).
+PFAST_HD double div_exact(double x, const DivBy& k) {
+    double q = fma(x, k.rh, x * k.rl);
+    if (!k.short_) q = fma(fma(-k.d, q, x), k.rh, q);
+    return q;
+}
+// The same with the remainder step always (the divisor differs between the lanes of a warp).
+PFAST_HD double div_exact4(double x, double d, double rh, double rl) {
+    const double q = fma(x, rh, x * rl);
+    return fma(fma(-d, q, x), rh, q);
+}
+// A value the compiler may not compute with ahead of the branch it is used in.
+PFAST_HD double here(double x) {
+#ifdef __CUDA_ARCH__
+    asm volatile("" : "+d"(x));
+#endif
+    return x;
+}
+// x / k.d for any x: zeros keep their sign, the ends of the exponent range divide.
+PFAST_HD double div_any(double x, const DivBy& k) {
+    const int e = exponent_of(x);
+    double q = div_exact(x, k);
+    if (is_zero(x)) q = x;
+    else if ((unsigned)(e - 123) > 1800u) q = here(x) / k.d;   // |x| < 2^-900, > 2^900, inf or NaN
+    return q;
+}
+
+// Grid constants of the exact updates.
+struct ExactGrid3 {
+    DivBy axis[3];     // d of x, y, z
+    DivBy pair[3];     // d*d of the two other axes, summed: pair[a] leaves axis a out
+    DivBy all[3];      // 1/d^2 summed with axis a last (the reference adds the smallest neighbour's axis last)
+    double dd[3];      // d*d
+    double d4;         // ((d*d)*d)*d of axis x
+    int iso;           // one spacing
+    int quick;         // the spacings lie in the range the identities need
+};
+
+inline ExactGrid3 exact_grid3(const double d[3]) {
+    ExactGrid3 g;
+    std::memset(&g, 0, sizeof(g));
+    g.quick = 1;
+    for (int a = 0; a < 3; ++a) {
+        if (!(d[a] > 0x1p-60 && d[a] < 0x1p60)) g.quick = 0;
+    }
+    if (!g.quick) return g;
+    double inv2[3];
+    for (int a = 0; a < 3; ++a) {
+        g.axis[a] = div_by(d[a]);
+        g.dd[a] = d[a] * d[a];
+        inv2[a] = 1.0 / d[a] / d[a];
+    }
+    for (int a = 0; a < 3; ++a) {
+        const int p = (a + 1) % 3, q = (a + 2) % 3;
+        g.pair[a] = div_by(g.dd[p] + g.dd[q]);
+        g.all[a] = div_by((inv2[p] + inv2[q]) + inv2[a]);
+    }
+    g.d4 = g.dd[0] * d[0] * d[0];
+    g.iso = d[0] == d[1] && d[1] == d[2];
+    return g;
+}
+
+// v = 0 or |v| in [2^-200, 2^200]
+PFAST_HD bool in_range(double v) { return (unsigned)(exponent_of(v) - 823) <= 400u; }
+
+// Magnitude of a value >= +0 as FP32 (truncated; +inf and beyond give a huge finite value).
+PFAST_HD float approx32(double v) {
+    const unsigned hi = (unsigned)((unsigned long long)bits_of(v) >> 32), lo = (unsigned)bits_of(v);
+    unsigned u = 0;
+    if (hi >= (1151u << 20)) u = 0x7f000000u;
+    else if (hi >= (897u << 20)) u = ((hi - (896u << 20)) << 3) | (lo >> 29);
+#ifdef __CUDA_ARCH__
+    return __uint_as_float(u);
+#else
+    float f;
+    std::memcpy(&f, &u, sizeof(f));
+    return f;
+#endif
+}
+
+// The reference's expressions as they stand: sorted neighbour minima a >= b >= c with their
+// spacings and 1/d^2, the 1-neighbour value already found above b.
+PFAST_HD double eik3_tail_ref(double a, double b, double c, double da, double db, double dc, double ia, double ib,
+                              double ic, double s) {
+    double A = dc * dc + db * db;
+    double B = -2. * (b * dc * dc + c * db * db);
+    double C = dc * dc * b * b + db * db * c * c - db * db * dc * dc * s * s;
+    double D = B * B - 4. * A * C;
+    double q = (D >= 0) ? (-B + sqrt(D)) / 2. / A : kUnreached;
+    if (bits_of(q) <= bits_of(a)) return q;
+    A = ia + ib + ic;
+    B = -2.0 * (a / da / da + b / db / db + c / dc / dc);
+    C = a * a / da / da + b * b / db / db + c * c / dc / dc - s * s;
+    D = B * B - 4. * A * C;
+    q = (D >= 0) ? (-B + sqrt(D)) / 2. / A : kUnreached;
+    return q;
+}
+
+// The reference's 3D Godunov solution (src/T_pfsm3d.h:99-119) for neighbour minima x, y, z along
+// the axes and slowness s, bit for bit.  With S = -B/2 and D = 4 (S*S - A*C) the factors 2 and 4
+// are exact and left out.  The 2- and the 3-neighbour solution share the square root and the
+// division: per warp at most 2 + 13 + 33 + 18 FP64 instructions (one spacing of few bits),
+// where the expressions as they stand take about 185; a 3D gradient of 96 x 96 x 48 nodes and 16
+// sources spent 210 ms in its forward sweeps with those.
+template <bool ISO>
+PFAST_HD double eik3_exact(double x, double y, double z, double s, const ExactGrid3& g, const double* inv2) {
+    double a = x, b = y, c = z, t;
+    int ka = 0, kb = 1, kc = 2, k;
+    if (bits_of(b) > bits_of(a)) { t = a; a = b; b = t; k = ka; ka = kb; kb = k; }
+    if (bits_of(c) > bits_of(a)) { t = a; a = c; c = t; k = ka; ka = kc; kc = k; }
+    if (bits_of(c) > bits_of(b)) { t = b; b = c; c = t; k = kb; kb = kc; kc = k; }
+    auto pick = [](int i, double v0, double v1, double v2) { return ISO ? v0 : (i == 0 ? v0 : (i == 1 ? v1 : v2)); };
+    const double dc = pick(kc, g.axis[0].d, g.axis[1].d, g.axis[2].d);
+    double q = dc * s + c;
+    if (bits_of(q) <= bits_of(b)) return q;
+    const double db = pick(kb, g.axis[0].d, g.axis[1].d, g.axis[2].d);
+    const bool ainf = bits_of(a) >= 0x7ff0000000000000ll;
+    if (!(in_range(b) && (is_zero(c) || in_range(c)) && (ainf || in_range(a)))) {
+        const double da = pick(ka, g.axis[0].d, g.axis[1].d, g.axis[2].d);
+        return eik3_tail_ref(a, b, c, da, db, dc, pick(ka, inv2[0], inv2[1], inv2[2]),
+                             pick(kb, inv2[0], inv2[1], inv2[2]), pick(kc, inv2[0], inv2[1], inv2[2]), s);
+    }
+    // Three neighbours for certain: the 2-neighbour solution exceeds a exactly where
+    // (a-b)^2/db^2 + (a-c)^2/dc^2 < s^2.  FP32 differences of truncated copies err by at most
+    // 2^-22 a; that is held below 1 % of the 1-neighbour step, where the FP64 formulas are
+    // accurate to 1e-6 of it, and the test asks for 2 %.  Anything closer evaluates both, in the
+    // reference's order.
+    bool three;
+    {
+        const float af = approx32(a), bf = approx32(b), cf = approx32(c), sf = approx32(s);
+        const float err = af * 2.4e-7f;
+        const float fb = (af - bf) + err, fc = (af - cf) + err;
+        const float hb = ISO ? 0.0f : approx32(db), hc = approx32(dc);
+        const float stepc = hc * sf, stepb = ISO ? stepc : hb * sf;   // 1-neighbour steps along the two axes
+        const float lo = stepc < stepb ? stepc : stepb;
+        // (fb / stepb)^2 + (fc / stepc)^2 < 0.98
+        three = err <= 0.01f * lo && fb * fb * (stepc * stepc) + fc * fc * (stepb * stepb) <
+                                         0.98f * (stepb * stepb) * (stepc * stepc) && lo > 1e-8f && af < 1e8f;
+    }
+    for (;;) {
+        double S, C, A, Ah, Al;
+        if (three) {
+            auto dv = [&](double v, int i) {
+                if (ISO) return div_exact(v, g.axis[0]);
+                // the divisor's constants by axis
+                const double d = pick(i, g.axis[0].d, g.axis[1].d, g.axis[2].d);
+                const double rh = pick(i, g.axis[0].rh, g.axis[1].rh, g.axis[2].rh);
+                const double rl = pick(i, g.axis[0].rl, g.axis[1].rl, g.axis[2].rl);
+                double r = fma(v, rh, v * rl);
+                if (!(g.axis[0].short_ && g.axis[1].short_ && g.axis[2].short_)) r = fma(fma(-d, r, v), rh, r);
+                return r;
+            };
+            S = dv(dv(a, ka), ka) + dv(dv(b, kb), kb) + dv(dv(c, kc), kc);
+            C = dv(dv(a * a, ka), ka) + dv(dv(b * b, kb), kb) + dv(dv(c * c, kc), kc) - s * s;
+            A = pick(kc, g.all[0].d, g.all[1].d, g.all[2].d);
+            Ah = pick(kc, g.all[0].rh, g.all[1].rh, g.all[2].rh);
+            Al = pick(kc, g.all[0].rl, g.all[1].rl, g.all[2].rl);
+        } else {
+            const double ddc = pick(kc, g.dd[0], g.dd[1], g.dd[2]), ddb = pick(kb, g.dd[0], g.dd[1], g.dd[2]);
+            S = b * dc * dc + c * db * db;
+            C = ddc * b * b + ddb * c * c - (ISO ? g.d4 : ddb * dc * dc) * s * s;
+            A = pick(ka, g.pair[0].d, g.pair[1].d, g.pair[2].d);
+            Ah = pick(ka, g.pair[0].rh, g.pair[1].rh, g.pair[2].rh);
+            Al = pick(ka, g.pair[0].rl, g.pair[1].rl, g.pair[2].rl);
+        }
+        const double D = S * S - A * C;
+        q = (D >= 0) ? div_exact4(S + sqrt(D), A, Ah, Al) : kUnreached;
+        if (three || bits_of(q) <= bits_of(a)) return q;
+        three = true;
+    }
+}
+
+// The reference's 3D adjoint update (src/T_padjoint3d.h:42-71), bit for bit, for reached
+// traveltimes (the caller returns 0 next to an unreached one).  Per axis at most one of the two
+// POS / NEG terms of a difference pair is nonzero except at a local extremum of T, so one product
+// and no subtraction remain there.  45 to 60 FP64 instructions (spacings of few bits) instead of
+// about 150.
+PFAST_HD double pos_part(double x) { return bits_of(x) > 0 ? x : 0.0; }                  // (x + |x|) / 2
+PFAST_HD double neg_part(double x) { return bits_of(x) < 0 ? x : 0.0; }                  // (x - |x|) / 2
+// p - m with one of the two zero (any signs): no FP64 instruction unless both are nonzero or both zero.
+PFAST_HD double sub_sparse(double p, double m) {
+    const bool zp = is_zero(p), zm = is_zero(m);
+    if (zp == zm) return p - m;
+    return zm ? p : from_bits(bits_of(m) ^ (long long)0x8000000000000000ull);
+}
+// One axis: den += ..., num += ... of the reference, g.. as its POS / NEG arguments.
+PFAST_HD void adj_axis_exact(double T0, double Tp, double Tm, double Lp, double Lm, const DivBy& k, double& den,
+                             double& num) {
+    const double gp = div_any(-(Tp - T0), k), gm = div_any(-(T0 - Tm), k);
+    const double pp = pos_part(gp), nm = neg_part(gm), pm = pos_part(gm), np = neg_part(gp);
+    den = div_any(sub_sparse(pp, nm), k);
+    // pm * Lm - np * Lp
+    const bool zpm = is_zero(pm), znp = is_zero(np);
+    double n;
+    if (zpm != znp) {
+        const double co = zpm ? np : pm, L = zpm ? Lp : Lm;   // the other product is a zero
+        double v = co * L;
+        if (zpm) v = from_bits(bits_of(v) ^ (long long)0x8000000000000000ull);
+        // a zero or non-finite result depends on the other term too: the expression as it stands
+        n = is_zero(v) || exponent_of(Lp) == 0x7ff || exponent_of(Lm) == 0x7ff ? pm * Lm - np * Lp : v;
+    } else {
+        n = pm * Lm - np * Lp;
+    }
+    num = div_any(n, k);
+}
+
+
+// ------------------------------------------------------------------ 2D
+struct ExactGrid2 {
+    DivBy x, z;     // dx, dz
+    DivBy all;      // 1/dx^2 + 1/dz^2
+    int quick, pad_;
+};
+
+inline ExactGrid2 exact_grid2(double dx, double dz) {
+    ExactGrid2 g;
+    std::memset(&g, 0, sizeof(g));
+    g.quick = dx > 0x1p-60 && dx < 0x1p60 && dz > 0x1p-60 && dz < 0x1p60;
+    if (!g.quick) return g;
+    g.x = div_by(dx);
+    g.z = div_by(dz);
+    g.all = div_by(1.0 / dx / dx + 1.0 / dz / dz);
+    return g;
+}
+
+// The reference's 2D Godunov solution (src/RT_pfsm2d.h:89-102), bit for bit: x-neighbour minimum
+// x, z-neighbour minimum z.  The two sums of the reference commute, so nothing is sorted beyond
+// the smaller neighbour.  36 FP64 instructions (spacings of few bits) instead of about 95.
+PFAST_HD double eik2_exact(double x, double z, double s, const ExactGrid2& g) {
+    const bool zlow = bits_of(z) <= bits_of(x);
+    const double lo = zlow ? z : x, hi = zlow ? x : z;
+    const double dlo = zlow ? g.z.d : g.x.d;
+    const double q = lo + dlo * s;
+    if (bits_of(q) <= bits_of(hi)) return q;
+    double S, C;
+    if (in_range(hi) && (is_zero(lo) || in_range(lo))) {
+        S = div_exact(div_exact(x, g.x), g.x) + div_exact(div_exact(z, g.z), g.z);
+        C = div_exact(div_exact(x * x, g.x), g.x) + div_exact(div_exact(z * z, g.z), g.z) - s * s;
+        const double D = S * S - g.all.d * C;
+        return (D >= 0) ? div_exact4(S + sqrt(D), g.all.d, g.all.rh, g.all.rl) : kUnreached;
+    }
+    const double A = g.all.d;
+    const double B = -2. * (x / g.x.d / g.x.d + z / g.z.d / g.z.d);
+    C = x * x / g.x.d / g.x.d + z * z / g.z.d / g.z.d - s * s;
+    const double D = B * B - 4 * A * C;
+    return (D >= 0) ? (-B + sqrt(D)) / 2. / A : kUnreached;
+}
+
+}  // namespace pfast

@@ -38,14 +38,15 @@ __host__ __device__ constexpr int warp_smem2() {
                (T::adj && !t_windows2<KIND>() ? H2I * R2 * sizeof(typename T::Aux) : 0));
 }
 
-__device__ __forceinline__ double ref_min(double x, double y) { return (x < y) ? x : y; }
+__device__ __forceinline__ double ref_min(double x, double y) { return min_nonneg(x, y); }   // values >= +0
 __device__ __forceinline__ float ref_min(float x, float y) { return (x < y) ? x : y; }
 
-// Reference 2D Godunov update (src/RT_pfsm2d.h:89-102), operand order kept.
+// Reference 2D Godunov update (src/RT_pfsm2d.h:89-102), operand order kept (exact_arith.h, or
+// for spacings outside its range the expressions as they stand).
 // a: x-neighbour minimum (spacing dx), b: z-neighbour minimum (dz).
-__device__ __forceinline__ double eik2_plain(double a, double b, double s, double dx, double dz, double i2x,
-                                             double i2z) {
-    double da = dx, db = dz, ia = i2x, ib = i2z, t;
+__device__ __forceinline__ double eik2_plain(double a, double b, double s, const Sweep2Args& K) {
+    if (K.ex.quick) return eik2_exact(a, b, s, K.ex);
+    double da = K.dx, db = K.dz, ia = K.inv2x, ib = K.inv2z, t;
     if (b > a) { t = a; a = b; b = t; t = da; da = db; db = t; t = ia; ia = ib; ib = t; }
     double q = b + db * s;
     if (q <= a) return q;
@@ -73,10 +74,20 @@ __device__ __forceinline__ R eik2_fast(R a, R b, R s, R dx, R dz, R wx, R wz, R 
 __device__ __forceinline__ double pos_ref(double x) { return (x + fabs(x)) / 2.0; }
 __device__ __forceinline__ double neg_ref(double x) { return (x - fabs(x)) / 2.0; }
 
-// Reference 2D adjoint update (src/RT_padjoint2d.h:42-65).
+// Reference 2D adjoint update (src/RT_padjoint2d.h:42-65), as eik2_plain.
 __device__ __forceinline__ double adj2_plain(double T0, double Txp, double Txm, double Tzp, double Tzm, double Lxp,
-                                             double Lxm, double Lzp, double Lzm, double dx, double dz) {
-    if (Txp >= kInf || T0 >= kInf || Txm >= kInf || Tzp >= kInf || Tzm >= kInf) return 0.0;
+                                             double Lxm, double Lzp, double Lzm, const Sweep2Args& K) {
+    const long long inf = dbits(kInf);   // T >= INF on the bit patterns (T >= 0)
+    if (dbits(Txp) >= inf || dbits(T0) >= inf || dbits(Txm) >= inf || dbits(Tzp) >= inf || dbits(Tzm) >= inf)
+        return 0.0;
+    if (K.ex.quick) {
+        double ex, ez, nx, nz;
+        adj_axis_exact(T0, Txp, Txm, Lxp, Lxm, K.ex.x, ex, nx);
+        adj_axis_exact(T0, Tzp, Tzm, Lzp, Lzm, K.ex.z, ez, nz);
+        const double den = ex + ez;
+        return fabs(den) > 1e-9 ? (nx + nz) / den : 0.0;
+    }
+    const double dx = K.dx, dz = K.dz;
     const double gxp = -(Txp - T0) / dx, gxm = -(T0 - Txm) / dx;
     const double gzp = -(Tzp - T0) / dz, gzm = -(T0 - Tzm) / dz;
     const double a1 = pos_ref(gxp), a2 = neg_ref(gxm);
@@ -368,13 +379,12 @@ __global__ void __launch_bounds__(kWarps2 * 32) sweep2d_kernel(const Sweep2Args 
     const int steps = ei + ej - 1;
     bool chg = false, chg_jlo = false, chg_jhi = false;
     unsigned sel = 0;
-    // Face marks and own re-marking as in the 3D sweeps: the plain kinds mark every changed
-    // face node; the others only where the neighbour's node depends on the changed one (forward:
-    // a neighbour below the node's value; adjoint: a larger traveltime).
-    constexpr bool kPrune = KIND != kFwdPlain64 && KIND != kAdjPlain64;
+    // Face marks and own re-marking as in the 3D sweeps: only where the neighbour's node depends on
+    // the changed one (forward: a neighbour below the node's value; adjoint: a larger traveltime;
+    // with the margins of the plain kinds there).
     bool m_ilo = false, m_ihi = false;
     bool restep = false;   // polish: a remainder above the floor (visit again in this order)
-    bool stale = false;    // FP32 bulk: a changed node feeds an in-tile node visited before it
+    bool stale = false;    // plain, FP32 bulk: a changed node feeds an in-tile node visited before it
 
     // ---- adjoint traveltime of the FP64 kinds through register windows (as in the 3D sweeps):
     // lane lif (flipped row) is at flipped column jf = t - lif in step t and keeps its row's
@@ -431,7 +441,7 @@ __global__ void __launch_bounds__(kWarps2 * 32) sweep2d_kernel(const Sweep2Args 
                     const Real ax = ref_min(box[c + 1], box[c - 1]);
                     const Real s = __ldg(slow + (long long)gi * nc + gj);
                     if constexpr (KIND == kFwdPlain64) {
-                        const double qv = eik2_plain(ax, bz, s, A.dx, A.dz, A.inv2x, A.inv2z);
+                        const double qv = eik2_plain(ax, bz, s, A);
                         nv = ref_min(old, qv);
                     } else if constexpr (KIND == kFwdFast32) {
                         const float qv = eik2_fast<float>(ax, bz, s, A.dxf, A.dzf, wx, wz, rsum);
@@ -451,19 +461,17 @@ __global__ void __launch_bounds__(kWarps2 * 32) sweep2d_kernel(const Sweep2Args 
                         box[c] = nv;
                         chg = true;
                         note_move(old, nv, dstep);
-                        if constexpr (kPrune) {
-                            auto dep = [&](int n) { return min(obits2(old), obits2(nv)) < obits2(box[n]); };
-                            if (li == 0 && dep(c - R2)) m_ilo = true;
-                            if (li == ei - 1 && dep(c + R2)) m_ihi = true;
-                            if (lj == 0 && dep(c - 1)) chg_jlo = true;
-                            if (lj == ej - 1 && dep(c + 1)) chg_jhi = true;
-                            if constexpr (!kSelective) {
-                                if (lif > 0 && dep(py ? c - R2 : c + R2)) stale = true;
-                                if (ljf > 0 && dep(px ? c - 1 : c + 1)) stale = true;
-                            }
-                        } else {
-                            if (lj == 0) chg_jlo = true;
-                            if (lj == ej - 1) chg_jhi = true;
+                        auto dep = [&](int n) {
+                            constexpr long long kMargin = KIND == kFwdPlain64 ? 1ll << 33 : 0;
+                            return min(obits2(old), obits2(nv)) < obits2(box[n]) + kMargin;
+                        };
+                        if (li == 0 && dep(c - R2)) m_ilo = true;
+                        if (li == ei - 1 && dep(c + R2)) m_ihi = true;
+                        if (lj == 0 && dep(c - 1)) chg_jlo = true;
+                        if (lj == ej - 1 && dep(c + 1)) chg_jhi = true;
+                        if constexpr (!kSelective) {
+                            if (lif > 0 && dep(py ? c - R2 : c + R2)) stale = true;
+                            if (ljf > 0 && dep(px ? c - 1 : c + 1)) stale = true;
                         }
                     }
                 }
@@ -477,8 +485,7 @@ __global__ void __launch_bounds__(kWarps2 * 32) sweep2d_kernel(const Sweep2Args 
                         T0 = tbox[c]; Txp = tbox[c + 1]; Txm = tbox[c - 1]; Tzp = tbox[c + R2]; Tzm = tbox[c - R2];
                     }
                     if constexpr (KIND == kAdjPlain64) {
-                        r = adj2_plain(T0, Txp, Txm, Tzp, Tzm, box[c + 1], box[c - 1], box[c + R2], box[c - R2], A.dx,
-                                       A.dz);
+                        r = adj2_plain(T0, Txp, Txm, Tzp, Tzm, box[c + 1], box[c - 1], box[c + R2], box[c - R2], A);
                     } else if constexpr (KIND == kAdjFast32) {
                         r = adj2_bulk(T0, Txp, Txm, Tzp, Tzm, box[c + 1], box[c - 1], box[c + R2], box[c - R2], wx, wz);
                     } else {
@@ -495,24 +502,21 @@ __global__ void __launch_bounds__(kWarps2 * 32) sweep2d_kernel(const Sweep2Args 
                         box[c] = r;
                         chg = true;
                         note_move(old, r, dstep);
-                        if constexpr (kPrune) {
-                            // lambda at the neighbour node reads this node if its traveltime is larger
-                            // (FP32 bulk: offsets from the tile's corner, compared as values)
-                            auto dep = [&](Aux tn) {
-                                if constexpr (sizeof(Aux) == 8) return obits2(T0) > obits2(tn);
-                                else return T0 > tn;
-                            };
-                            if (li == 0 && dep(Tzm)) m_ilo = true;
-                            if (li == ei - 1 && dep(Tzp)) m_ihi = true;
-                            if (lj == 0 && dep(Txm)) chg_jlo = true;
-                            if (lj == ej - 1 && dep(Txp)) chg_jhi = true;
-                            if constexpr (!kSelective) {
-                                if (lif > 0 && dep(py ? Tzm : Tzp)) stale = true;
-                                if (ljf > 0 && dep(px ? Txm : Txp)) stale = true;
-                            }
-                        } else {
-                            if (lj == 0) chg_jlo = true;
-                            if (lj == ej - 1) chg_jhi = true;
+                        // lambda at the neighbour node reads this node if its traveltime is larger
+                        // (FP32 bulk: offsets from the tile's corner, compared as values)
+                        auto dep = [&](Aux tn, int n) {
+                            if constexpr (KIND == kAdjPlain64)
+                                return ordered(T0) > ordered(tn) || is_zero(box[n]) || exponent_of(r) == 0x7ff;
+                            else if constexpr (sizeof(Aux) == 8) return obits2(T0) > obits2(tn);
+                            else return T0 > tn;
+                        };
+                        if (li == 0 && dep(Tzm, c - R2)) m_ilo = true;
+                        if (li == ei - 1 && dep(Tzp, c + R2)) m_ihi = true;
+                        if (lj == 0 && dep(Txm, c - 1)) chg_jlo = true;
+                        if (lj == ej - 1 && dep(Txp, c + 1)) chg_jhi = true;
+                        if constexpr (!kSelective) {
+                            if (lif > 0 && dep(py ? Tzm : Tzp, py ? c - R2 : c + R2)) stale = true;
+                            if (ljf > 0 && dep(px ? Txm : Txp, px ? c - 1 : c + 1)) stale = true;
                         }
                     }
                 }
@@ -534,16 +538,16 @@ __global__ void __launch_bounds__(kWarps2 * 32) sweep2d_kernel(const Sweep2Args 
     // nothing changed: the field and its convergence flag stand as they are
     if (!__any_sync(0xffffffffu, chg)) return;
     // unlock this tile and the face neighbours that see a changed face node (lane = row)
-    const unsigned f_ilo = __ballot_sync(0xffffffffu, kPrune ? m_ilo : chg && li == 0);
-    const unsigned f_ihi = __ballot_sync(0xffffffffu, kPrune ? m_ihi : chg && li == ei - 1);
+    const unsigned f_ilo = __ballot_sync(0xffffffffu, m_ilo);
+    const unsigned f_ihi = __ballot_sync(0xffffffffu, m_ihi);
     const unsigned f_jlo = __ballot_sync(0xffffffffu, chg_jlo);
     const unsigned f_jhi = __ballot_sync(0xffffffffu, chg_jhi);
     // own re-marking (see the 3D sweeps): a polish tile stays locked in this order after
-    // updates with remainders below the floor; an FP32 bulk tile none of whose changed nodes
+    // updates with remainders below the floor; a plain or FP32 bulk tile none of whose changed nodes
     // feeds an already visited node is a fixed point until a neighbour marks it
     bool again = true;
     if constexpr (kSelective) again = __any_sync(0xffffffffu, restep);
-    else if constexpr (kPrune) again = __any_sync(0xffffffffu, stale);
+    else again = __any_sync(0xffffffffu, stale);
     if (lane == 0) {
         dirty[tid] = dword | (again ? 0xf : (kSelective ? (0xf & ~obit) : 0));
         if (f_ilo && ti > 0) atomicOr(dirty + tid - A.nbj, 0xf);
@@ -556,8 +560,10 @@ __global__ void __launch_bounds__(kWarps2 * 32) sweep2d_kernel(const Sweep2Args 
             const long long at = (long long)(i0 + y) * nc + j0 + x;
             const Real v = box[(y + 1) * R2 + x + 1];
             fld[at] = v;
-            if constexpr (kSnap)
-                if (fabs(__ldcg(snp + at) - v) > A.tol_abs + A.tol_rel * fabs(v)) moved = true;   // isconv
+            if constexpr (kSnap) {   // isconv (equal bits need no FP64 instruction)
+                const Real was = __ldcg(snp + at);
+                if (!bits_same(was, v) && fabs(was - v) > A.tol_abs + A.tol_rel * fabs(v)) moved = true;
+            }
         }
     }
     const bool any_moved = __any_sync(0xffffffffu, moved);

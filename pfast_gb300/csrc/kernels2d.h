@@ -31,6 +31,7 @@ struct Sweep2Args {
     int nr, nc, nbi, nbj;
     double dx, dz;
     double inv2x, inv2z;         // (1.0/dx)/dx, (1.0/dz)/dz
+    ExactGrid2 ex;               // constants of the plain updates (exact_arith.h)
     float dxf, dzf;              // FP32 copies of dx, dz (no FP64 instruction in the FP32 sweeps)
     float wxf, wzf, rsumf;       // FP32 inv2x, inv2z, 1/(inv2x + inv2z)
     float polish_floor;          // polish corrections at or below this are dropped

@@ -96,29 +96,20 @@ __host__ __device__ constexpr int warp_smem_bytes() {
 // ----------------------------------------------------------- node updates
 // Reference Godunov update (src/T_pfsm3d.h:99-119).  a/b/c: neighbour minima along
 // x/y/z; s: slowness 1.0/vp (precomputed, bit-identical to the reference's per-node
-// division).  Expressions keep the reference's operand order; the ordering tests
-// run on the bit patterns (same outcome for non-negative values).
+// division).  exact_arith.h gives the reference's bits with a third of its FP64 instructions;
+// spacings outside the range of its identities take the expressions as they stand.  The ordering
+// tests run on the bit patterns (same outcome for non-negative values).
 __device__ __forceinline__ double eik3_plain(double a, double b, double c, double s, const Spacing3& sp) {
+    if (sp.ex.quick)
+        return sp.ex.iso ? eik3_exact<true>(a, b, c, s, sp.ex, sp.inv2) : eik3_exact<false>(a, b, c, s, sp.ex, sp.inv2);
     double da = sp.d[0], db = sp.d[1], dc = sp.d[2];
     double ia = sp.inv2[0], ib = sp.inv2[1], ic = sp.inv2[2];
     double t;
     if (dbits(b) > dbits(a)) { t = a; a = b; b = t; t = da; da = db; db = t; t = ia; ia = ib; ib = t; }
     if (dbits(c) > dbits(a)) { t = a; a = c; c = t; t = da; da = dc; dc = t; t = ia; ia = ic; ic = t; }
     if (dbits(c) > dbits(b)) { t = b; b = c; c = t; t = db; db = dc; dc = t; t = ib; ib = ic; ic = t; }
-    double q = dc * s + c;
-    if (dbits(q) <= dbits(b)) return q;
-    double A = dc * dc + db * db;
-    double B = -2. * (b * dc * dc + c * db * db);
-    double C = dc * dc * b * b + db * db * c * c - db * db * dc * dc * s * s;
-    double D = B * B - 4. * A * C;
-    q = (D >= 0) ? (-B + sqrt(D)) / 2. / A : kInf;
-    if (dbits(q) <= dbits(a)) return q;
-    A = ia + ib + ic;   // 1.0/da/da + 1.0/db/db + 1.0/dc/dc, each term precomputed as (1.0/d)/d
-    B = -2.0 * (a / da / da + b / db / db + c / dc / dc);
-    C = a * a / da / da + b * b / db / db + c * c / dc / dc - s * s;
-    D = B * B - 4. * A * C;
-    q = (D >= 0) ? (-B + sqrt(D)) / 2. / A : kInf;
-    return q;
+    const double q = dc * s + c;
+    return dbits(q) <= dbits(b) ? q : eik3_tail_ref(a, b, c, da, db, dc, ia, ib, ic, s);
 }
 
 // FP32 Godunov solution in difference form relative to the smallest neighbour c
@@ -234,7 +225,8 @@ __device__ __forceinline__ double eik3_newton(double U0, double a, double b, dou
 // (POS(-(T_p-T0)/d)/d = w max(-e_p,0), -NEG(-(T0-T_m)/d)/d = w max(-e_m,0),
 //  POS(-(T0-T_m)/d)/d = w max(e_m,0), -NEG(-(T_p-T0)/d)/d = w max(e_p,0)).
 
-// Reference adjoint update (src/T_padjoint3d.h:42-71); operand order kept.
+// Reference adjoint update (src/T_padjoint3d.h:42-71); operand order kept (exact_arith.h, or for
+// spacings outside its range the expressions as they stand).
 __device__ __forceinline__ double pos_ref(double x) { return (x + fabs(x)) / 2.0; }   // POS macro
 __device__ __forceinline__ double neg_ref(double x) { return (x - fabs(x)) / 2.0; }   // NEG macro
 __device__ __forceinline__ bool unreached64(double T0, double a, double b, double c, double d, double e, double f) {
@@ -247,6 +239,14 @@ __device__ __forceinline__ double adj3_plain(double T0, double Txp, double Txm, 
                                              double Tzp, double Tzm, double Lxp, double Lxm, double Lyp,
                                              double Lym, double Lzp, double Lzm, const Spacing3& sp) {
     if (unreached64(T0, Txp, Txm, Typ, Tym, Tzp, Tzm)) return 0.0;
+    if (sp.ex.quick) {
+        double ex, ey, ez, nx, ny, nz;
+        adj_axis_exact(T0, Txp, Txm, Lxp, Lxm, sp.ex.axis[0], ex, nx);
+        adj_axis_exact(T0, Typ, Tym, Lyp, Lym, sp.ex.axis[1], ey, ny);
+        adj_axis_exact(T0, Tzp, Tzm, Lzp, Lzm, sp.ex.axis[2], ez, nz);
+        const double den = ex + ey + ez;
+        return fabs(den) > 1e-9 ? (nx + ny + nz) / den : 0.0;
+    }
     const double dx = sp.d[0], dy = sp.d[1], dz = sp.d[2];
     const double gxp = -(Txp - T0) / dx, gxm = -(T0 - Txm) / dx;
     const double gyp = -(Typ - T0) / dy, gym = -(T0 - Tym) / dy;
@@ -609,6 +609,27 @@ __device__ __forceinline__ unsigned adj_orders(long long t, long long xlo, long 
 __device__ __forceinline__ long long obits(double x) { return __double_as_longlong(x); }
 __device__ __forceinline__ int obits(float x) { return __float_as_int(x); }
 
+// Whether the update of a neighbour (value vn, traveltime tn) can depend on a node that changed
+// to nv; lo: the smaller of the node's old and new value (ordered bits), t0: its traveltime.
+// Forward: the Godunov update and its Newton form exclude neighbours above the node's value.
+// Adjoint: lambda at a node weighs its neighbours with max(T_neighbour - T_node, 0).
+// The plain kinds skip tiles only where that leaves every bit as it is:
+//   forward: the reference's formula is the exact solution to within sqrt(8 eps) = 4e-8 relative at
+//   worst (its discriminant cancels), so a neighbour value more than 2^-20 relative above the
+//   node's can neither lower the minimum of the node's value and the formula's nor take part in
+//   it; closer values count as a dependency;
+//   adjoint: a neighbour of smaller or equal traveltime enters as +0 * lambda, which can change
+//   no bit of a nonzero sum of finite terms; a zero lambda (the sign of a zero sum) and a
+//   non-finite change count as dependencies.
+template <int KIND, typename B, typename Real, typename Aux>
+__device__ __forceinline__ bool depends_on(B lo, Real nv, Aux t0, Real vn, Aux tn) {
+    if constexpr (KIND == kFwdPlain64) return lo < obits(vn) + (1ll << 33);
+    else if constexpr (KIND == kAdjPlain64)
+        return ordered(t0) > ordered(tn) || is_zero(vn) || exponent_of(nv) == 0x7ff;
+    else if constexpr (Traits<KIND>::adj) return obits(t0) > obits(tn);
+    else return lo < obits(vn);
+}
+
 // ----------------------------------------------------------- the sweep kernel
 // Tile locking: a tile whose processing changed no bit of its field, and none of
 // whose face neighbours has changed a face node since, is a fixed point of the node
@@ -764,15 +785,12 @@ __device__ __forceinline__ void process_tile(const Sweep3Args& A, const int inst
     const Aux* srow = ADJ ? nullptr : reinterpret_cast<const Aux*>(A.aux) + rowbase;
     bool chg = false;   // this lane's pencil changed
     // Face marks in flipped terms (u: the upstream face of the sweep, d: the downstream one): a
-    // changed face node that a node of the face neighbour depends on.  The plain kinds mark
-    // every changed face node (their tile skipping must stay exact).  Elsewhere the dependency
-    // is one-directional: a forward update reads only neighbours below the node's value (the
-    // Godunov update and its Newton form exclude larger ones), and lambda at a node reads only
-    // neighbours of larger traveltime.
-    constexpr bool kPrune = KIND != kFwdPlain64 && KIND != kAdjPlain64;
+    // changed face node that a node of the face neighbour depends on (depends_on: a forward
+    // update reads only neighbours below the node's value, lambda at a node only neighbours of
+    // larger traveltime).
     bool m_zu = false, m_zd = false, m_yu = false, m_yd = false, m_xu = false, m_xd = false;
     bool restep = false;   // polish: some update left a remainder above the floor (visit again in this order)
-    // FP32 bulk: some changed node feeds an in-tile node that this pass visited before it
+    // plain, FP32 bulk: some changed node feeds an in-tile node that this pass visited before it
     // (so the tile is not yet a fixed point of the update)
     bool stale = false;
     bool moved = false;   // FP32 bulk, polish: some node of this lane moved by more than the tolerance
@@ -973,29 +991,21 @@ __device__ __forceinline__ void process_tile(const Sweep3Args& A, const int inst
                 } else if constexpr (!kSnap) {
                     if (fabsf(old - nv) > A.tol_abs_f + A.tol_rel_f * fabsf(nv)) moved = true;
                 }
-                if constexpr (kPrune) {
-                    // does the neighbour across a face (value vn, traveltime tn) depend on this node?
-                    // The neighbour values were read before this step's stores, none of which
-                    // touches them (they lie on the hyperplanes t - 1 and t + 1).
-                    const auto lo = min(obits(old), obits(nv));
-                    auto dep = [&](Real vn, Aux tn) {
-                        if constexpr (ADJ) return obits(t0) > obits(tn);
-                        else return lo < obits(vn);
-                    };
-                    if (lkf == 0 && dep(zu, Tzu)) m_zu = true;
-                    if (lkf == ek - 1 && dep(zd, Tzd)) m_zd = true;
-                    if (lif == 0 && dep(yu, Tyu)) m_yu = true;
-                    if (lif == ei - 1 && dep(yd, Tyd)) m_yd = true;
-                    if (ljf == 0 && dep(xu, Txu)) m_xu = true;
-                    if (ljf == ej - 1 && dep(xd, Txd)) m_xd = true;
-                    if constexpr (!kSelective) {
-                        // the in-tile neighbours this pass visited before the node (flipped upstream)
-                        if ((lkf > 0 && dep(zu, Tzu)) || (lif > 0 && dep(yu, Tyu)) || (ljf > 0 && dep(xu, Txu)))
-                            stale = true;
-                    }
-                } else {
-                    if (ljf == 0) m_xu = true;
-                    if (ljf == ej - 1) m_xd = true;
+                // does the neighbour across a face (value vn, traveltime tn) depend on this node?
+                // The neighbour values were read before this step's stores, none of which
+                // touches them (they lie on the hyperplanes t - 1 and t + 1).
+                const auto lo = min(obits(old), obits(nv));
+                auto dep = [&](Real vn, Aux tn) { return depends_on<KIND>(lo, nv, t0, vn, tn); };
+                if (lkf == 0 && dep(zu, Tzu)) m_zu = true;
+                if (lkf == ek - 1 && dep(zd, Tzd)) m_zd = true;
+                if (lif == 0 && dep(yu, Tyu)) m_yu = true;
+                if (lif == ei - 1 && dep(yd, Tyd)) m_yd = true;
+                if (ljf == 0 && dep(xu, Txu)) m_xu = true;
+                if (ljf == ej - 1 && dep(xd, Txd)) m_xd = true;
+                if constexpr (!kSelective) {
+                    // the in-tile neighbours this pass visited before the node (flipped upstream)
+                    if ((lkf > 0 && dep(zu, Tzu)) || (lif > 0 && dep(yu, Tyu)) || (ljf > 0 && dep(xu, Txu)))
+                        stale = true;
                 }
             }
         }
@@ -1021,23 +1031,20 @@ __device__ __forceinline__ void process_tile(const Sweep3Args& A, const int inst
 
     // ---- unlock this tile and every face neighbour that sees a changed face node (flipped
     // faces mapped back to grid faces)
-    const bool klo = kPrune ? (pz ? m_zu : m_zd) : chg && lk == 0, khi = kPrune ? (pz ? m_zd : m_zu) : chg && lk == ek - 1;
-    const bool ilo = kPrune ? (py ? m_yu : m_yd) : chg && li == 0, ihi = kPrune ? (py ? m_yd : m_yu) : chg && li == ei - 1;
-    const unsigned f_klo = __ballot_sync(0xffffffffu, klo);
-    const unsigned f_khi = __ballot_sync(0xffffffffu, khi);
-    const unsigned f_ilo = __ballot_sync(0xffffffffu, ilo);
-    const unsigned f_ihi = __ballot_sync(0xffffffffu, ihi);
+    const unsigned f_klo = __ballot_sync(0xffffffffu, pz ? m_zu : m_zd);
+    const unsigned f_khi = __ballot_sync(0xffffffffu, pz ? m_zd : m_zu);
+    const unsigned f_ilo = __ballot_sync(0xffffffffu, py ? m_yu : m_yd);
+    const unsigned f_ihi = __ballot_sync(0xffffffffu, py ? m_yd : m_yu);
     const unsigned f_jlo = __ballot_sync(0xffffffffu, px ? m_xu : m_xd);
     const unsigned f_jhi = __ballot_sync(0xffffffffu, px ? m_xd : m_xu);
     // Own re-marking.  A polish sweep in order o leaves every node that selects o consistent
     // with the values it reads (its active neighbours come before it in o), so after small
     // updates the tile is due again in o only when a neighbour or another order changes
-    // something.  An FP32 bulk pass in which no changed node feeds an already visited node
+    // something.  A plain or FP32 bulk pass in which no changed node feeds an already visited node
     // leaves the tile a fixed point of the update: it stays locked until a neighbour marks it.
-    // The plain kinds re-mark all orders (their tile skipping must stay exact).
     bool again = true;
     if constexpr (kSelective) again = __any_sync(0xffffffffu, restep);
-    else if constexpr (kPrune) again = __any_sync(0xffffffffu, stale);
+    else again = __any_sync(0xffffffffu, stale);
     if (lane == 0) {
         // neighbours keep their selection bits: OR in the eight order bits (two tiles of one
         // launch can share a face neighbour, hence atomic)
@@ -1083,7 +1090,8 @@ __device__ __forceinline__ void process_tile(const Sweep3Args& A, const int inst
                 if (rk < ek && ri < ei && lane < ej) {
                     const Real v = box[box_index<SH>(rk, ri, lane, ek, ei, ej, pz, py, px)];
                     fld[(k0 + rk) * plane + (long long)(i0 + ri) * nc + j0 + lane] = v;
-                    if (fabs(p[u] - v) > A.tol_abs) moved = true;   // isconv, src/T_pfsm3d.h:126
+                    // isconv, src/T_pfsm3d.h:126 (equal bits need no FP64 instruction)
+                    if (dbits(p[u]) != dbits(v) && fabs(p[u] - v) > A.tol_abs) moved = true;
                 }
             }
         }

@@ -183,6 +183,7 @@ extern "C" pfast_status pfast_fsm3d_noalloc(const double* vp, double* U, int src
         a.sp.d2[k] = dd[k] * dd[k];
         a.sp.inv2[k] = 1.0 / dd[k] / dd[k];
     }
+    a.sp.ex = exact_grid3(dd);
     a.tol_abs = kConvTol;
     a.ntiles = ntiles;
     a.dirty = d_dirty;
