@@ -166,10 +166,12 @@ Spacing3 make_spacing(double dx, double dy, double dz) {
 static std::mutex g_tune_mu;
 static std::map<std::tuple<int, int, int, int, int, int>, TuneEntry> g_tune;
 
+// The fastest allowed candidate once all are timed; -1 before that.
 static int tuned_candidate(const std::tuple<int, int, int, int, int, int>& key, unsigned allowed, int sms) {
     std::lock_guard<std::mutex> g(g_tune_mu);
     auto it = g_tune.find(key);
-    return tune_pick(it != g_tune.end() ? &it->second : nullptr, allowed, std::get<5>(key), sms);
+    if (it == g_tune.end() || !tune_complete(&it->second, allowed)) return -1;
+    return tune_pick(&it->second, allowed, std::get<5>(key), sms);
 }
 
 static void tune_record(const std::tuple<int, int, int, int, int, int>& key, int which, double ms) {
@@ -261,18 +263,25 @@ pfast_status run_sweeps3(pfast_ctx* ctx, Sweep3Args a, int kind, int nb, std::ve
     PFAST_CUDA_TRY(cudaGetDevice(&dev));
     PFAST_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const auto tkey = std::make_tuple(dev, kind, a.nz, a.nr, a.nc, (int)active.size());
-    int dwarps[kTileShapes] = {}, dblocks[kTileShapes] = {};
+    DataflowShape dshape[kTileShapes];
     bool fits[kTileShapes] = {};
     for (int shape = 0; shape < kTileShapes; ++shape) {
         if (ctx->tile_shape != PFAST_TILE_AUTO && ctx->tile_shape - 1 != shape) continue;
         DiagTable3* t = nullptr;
         PFAST_TRY(ctx_diag3(ctx, a.nz, a.nr, a.nc, shape, &t));
         const int ntl = t->nbk * t->nbi * t->nbj;
-        if (!active.empty()) PFAST_TRY(dataflow_shape(kind, shape, ntl, (int)active.size(), &dwarps[shape], &dblocks[shape]));
-        fits[shape] = dwarps[shape] > 0;
+        if (!active.empty()) PFAST_TRY(dataflow_shape(kind, shape, ntl, (int)active.size(), &dshape[shape]));
+        fits[shape] = dshape[shape].warps > 0;
     }
     const unsigned allowed = tune_allowed(ctx->schedule, ctx->tile_shape, fits);
-    const int cand = tuned_candidate(tkey, allowed, sms);
+    int cand = tuned_candidate(tkey, allowed, sms);
+    if (cand < 0) {
+        const int shape = ctx->tile_shape == PFAST_TILE_AUTO ? 0 : ctx->tile_shape - 1;
+        DiagTable3* t = nullptr;
+        PFAST_TRY(ctx_diag3(ctx, a.nz, a.nr, a.nc, shape, &t));
+        cand = untuned_pick(allowed, kind == kFwdPlain64 || kind == kAdjPlain64, kind == kFwdFast32 || kind == kAdjFast32,
+                            dshape[shape].cluster, (int)active.size(), (long long)t->nbk * t->nbi * t->nbj, t->ndiag, sms);
+    }
     ctx->candidates = (ctx->candidates & ~(15 << 4 * kind)) | (cand + 1) << 4 * kind;
     const bool persistent = cand >> 1 == 1, hybrid = cand >> 1 == 2;
     a.shape = cand & 1;
@@ -339,8 +348,7 @@ pfast_status run_sweeps3(pfast_ctx* ctx, Sweep3Args a, int kind, int nb, std::ve
         Sweep3Args b = a;
         b.iter = base;
         b.dyn = nullptr;
-        PFAST_TRY(launch_sweep3_dataflow(kind, b, nact, maxiter, ctx->queue.as<int>(), a.changed, dwarps[a.shape],
-                                         dblocks[a.shape], st));
+        PFAST_TRY(launch_sweep3_dataflow(kind, b, nact, maxiter, ctx->queue.as<int>(), a.changed, dshape[a.shape], st));
         ++ctx->launches;
         PFAST_TRY(ctx->h_dyn.ensure(2 * sizeof(int)));
         int* hq = ctx->h_dyn.as<int>();

@@ -80,23 +80,27 @@ pfast_status launch_seed_tiles3(int kind, const Sweep3Args& a, int nact, cudaStr
 // One tile-diagonal launch over grid (tiles, nact): a.act must hold at least nact entries
 // (every block reads a.act[blockIdx.y] before it tests whether its instance is still active).
 pfast_status launch_sweep3(int kind, const Sweep3Args& a, int d0, int tiles, int nact, cudaStream_t st);
-// Dataflow sweep kernel (one launch per phase): `blocks` blocks of `warps` warps take the
+// Launch shape of the dataflow sweep kernel: warps per block (as many as shared memory holds; 0
+// when the grid does not fit), blocks per instance (a thread-block cluster when > 1) and resident
+// blocks.
+struct DataflowShape {
+    int warps = 0, cluster = 1, blocks = 0;
+};
+pfast_status dataflow_shape(int kind, int shape, int ntiles, int nact, DataflowShape* out, bool multi = false);
+// Dataflow sweep kernel (one launch per phase): blocks or clusters take the
 // nact instances of a.act from queue[0] (zeroed by the caller) and solve each to convergence
 // (maxiter outer iterations at most); result[inst] = iterations | 1<<30 if not converged
 // (| 1<<29 and queue[1] |= 1 if a block stalled: an internal error).  a.dirty, a.diff,
 // a.stamp as for the per-diagonal launches; a.ntiles <= kDataflowMaxTiles.
 pfast_status launch_sweep3_dataflow(int kind, const Sweep3Args& a, int nact, int maxiter, int* queue, int* result,
-                                    int warps, int blocks, cudaStream_t st);
+                                    const DataflowShape& ds, cudaStream_t st);
 // The dataflow kernel over instances of several grids: item q is instance items[q].y of the grid
 // whose arguments are models[items[q].x] (a device array; each model's result goes to its own
-// `changed` array); max_ntiles: the largest grid's tile count (<= kDataflowMaxTiles); warps and
-// blocks from dataflow_shape(kind, shape, max_ntiles, nitems, warps, blocks, true).
+// `changed` array); max_ntiles: the largest grid's tile count (<= kDataflowMaxTiles); ds
+// from dataflow_shape(kind, shape, max_ntiles, nitems, &ds, true).
 pfast_status launch_sweep3_dataflow_multi(int kind, int shape, const Sweep3Args* models, const int2* items, int nitems,
-                                          int max_ntiles, int maxiter, int* queue, int warps, int blocks,
+                                          int max_ntiles, int maxiter, int* queue, const DataflowShape& ds,
                                           cudaStream_t st);
-// Warps per block (as many as shared memory holds) and resident blocks
-// of the dataflow kernel; *warps = 0 when a grid of ntiles tiles does not fit.
-pfast_status dataflow_shape(int kind, int shape, int ntiles, int nact, int* warps, int* blocks, bool multi = false);
 
 // The sweep launchers of one tile shape (kernels3d_tiles.cuh; instantiated for Shape48 in
 // kernels3d.cu and for Shape84 in kernels3d_s84.cu); the functions above dispatch to them.
@@ -104,10 +108,10 @@ template <class SH>
 struct ShapeLaunchers {
     static pfast_status sweep(int kind, const Sweep3Args& a, int d0, int tiles, int nact, cudaStream_t st);
     static pfast_status dataflow(int kind, const Sweep3Args& a, int nact, int maxiter, int* queue, int* result,
-                                 int warps, int blocks, cudaStream_t st);
+                                 const DataflowShape& ds, cudaStream_t st);
     static pfast_status dataflow_multi(int kind, const Sweep3Args* models, const int2* items, int nitems,
-                                       int max_ntiles, int maxiter, int* queue, int warps, int blocks, cudaStream_t st);
-    static pfast_status dataflow_shape(int kind, int ntiles, int nact, bool multi, int* warps, int* blocks);
+                                       int max_ntiles, int maxiter, int* queue, const DataflowShape& ds, cudaStream_t st);
+    static pfast_status dataflow_shape(int kind, int ntiles, int nact, bool multi, DataflowShape* out);
     static pfast_status seed(int kind, const Sweep3Args& a, int nact, cudaStream_t st);
     static pfast_status orders(int kind, const Sweep3Args& a, int nact, cudaStream_t st);
 };

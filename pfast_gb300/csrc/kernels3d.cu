@@ -88,37 +88,35 @@ pfast_status launch_sweep3(int kind, const Sweep3Args& a, int d0, int tiles, int
                    : ShapeLaunchers<Shape48>::sweep(kind, a, d0, tiles, nact, st);
 }
 
+static bool good_shape(const DataflowShape& ds, int ntiles) {
+    if (ds.warps >= 1 && ds.warps <= 32 && ds.cluster >= 1 && ds.blocks >= ds.cluster && ntiles <= kDataflowMaxTiles)
+        return true;
+    set_last_error("dataflow sweep: bad shape (%d warps, %d blocks in clusters of %d, %d tiles)", ds.warps, ds.blocks,
+                   ds.cluster, ntiles);
+    return false;
+}
+
 pfast_status launch_sweep3_dataflow(int kind, const Sweep3Args& a, int nact, int maxiter, int* queue, int* result,
-                                    int warps, int blocks, cudaStream_t st) {
+                                    const DataflowShape& ds, cudaStream_t st) {
     if (nact <= 0 || maxiter <= 0) return PFAST_OK;
-    if (warps < 1 || warps > 32 || blocks < 1 || a.ntiles > kDataflowMaxTiles) {
-        set_last_error("dataflow sweep: bad shape (%d warps, %d blocks, %d tiles)", warps, blocks, a.ntiles);
-        return PFAST_ERR_INVALID;
-    }
-    if (!known_shape(a.shape)) return PFAST_ERR_INVALID;
-    return a.shape ? ShapeLaunchers<Shape84>::dataflow(kind, a, nact, maxiter, queue, result, warps, blocks, st)
-                   : ShapeLaunchers<Shape48>::dataflow(kind, a, nact, maxiter, queue, result, warps, blocks, st);
+    if (!good_shape(ds, a.ntiles) || !known_shape(a.shape)) return PFAST_ERR_INVALID;
+    return a.shape ? ShapeLaunchers<Shape84>::dataflow(kind, a, nact, maxiter, queue, result, ds, st)
+                   : ShapeLaunchers<Shape48>::dataflow(kind, a, nact, maxiter, queue, result, ds, st);
 }
 
 pfast_status launch_sweep3_dataflow_multi(int kind, int shape, const Sweep3Args* models, const int2* items, int nitems,
-                                          int max_ntiles, int maxiter, int* queue, int warps, int blocks,
+                                          int max_ntiles, int maxiter, int* queue, const DataflowShape& ds,
                                           cudaStream_t st) {
     if (nitems <= 0 || maxiter <= 0) return PFAST_OK;
-    if (warps < 1 || warps > 32 || blocks < 1 || max_ntiles > kDataflowMaxTiles) {
-        set_last_error("dataflow sweep: bad shape (%d warps, %d blocks, %d tiles)", warps, blocks, max_ntiles);
-        return PFAST_ERR_INVALID;
-    }
-    if (!known_shape(shape)) return PFAST_ERR_INVALID;
-    return shape ? ShapeLaunchers<Shape84>::dataflow_multi(kind, models, items, nitems, max_ntiles, maxiter, queue, warps,
-                                                           blocks, st)
-                 : ShapeLaunchers<Shape48>::dataflow_multi(kind, models, items, nitems, max_ntiles, maxiter, queue, warps,
-                                                           blocks, st);
+    if (!good_shape(ds, max_ntiles) || !known_shape(shape)) return PFAST_ERR_INVALID;
+    return shape ? ShapeLaunchers<Shape84>::dataflow_multi(kind, models, items, nitems, max_ntiles, maxiter, queue, ds, st)
+                 : ShapeLaunchers<Shape48>::dataflow_multi(kind, models, items, nitems, max_ntiles, maxiter, queue, ds, st);
 }
 
-pfast_status dataflow_shape(int kind, int shape, int ntiles, int nact, int* warps, int* blocks, bool multi) {
+pfast_status dataflow_shape(int kind, int shape, int ntiles, int nact, DataflowShape* out, bool multi) {
     if (!known_shape(shape)) return PFAST_ERR_INVALID;
-    return shape ? ShapeLaunchers<Shape84>::dataflow_shape(kind, ntiles, nact, multi, warps, blocks)
-                 : ShapeLaunchers<Shape48>::dataflow_shape(kind, ntiles, nact, multi, warps, blocks);
+    return shape ? ShapeLaunchers<Shape84>::dataflow_shape(kind, ntiles, nact, multi, out)
+                 : ShapeLaunchers<Shape48>::dataflow_shape(kind, ntiles, nact, multi, out);
 }
 
 pfast_status launch_seed_tiles3(int kind, const Sweep3Args& a, int nact, cudaStream_t st) {

@@ -29,13 +29,16 @@
 #include <vector>
 #include <algorithm>
 #include <type_traits>
+#include <cooperative_groups.h>
 #include "kernels.h"
 #include "dataflow3.h"
+#include "tune_policy.h"
 
 namespace pfast {
 
 namespace {
 
+namespace cg = cooperative_groups;
 
 template <int KIND> struct Traits;
 template <> struct Traits<kFwdPlain64>   { using Real = double; using Aux = double; static constexpr bool adj = false; };
@@ -1155,11 +1158,12 @@ constexpr unsigned kSlotEmpty = 0xffffffffu;
 constexpr int kDfArgsBytes = (int)((sizeof(Sweep3Args) + 15) / 16 * 16);
 static_assert(sizeof(Sweep3Args) % 8 == 0 && sizeof(Sweep3Args) % 4 == 0, "argument copy by words");
 
-struct DataflowShared {
+struct alignas(16) DataflowShared {
     unsigned head, tail;   // ring positions: next to take / next to fill
     int done;              // items completed in this outer iteration
     int abort;
     int item;
+    int flags[2];          // clusters, by iteration parity: bit 0 some tile moved, bit 1 some tile due
 };
 
 __device__ __forceinline__ unsigned long long global_ns() {
@@ -1168,90 +1172,166 @@ __device__ __forceinline__ unsigned long long global_ns() {
     return t;
 }
 
-__device__ __forceinline__ void df_push(unsigned* slots, unsigned qmask, DataflowShared* sh, unsigned e) {
-    const unsigned p = atomicAdd(&sh->tail, 1u);
-    unsigned* slot = slots + (p & qmask);
+// Orders this thread's earlier accesses before its later ones for the other warps of the block
+// (CL: of the cluster; the field then travels through L2 between SMs).
+template <bool CL>
+__device__ __forceinline__ void df_fence() {
+    if constexpr (CL) asm volatile("fence.acq_rel.cluster;" ::: "memory");
+    else __threadfence_block();
+}
+
+// The queue words of a block or cluster: the counters, the ring and its state (CL: in the shared
+// memory of the cluster's first block, reached through distributed shared memory).
+struct DataflowQueue {
+    unsigned* cnt;
+    unsigned* slots;
+    unsigned qmask;
+    DataflowShared* sh;
+};
+
+__device__ __forceinline__ void df_push(const DataflowQueue& Q, unsigned e) {
+    const unsigned p = atomicAdd(&Q.sh->tail, 1u);
+    unsigned* slot = Q.slots + (p & Q.qmask);
     // a slot still holds an earlier round's item only while that item's taker is about to
     // exchange it out (at most ntiles <= ring size items are outstanding): wait for it
     for (int spin = 0; atomicCAS(slot, kSlotEmpty, e) != kSlotEmpty; ++spin)
-        if (spin > (1 << 22) || *(volatile int*)&sh->abort) { *(volatile int*)&sh->abort = 1; return; }
+        if (spin > (1 << 22) || *(volatile int*)&Q.sh->abort) { *(volatile int*)&Q.sh->abort = 1; return; }
 }
 
-// One missing dependency of item (od, y) fewer; push it when it was the last.
-__device__ __forceinline__ void df_notify(unsigned* cnt, unsigned* slots, unsigned qmask, DataflowShared* sh, int y,
-                                          int od) {
-    const unsigned shf = 8u * (unsigned)(y & 3) + 4u * (unsigned)(od & 1);
-    const unsigned old = (atomicSub(cnt + (y >> 2), 1u << shf) >> shf) & 15u;
-    if (old == 1u) df_push(slots, qmask, sh, ((unsigned)y << 3) | (unsigned)od);
-    else if (old == 0u) *(volatile int*)&sh->abort = 1;   // more completions than dependencies: stop
+// The k-th possible dependent of item (o, x), k < 13 (dataflow3.h: dependents()): -1, or the item
+// that has one missing dependency fewer.
+__device__ __forceinline__ int df_dependent(const TileGrid3& g, int o, int x, int k) {
+    if (k == 0) return o < 7 ? (x << 3) | (o + 1) : -1;
+    const int a = (k - 1) >> 2, s = ((k - 1) >> 1) & 1, later = (k - 1) & 1;
+    const int y = tile_neighbour(g, x, a, s);
+    if (y < 0) return -1;
+    if (!later) return side_upstream(o, a, 1 - s) ? (y << 3) | o : -1;
+    return o < 7 && !side_upstream(o + 1, a, 1 - s) ? (y << 3) | (o + 1) : -1;
 }
 
-// Completion of item (o, x): re-arm x's counter of parity o for order o + 2 (it is zero: it
-// fired for (o, x), and no dependency of (o + 2, x) completes before (o, x) did), then notify
-// the dependents (dataflow3.h: dependents()).
-__device__ __forceinline__ void df_complete(const TileGrid3& g, unsigned* cnt, unsigned* slots, unsigned qmask,
-                                            DataflowShared* sh, int o, int x) {
+// Item e has one missing dependency fewer; returns its count before.
+__device__ __forceinline__ unsigned df_notify(const DataflowQueue& Q, int e) {
+    const int y = e >> 3;
+    const unsigned shf = 8u * (unsigned)(y & 3) + 4u * (unsigned)(e & 1);
+    return (atomicSub(Q.cnt + (y >> 2), 1u << shf) >> shf) & 15u;
+}
+
+// Re-arm x's counter of parity o for order o + 2 (it is zero: it fired for (o, x), and no
+// dependency of (o + 2, x) completes before (o, x) did).
+__device__ __forceinline__ void df_rearm(const TileGrid3& g, const DataflowQueue& Q, int o, int x) {
     if (o + 2 < 8)
-        atomicAdd(cnt + (x >> 2), (unsigned)dep_count(g, o + 2, x) << (8u * (unsigned)(x & 3) + 4u * (unsigned)(o & 1)));
-    __threadfence_block();
-    if (o < 7) df_notify(cnt, slots, qmask, sh, x, o + 1);
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-#pragma unroll
-        for (int s = 0; s < 2; ++s) {
-            const int y = tile_neighbour(g, x, a, s);
-            if (y < 0) continue;
-            if (side_upstream(o, a, 1 - s)) df_notify(cnt, slots, qmask, sh, y, o);
-            if (o < 7 && !side_upstream(o + 1, a, 1 - s)) df_notify(cnt, slots, qmask, sh, y, o + 1);
-        }
+        atomicAdd(Q.cnt + (x >> 2), (unsigned)dep_count(g, o + 2, x) << (8u * (unsigned)(x & 3) + 4u * (unsigned)(o & 1)));
 }
 
-// The warps' part of one outer iteration of instance inst.
-template <int KIND, class SH>
+// Completion of item (o, x) by one lane: re-arm, then notify the dependents (the notifications
+// are all in flight together).  Of the items that become ready, one is returned for the lane to
+// go on with; the others join the ring.
+template <bool CL>
+__device__ __forceinline__ unsigned df_complete(const TileGrid3& g, const DataflowQueue& Q, int o, int x) {
+    df_rearm(g, Q, o, x);
+    df_fence<CL>();
+    int dep[13];
+    unsigned old[13];
+#pragma unroll
+    for (int k = 0; k < 13; ++k) {
+        dep[k] = df_dependent(g, o, x, k);
+        old[k] = dep[k] >= 0 ? df_notify(Q, dep[k]) : 2u;
+    }
+    unsigned keep = kSlotEmpty;
+#pragma unroll
+    for (int k = 0; k < 13; ++k) {
+        if (old[k] == 1u) {
+            if (keep == kSlotEmpty) keep = (unsigned)dep[k];
+            else df_push(Q, (unsigned)dep[k]);
+        } else if (old[k] == 0u) {
+            *(volatile int*)&Q.sh->abort = 1;   // more completions than dependencies: stop
+        }
+    }
+    return keep;
+}
+
+// The same by a whole warp, one dependent per lane: each lane returns its dependent if that
+// became ready.
+template <bool CL>
+__device__ __forceinline__ unsigned df_complete_warp(const TileGrid3& g, const DataflowQueue& Q, int o, int x, int lane) {
+    if (lane == 0) {
+        df_rearm(g, Q, o, x);
+        df_fence<CL>();
+    }
+    __syncwarp();
+    unsigned keep = kSlotEmpty;
+    const int dep = lane < 13 ? df_dependent(g, o, x, lane) : -1;
+    if (dep >= 0) {
+        df_fence<CL>();   // the warp's tile (seen by this lane through the warp barrier) first
+        const unsigned old = df_notify(Q, dep);
+        if (old == 1u) keep = (unsigned)dep;
+        else if (old == 0u) *(volatile int*)&Q.sh->abort = 1;
+    }
+    __syncwarp();
+    return keep;
+}
+
+// The warps' part of one outer iteration of instance inst; nw: warps of the block or cluster.
+template <int KIND, bool CL, class SH>
 __device__ __forceinline__ void df_iteration(const Sweep3Args& A, const int inst, const int iter, const TileGrid3& g,
-                                             unsigned* cnt, unsigned* slots, const unsigned qmask,
-                                             DataflowShared* sh, unsigned char* wsm, const int lane, const int nw) {
+                                             const DataflowQueue& Q, unsigned char* wsm, const int lane, const int nw) {
     PFAST_TILE_SHAPE(SH);
+    // Items that become ready at a completion: a cluster's warps go on with them (the way through
+    // the ring costs several remote accesses; 3D gradient of 128 x 128 x 64 nodes, 64 sources:
+    // polish 29.4 -> 27.9 ms); a block's put them into the ring, which keeps the oldest first (there
+    // going on with the newest was 5 to 20 % slower).
+    constexpr bool kKeep = CL;
     const int total = 8 * A.ntiles;
     const int* dirty = A.dirty + (long long)inst * A.ntiles;
     int last_done = -1;
     unsigned long long idle_since = 0;
+    unsigned pause = 128;
+    unsigned e = kSlotEmpty;   // this lane's item
     for (;;) {
-        if (*(volatile int*)&sh->abort) return;   // a stalled block gives up (warp-uniform read)
-        // ---- take up to 32 ready items, about this warp's share of the ring
-        unsigned h = 0;
-        int n = 0;
-        if (lane == 0) {
-            for (int tries = 0; tries < 32; ++tries) {
-                const unsigned hh = *(volatile unsigned*)&sh->head, tt = *(volatile unsigned*)&sh->tail;
-                const int avail = (int)(tt - hh);
-                if (avail <= 0) break;
-                const int want = min(32, max(1, avail / nw));
-                if (atomicCAS(&sh->head, hh, hh + (unsigned)want) == hh) { h = hh; n = want; break; }
+        if (!__any_sync(0xffffffffu, e != kSlotEmpty)) {
+            // ---- take up to 32 ready items, about this warp's share of the ring
+            unsigned h = 0;
+            int n = 0, done = 0, stop = 0;
+            if (lane == 0) {
+                for (int tries = 0; tries < 32; ++tries) {
+                    const unsigned long long ht = *(volatile unsigned long long*)&Q.sh->head;
+                    const unsigned hh = (unsigned)ht, tt = (unsigned)(ht >> 32);
+                    const int avail = (int)(tt - hh);
+                    if (avail <= 0) break;
+                    const int want = min(32, max(1, avail / nw));
+                    if (atomicCAS(&Q.sh->head, hh, hh + (unsigned)want) == hh) { h = hh; n = want; break; }
+                }
+                if (n == 0) {
+                    const unsigned long long da = *(volatile unsigned long long*)&Q.sh->done;
+                    done = (int)(unsigned)da;
+                    stop = (int)(da >> 32);
+                }
+            }
+            n = __shfl_sync(0xffffffffu, n, 0);
+            h = __shfl_sync(0xffffffffu, h, 0);
+            if (n == 0) {
+                done = __shfl_sync(0xffffffffu, done, 0);
+                stop = __shfl_sync(0xffffffffu, stop, 0);
+                if (done >= total || stop) return;   // finished, or a stalled block gives up
+                if (lane == 0) {   // nothing ready while other warps work: wait, bounded
+                    const unsigned long long now = global_ns();
+                    if (done != last_done) { last_done = done; idle_since = now; }
+                    else if (now - idle_since > 2000000000ull) *(volatile int*)&Q.sh->abort = 1;
+                }
+                __nanosleep(pause);
+                pause = min(pause * 2u, 512u);
+                __syncwarp();
+                continue;
+            }
+            pause = 128;
+            if (lane < n) {
+                unsigned* slot = Q.slots + ((h + (unsigned)lane) & Q.qmask);
+                // the item's producer reserved this position before we took it: it is being written
+                for (int spin = 0; (e = atomicExch(slot, kSlotEmpty)) == kSlotEmpty; ++spin)
+                    if (spin > (1 << 22) || *(volatile int*)&Q.sh->abort) { *(volatile int*)&Q.sh->abort = 1; break; }
             }
         }
-        n = __shfl_sync(0xffffffffu, n, 0);
-        h = __shfl_sync(0xffffffffu, h, 0);
-        if (n == 0) {
-            const int d = *(volatile int*)&sh->done;
-            if (d >= total || *(volatile int*)&sh->abort) return;
-            if (lane == 0) {   // nothing ready while other warps work: wait, bounded
-                const unsigned long long now = global_ns();
-                if (d != last_done) { last_done = d; idle_since = now; }
-                else if (now - idle_since > 2000000000ull) *(volatile int*)&sh->abort = 1;
-            }
-            __nanosleep(128);
-            __syncwarp();
-            continue;
-        }
-        unsigned e = kSlotEmpty;
-        if (lane < n) {
-            unsigned* slot = slots + ((h + (unsigned)lane) & qmask);
-            // the item's producer reserved this position before we took it: it is being written
-            for (int spin = 0; (e = atomicExch(slot, kSlotEmpty)) == kSlotEmpty; ++spin)
-                if (spin > (1 << 22) || *(volatile int*)&sh->abort) { *(volatile int*)&sh->abort = 1; break; }
-        }
-        __threadfence_block();
+        df_fence<CL>();
         const bool have = e != kSlotEmpty;
         const int x = (int)(e >> 3), o = (int)(e & 7u);
         int dm = 0;
@@ -1262,26 +1342,31 @@ __device__ __forceinline__ void df_iteration(const Sweep3Args& A, const int inst
         }
         const unsigned dmask = __ballot_sync(0xffffffffu, due);
         const int mine = dmask ? __ffs(dmask) - 1 : -1;
+        unsigned next = kSlotEmpty;
         int ncomp = 0;
         if (have && !due) {   // locked in this order: nothing to compute
-            df_complete(g, cnt, slots, qmask, sh, o, x);
+            next = df_complete<CL>(g, Q, o, x);
             ncomp = 1;
         }
-        if (due && lane != mine) df_push(slots, qmask, sh, e);   // for an idle warp
         if (mine >= 0) {
+            if (due && lane != mine) next = e;
+            if (next != kSlotEmpty) df_push(Q, next);   // for an idle warp
             const int ex = __shfl_sync(0xffffffffu, x, mine), eo = __shfl_sync(0xffffffffu, o, mine);
             const int edm = __shfl_sync(0xffffffffu, dm, mine);
             const int tj = ex % g.nbj, ti = (ex / g.nbj) % g.nbi, tk = ex / (g.nbj * g.nbi);
             process_tile<KIND, true, SH>(A, inst, ex, tk, ti, tj, eo, iter, edm, wsm, lane);
-            __threadfence_block();   // the tile's field and lock words before its dependents start
+            df_fence<CL>();   // the tile's field and lock words before its dependents start
             __syncwarp();
-            if (lane == 0) {
-                df_complete(g, cnt, slots, qmask, sh, eo, ex);
-                ++ncomp;
-            }
+            next = df_complete_warp<CL>(g, Q, eo, ex, lane);
+            if (lane == 0) ++ncomp;
         }
+        if constexpr (!kKeep) {
+            if (next != kSlotEmpty) df_push(Q, next);
+            next = kSlotEmpty;
+        }
+        e = next;
         const int c = __reduce_add_sync(0xffffffffu, ncomp);
-        if (lane == 0 && c) atomicAdd(&sh->done, c);
+        if (lane == 0 && c) atomicAdd(&Q.sh->done, c);
     }
 }
 
@@ -1302,7 +1387,11 @@ __host__ __device__ constexpr int df_max_warps() {
 // instance items[q].y; the block copies that model's arguments into shared memory when it takes
 // the item, and the result goes to the model's `changed` array.  Otherwise the instances are
 // A.act[q] of the one grid in A and results go to result[].
-template <int KIND, bool MULTI, class SH>
+// CL: a thread-block cluster instead of a block solves an instance.  Its blocks share the queue
+// (counters, ring) of the first one through distributed shared memory, so that a survey with fewer
+// sources than SMs uses the SMs it would leave idle; the blocks of a cluster run at the same time
+// by construction, so their waits on one another end.
+template <int KIND, bool MULTI, bool CL, class SH>
 __global__ void __launch_bounds__(df_max_warps<KIND, SH>() * 32, 1) sweep3d_dataflow(const Sweep3Args A0,
                                                                       const Sweep3Args* __restrict__ models,
                                                                       const int2* __restrict__ items, const int nact,
@@ -1312,21 +1401,35 @@ __global__ void __launch_bounds__(df_max_warps<KIND, SH>() * 32, 1) sweep3d_data
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ DataflowShared sh;
     constexpr bool kSelective = (KIND == kFwdPolish64 || KIND == kAdjPolish64);
-    const int nthr = blockDim.x, nw = nthr >> 5;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int rank = 0, csize = 1;
+    if constexpr (CL) {
+        rank = (int)cg::this_cluster().block_rank();
+        csize = (int)cg::this_cluster().num_blocks();
+    }
+    const int nthr = blockDim.x, nw = (nthr >> 5) * csize;
+    const int cthr = rank * nthr + threadIdx.x, cnthr = csize * nthr;   // threads of the cluster
+    auto sync = [&]() {
+        if constexpr (CL) cg::this_cluster().sync();
+        else __syncthreads();
+    };
     unsigned char* wsm = smem_raw + warp * warp_smem_bytes<KIND, SH, true>();
     // after the warps' boxes: (MULTI: the current model's arguments,) the counters, the ring
-    unsigned char* dyn = smem_raw + nw * warp_smem_bytes<KIND, SH, true>();
+    unsigned char* dyn = smem_raw + (nthr >> 5) * warp_smem_bytes<KIND, SH, true>();
     Sweep3Args& s_args = *reinterpret_cast<Sweep3Args*>(dyn);
     unsigned* cnt = reinterpret_cast<unsigned*>(dyn + (MULTI ? kDfArgsBytes : 0));
-    const unsigned qmask = (unsigned)qcap - 1u;
+    DataflowQueue Q{cnt, cnt, (unsigned)qcap - 1u, &sh};
+    if constexpr (CL) {
+        Q.cnt = cg::this_cluster().map_shared_rank(cnt, 0);
+        Q.sh = cg::this_cluster().map_shared_rank(&sh, 0);
+    }
     int cur_model = -1;
     for (;;) {
-        if (threadIdx.x == 0) sh.item = atomicAdd(queue, 1);
-        __syncthreads();
-        const int item = sh.item;
-        __syncthreads();
-        if (item >= nact) return;   // block-uniform
+        if (cthr == 0) sh.item = atomicAdd(queue, 1);
+        sync();
+        const int item = Q.sh->item;
+        sync();
+        if (item >= nact) return;   // uniform over the block or cluster
         int inst;
         if constexpr (MULTI) {
             const int2 mi = items[item];
@@ -1343,7 +1446,7 @@ __global__ void __launch_bounds__(df_max_warps<KIND, SH>() * 32, 1) sweep3d_data
         }
         const Sweep3Args& A = MULTI ? s_args : A0;
         const int ntiles = A.ntiles, ncw = (ntiles + 3) >> 2;
-        unsigned* slots = cnt + ncw;
+        Q.slots = Q.cnt + ncw;
         const TileGrid3 g{A.nbk, A.nbi, A.nbj};
         int* diff = A.diff + (long long)inst * ntiles;
         const int* dirty = A.dirty + (long long)inst * ntiles;
@@ -1351,50 +1454,63 @@ __global__ void __launch_bounds__(df_max_warps<KIND, SH>() * 32, 1) sweep3d_data
         bool moved = true, aborted = false;
         while (it < maxiter) {
             // counters of orders 0 and 1, an empty ring, cleared per-tile change flags
-            for (int w = threadIdx.x; w < ncw; w += nthr) {
-                unsigned v = 0;
-                for (int b = 0; b < 4; ++b) {
-                    const int x = 4 * w + b;
-                    if (x < ntiles) v |= (unsigned)(dep_count(g, 0, x) | (dep_count(g, 1, x) << 4)) << (8 * b);
+            if (rank == 0) {
+                unsigned* slots = cnt + ncw;
+                for (int w = threadIdx.x; w < ncw; w += nthr) {
+                    unsigned v = 0;
+                    for (int b = 0; b < 4; ++b) {
+                        const int x = 4 * w + b;
+                        if (x < ntiles) v |= (unsigned)(dep_count(g, 0, x) | (dep_count(g, 1, x) << 4)) << (8 * b);
+                    }
+                    cnt[w] = v;
                 }
-                cnt[w] = v;
+                // the ring starts with (order 0, first tile)
+                for (int q = threadIdx.x; q < qcap; q += nthr) slots[q] = q ? kSlotEmpty : (unsigned)first_tile(g) << 3;
+                if (threadIdx.x == 0) {
+                    sh.head = 0;
+                    sh.tail = 1;
+                    sh.done = 0;
+                    sh.abort = 0;
+                    sh.flags[it & 1] = 0;
+                }
             }
-            for (int q = threadIdx.x; q < qcap; q += nthr) slots[q] = kSlotEmpty;
-            for (int t = threadIdx.x; t < ntiles; t += nthr) diff[t] = 0;
-            if (threadIdx.x == 0) {
-                sh.head = 0;
-                sh.tail = 1;
-                sh.done = 0;
-                sh.abort = 0;
-            }
-            __syncthreads();
-            if (threadIdx.x == 0) slots[0] = (unsigned)first_tile(g) << 3;   // (order 0, first tile)
-            __syncthreads();
-            df_iteration<KIND, SH>(A, inst, it, g, cnt, slots, qmask, &sh, wsm, lane, nw);
-            __syncthreads();
-            if (sh.abort) { aborted = true; break; }   // block-uniform
+            for (int t = cthr; t < ntiles; t += cnthr) diff[t] = 0;
+            sync();
+            df_iteration<KIND, CL, SH>(A, inst, it, g, Q, wsm, lane, nw);
+            sync();
+            if (*(volatile int*)&Q.sh->abort) aborted = true;   // uniform: written before the barrier
             // convergence: some tile moved in this iteration / some tile still due in some order
             int any = 0, due = 0;
-            for (int t = threadIdx.x; t < ntiles; t += nthr) {
+            for (int t = cthr; t < ntiles; t += cnthr) {
                 any |= __ldcg(diff + t);
                 const int dm = __ldcg(dirty + t);
                 due |= (kSelective ? (dm & (dm >> 8)) : dm) & 0xff;
             }
             any = __syncthreads_or(any);
             due = __syncthreads_or(due);
+            if constexpr (CL) {
+                int* fl = &Q.sh->flags[it & 1];   // the next iteration clears the other word
+                if (threadIdx.x == 0 && (any || due)) atomicOr(fl, (any ? 1 : 0) | (due ? 2 : 0));
+                sync();
+                const int f = *(volatile int*)fl;
+                any = f & 1;
+                due = f & 2;
+            }
+            if (aborted) break;
             ++it;
             if (!any) { moved = false; break; }
             // moved, but every tile is a fixed point of its update: the next iteration would
             // change nothing and pass the test; it is counted without running
             if (!due && it < maxiter) { ++it; moved = false; break; }
         }
-        if (threadIdx.x == 0) {
+        if (cthr == 0) {
             int* res = MULTI ? A.changed : result;
             res[inst] = it | (moved ? (1 << 30) : 0) | (aborted ? (1 << 29) : 0);
         }
         if (aborted) {
-            if (threadIdx.x == 0) atomicOr(queue + 1, 1);   // the host reports the stall
-            return;                                        // block-uniform
+            if (cthr == 0) atomicOr(queue + 1, 1);   // the host reports the stall
+            sync();   // no block leaves while another may still read its queue words
+            return;   // uniform
         }
     }
 }
@@ -1527,8 +1643,14 @@ pfast_status launch_one(const Sweep3Args& a, int d0, int tiles, int nact, cudaSt
 }
 
 template <int KIND, class SH>
-pfast_status dataflow_shape_k(int ntiles, int nact, bool multi, int* warps, int* blocks) {
-    static std::map<std::tuple<int, int, int, bool>, std::pair<int, int>> cache;   // (device, ntiles, nact, multi)
+const void* dataflow_fn(bool multi, bool cluster) {
+    return cluster ? (multi ? (const void*)sweep3d_dataflow<KIND, true, true, SH> : (const void*)sweep3d_dataflow<KIND, false, true, SH>)
+                   : (multi ? (const void*)sweep3d_dataflow<KIND, true, false, SH> : (const void*)sweep3d_dataflow<KIND, false, false, SH>);
+}
+
+template <int KIND, class SH>
+pfast_status dataflow_shape_k(int ntiles, int nact, bool multi, DataflowShape* out) {
+    static std::map<std::tuple<int, int, int, bool>, DataflowShape> cache;   // (device, ntiles, nact, multi)
     static std::mutex mu;
     int dev = 0, sms = 0, smem_max = 0;
     PFAST_CUDA_TRY(cudaGetDevice(&dev));
@@ -1536,57 +1658,84 @@ pfast_status dataflow_shape_k(int ntiles, int nact, bool multi, int* warps, int*
         std::lock_guard<std::mutex> lk(mu);
         auto it = cache.find(std::make_tuple(dev, ntiles, nact, multi));
         if (it != cache.end()) {
-            *warps = it->second.first;
-            *blocks = it->second.second;
+            *out = it->second;
             return PFAST_OK;
         }
     }
     PFAST_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     PFAST_CUDA_TRY(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     const long long room = (long long)smem_max - 256 - (long long)dataflow_extra_bytes(ntiles, multi);
-    const int w = (int)std::min<long long>(df_max_warps<KIND, SH>(), room / warp_smem_bytes<KIND, SH, true>());
-    if (ntiles > kDataflowMaxTiles || w < 1) {
-        *warps = 0;
-        *blocks = 0;
-        return PFAST_OK;
+    const int wmax = (int)std::min<long long>(df_max_warps<KIND, SH>(), room / warp_smem_bytes<KIND, SH, true>());
+    *out = DataflowShape();
+    if (ntiles > kDataflowMaxTiles || wmax < 1) return PFAST_OK;
+    for (bool cluster : {false, true}) {
+        // the opt-in maximum (less the kernel's static shared memory), not this grid's size: a cached
+        // shape of a larger grid launches later with more than a smaller grid's call would allow
+        const void* fn = dataflow_fn<KIND, SH>(multi, cluster);
+        cudaFuncAttributes fa;
+        PFAST_CUDA_TRY(cudaFuncGetAttributes(&fa, fn));
+        PFAST_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            smem_max - (int)fa.sharedSizeBytes));
+        if (cluster) PFAST_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     }
-    const size_t smem = (size_t)w * warp_smem_bytes<KIND, SH, true>() + dataflow_extra_bytes(ntiles, multi);
-    auto fn = multi ? sweep3d_dataflow<KIND, true, SH> : sweep3d_dataflow<KIND, false, SH>;
-    // the opt-in maximum (less the kernel's static shared memory), not this grid's size: a cached
-    // shape of a larger grid launches later with more than a smaller grid's call would allow
-    cudaFuncAttributes fa;
-    PFAST_CUDA_TRY(cudaFuncGetAttributes(&fa, fn));
-    PFAST_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        smem_max - (int)fa.sharedSizeBytes));
-    int per_sm = 0;
-    PFAST_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, w * 32, smem));
-    *warps = w;
-    *blocks = std::max(1, std::min(nact, std::max(1, per_sm) * sms));
+    auto smem_of = [&](int w) { return (size_t)w * warp_smem_bytes<KIND, SH, true>() + dataflow_extra_bytes(ntiles, multi); };
+    // the largest cluster size at which every instance has a cluster of its own at the same time
+    for (int cs = kMaxCluster; cs > 1 && !out->warps; cs /= 2) {
+        constexpr bool kPlain = KIND == kFwdPlain64 || KIND == kAdjPlain64;
+        if (!cluster_wanted(cs, kPlain, nact, ntiles, sms)) continue;
+        const int w = std::min(wmax, cluster_warps(cs, kPlain));
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute at = {};
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = cs;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cfg.gridDim = dim3(cs);
+        cfg.blockDim = dim3(w * 32);
+        cfg.dynamicSmemBytes = smem_of(w);
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        int resident = 0;
+        if (cudaOccupancyMaxActiveClusters(&resident, dataflow_fn<KIND, SH>(multi, true), &cfg) != cudaSuccess) {
+            cudaGetLastError();   // not available at this size: not used
+            continue;
+        }
+        if (resident < nact) continue;
+        out->warps = w;
+        out->cluster = cs;
+        out->blocks = nact * cs;
+    }
+    if (!out->warps) {
+        int per_sm = 0;
+        PFAST_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dataflow_fn<KIND, SH>(multi, false),
+                                                                     wmax * 32, smem_of(wmax)));
+        out->warps = wmax;
+        out->cluster = 1;
+        out->blocks = std::max(1, std::min(nact, std::max(1, per_sm) * sms));
+    }
     std::lock_guard<std::mutex> lk(mu);
-    cache[std::make_tuple(dev, ntiles, nact, multi)] = {*warps, *blocks};
+    cache[std::make_tuple(dev, ntiles, nact, multi)] = *out;
     return PFAST_OK;
 }
 
 template <int KIND, class SH>
-pfast_status launch_dataflow_k(const Sweep3Args& a, int nact, int maxiter, int* queue, int* result, int warps,
-                               int blocks, cudaStream_t st) {
-    const size_t smem = (size_t)warps * warp_smem_bytes<KIND, SH, true>() + dataflow_extra_bytes(a.ntiles, false);
-    sweep3d_dataflow<KIND, false, SH><<<blocks, warps * 32, smem, st>>>(a, nullptr, nullptr, nact, maxiter, queue,
-                                                                        result, dataflow_qcap(a.ntiles));
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return cuda_fail(e, "dataflow sweep launch", __FILE__, __LINE__);
-    return PFAST_OK;
-}
-
-template <int KIND, class SH>
-pfast_status launch_dataflow_multi_k(const Sweep3Args* models, const int2* items, int nitems, int max_ntiles,
-                                     int maxiter, int* queue, int warps, int blocks, cudaStream_t st) {
-    const size_t smem = (size_t)warps * warp_smem_bytes<KIND, SH, true>() + dataflow_extra_bytes(max_ntiles, true);
-    Sweep3Args unused;
-    std::memset(&unused, 0, sizeof(unused));
-    sweep3d_dataflow<KIND, true, SH><<<blocks, warps * 32, smem, st>>>(unused, models, items, nitems, maxiter, queue,
-                                                                       nullptr, dataflow_qcap(max_ntiles));
-    cudaError_t e = cudaGetLastError();
+pfast_status launch_dataflow_any(const Sweep3Args& a, const Sweep3Args* models, const int2* items, int nact, int ntiles,
+                                 int maxiter, int* queue, int* result, const DataflowShape& ds, cudaStream_t st) {
+    const bool multi = models != nullptr;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = ds.cluster;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.gridDim = dim3(ds.blocks);
+    cfg.blockDim = dim3(ds.warps * 32);
+    cfg.dynamicSmemBytes = (size_t)ds.warps * warp_smem_bytes<KIND, SH, true>() + dataflow_extra_bytes(ntiles, multi);
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = ds.cluster > 1 ? 1 : 0;
+    int qcap = dataflow_qcap(ntiles);
+    void* args[] = {(void*)&a, (void*)&models, (void*)&items, (void*)&nact, (void*)&maxiter, (void*)&queue,
+                    (void*)&result, (void*)&qcap};
+    const cudaError_t e = cudaLaunchKernelExC(&cfg, dataflow_fn<KIND, SH>(multi, ds.cluster > 1), args);
     if (e != cudaSuccess) return cuda_fail(e, "dataflow sweep launch", __FILE__, __LINE__);
     return PFAST_OK;
 }
@@ -1613,21 +1762,23 @@ pfast_status ShapeLaunchers<SH>::sweep(int kind, const Sweep3Args& a, int d0, in
 
 template <class SH>
 pfast_status ShapeLaunchers<SH>::dataflow(int kind, const Sweep3Args& a, int nact, int maxiter, int* queue,
-                                          int* result, int warps, int blocks, cudaStream_t st) {
-    PFAST_KIND_SWITCH(kind, (launch_dataflow_k<K, SH>(a, nact, maxiter, queue, result, warps, blocks, st)));
+                                          int* result, const DataflowShape& ds, cudaStream_t st) {
+    PFAST_KIND_SWITCH(kind, (launch_dataflow_any<K, SH>(a, nullptr, nullptr, nact, a.ntiles, maxiter, queue, result, ds, st)));
 }
 
 template <class SH>
 pfast_status ShapeLaunchers<SH>::dataflow_multi(int kind, const Sweep3Args* models, const int2* items, int nitems,
-                                                int max_ntiles, int maxiter, int* queue, int warps, int blocks,
+                                                int max_ntiles, int maxiter, int* queue, const DataflowShape& ds,
                                                 cudaStream_t st) {
-    PFAST_KIND_SWITCH(kind, (launch_dataflow_multi_k<K, SH>(models, items, nitems, max_ntiles, maxiter, queue, warps,
-                                                             blocks, st)));
+    Sweep3Args unused;
+    std::memset(&unused, 0, sizeof(unused));
+    PFAST_KIND_SWITCH(kind, (launch_dataflow_any<K, SH>(unused, models, items, nitems, max_ntiles, maxiter, queue, nullptr,
+                                                        ds, st)));
 }
 
 template <class SH>
-pfast_status ShapeLaunchers<SH>::dataflow_shape(int kind, int ntiles, int nact, bool multi, int* warps, int* blocks) {
-    PFAST_KIND_SWITCH(kind, (dataflow_shape_k<K, SH>(ntiles, nact, multi, warps, blocks)));
+pfast_status ShapeLaunchers<SH>::dataflow_shape(int kind, int ntiles, int nact, bool multi, DataflowShape* out) {
+    PFAST_KIND_SWITCH(kind, (dataflow_shape_k<K, SH>(ntiles, nact, multi, out)));
 }
 
 template <class SH>

@@ -55,4 +55,58 @@ inline int tune_pick(const TuneEntry* e, unsigned allowed, int nact, int sms) {
     return 0;
 }
 
+// The dataflow kernel solves an instance with one block, or with a cluster of cs = 2..16 blocks that
+// share its queue, where the instances alone would leave SMs idle.  A cluster size is wanted
+// while the clusters need about one block per SM (the hardware packs the blocks of a cluster
+// densely, so beyond that some SMs hold several and others none) and the grid has tiles for them.
+// Measured (ms of a mixed gradient of 128 x 128 x 64 nodes, blocks per source): 64 sources 95 (1), 81
+// (2); 40 sources 71 (2), 70 (4); 100 sources 99 (1), 103 (2); plain, 96 x 96 x 48: 16 sources 602
+// (1), 331 (2), 202 (4), 175 (8), 287 (16); 40 sources 331 (2), 299 (4).
+constexpr int kMaxCluster = 16;
+
+inline bool cluster_wanted(int cs, bool plain, int nact, int ntiles, int sms) {
+    return 10LL * nact * cs <= (plain ? 11LL : 13LL) * sms && ntiles >= 8 * cs;
+}
+
+// Warps per block of a cluster.  Few: the ready tiles of a source are few as well, and what
+// bounds them is the latency of one tile, so they should lie on different SM sub-partitions, and
+// idle warps only poll the queue.  The plain kinds saturate a sub-partition's FP64 pipe with one warp.
+// Measured (ms; warps per block): one shot of 128 x 128 x 64 nodes, plain, 16 blocks: 117 (2),
+// 88 (4), 102 (6), 171 (11, all that fit); 16 sources of 96 x 96 x 48, plain gradient, 8 blocks: 208
+// (2), 175 (4), 235 (6), 361 (11); 24 sources of 155 x 75 x 101, mixed forward, 8 blocks: 72 (2),
+// 49 (4), 48 (6), 54 (8); 9 sources of 90 x 71 x 53, mixed gradient, 16 blocks: 40.1 (2), 39.9 (4),
+// 41.3 (6); 64 sources of 128 x 128 x 64, mixed gradient, 2 blocks: 97 (8), 83 (12), 81 (24).
+inline int cluster_warps(int cs, bool plain) {
+    if (plain || cs >= 8) return 4;
+    return cs >= 4 ? 6 : 24;
+}
+
+// The candidate of a phase that has not been timed, among `allowed` (tune_allowed): the dataflow
+// kernel, except where one launch per tile diagonal is ahead: the plain kinds with one block per
+// instance and fewer instances than SMs (100 sources of 96 x 96 x 48: 566 against 706 ms; 200 sources
+// 880 against 722), and the FP32 bulk kinds with one block per instance where a diagonal
+// holds many tiles (256 sources of 256 x 256 x 128, 30,000 tiles a diagonal: forward 193 against 214 ms;
+// 300 sources of 128 x 128 x 64, 9,000: 30 against 26).  cluster: blocks per instance of the dataflow
+// kernel; plain / fp32: the phase's kind (neither: polish).
+inline int untuned_pick(unsigned allowed, bool plain, bool fp32, int cluster, int nact, long long ntiles, int ndiag,
+                        int sms) {
+    bool dataflow = true;
+    if (cluster <= 1) {
+        if (plain) dataflow = nact >= sms;
+        if (fp32) dataflow = ntiles * nact < 16384LL * ndiag;
+    }
+    const int order[2][kTuneCandidates] = {{0, 1, 2, 3, 4, 5}, {2, 3, 4, 5, 0, 1}};
+    for (int c : order[dataflow])
+        if (allowed >> c & 1) return c;
+    return 0;
+}
+
+// Whether every allowed candidate has been timed (tune_pick then takes the fastest).
+inline bool tune_complete(const TuneEntry* e, unsigned allowed) {
+    if (!e) return false;
+    for (int c = 0; c < kTuneCandidates; ++c)
+        if ((allowed >> c & 1) && e->n[c] == 0) return false;
+    return true;
+}
+
 }  // namespace pfast
