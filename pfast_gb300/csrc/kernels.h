@@ -81,10 +81,11 @@ pfast_status launch_seed_tiles3(int kind, const Sweep3Args& a, int nact, cudaStr
 // (every block reads a.act[blockIdx.y] before it tests whether its instance is still active).
 pfast_status launch_sweep3(int kind, const Sweep3Args& a, int d0, int tiles, int nact, cudaStream_t st);
 // Launch shape of the dataflow sweep kernel: warps per block (as many as shared memory holds; 0
-// when the grid does not fit), blocks per instance (a thread-block cluster when > 1) and resident
-// blocks.
+// when the grid does not fit), blocks per instance (a thread-block cluster when > 1), resident
+// blocks, where a warp keeps its tile (kernels3d_tiles.cuh: kForm*) and a block's shared memory.
 struct DataflowShape {
-    int warps = 0, cluster = 1, blocks = 0;
+    int warps = 0, cluster = 1, blocks = 0, form = 0;
+    size_t smem = 0;
 };
 pfast_status dataflow_shape(int kind, int shape, int ntiles, int nact, DataflowShape* out, bool multi = false);
 // Dataflow sweep kernel (one launch per phase): blocks or clusters take the

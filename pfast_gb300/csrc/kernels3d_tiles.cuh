@@ -48,26 +48,34 @@ template <> struct Traits<kAdjPlain64>   { using Real = double; using Aux = doub
 template <> struct Traits<kAdjFast32>    { using Real = float;  using Aux = float;  static constexpr bool adj = true; };
 template <> struct Traits<kAdjPolish64>  { using Real = double; using Aux = double; static constexpr bool adj = true; };
 
-// Whether the adjoint's traveltime is read through register windows and warp shuffles
-// (FP64 kinds, whose two FP64 boxes would halve the resident warps) or staged as a halo
-// box like the field (FP32 bulk: a small box, and a coalesced load beats per-lane reads).
-template <int KIND>
-__host__ __device__ constexpr bool t_windows() {
-    return Traits<KIND>::adj && sizeof(typename Traits<KIND>::Aux) == 8;
-}
+// Where a warp keeps its tile.
+//   kFormBox      the field in a halo box in shared memory; the adjoint's traveltime in register
+//                 windows with warp shuffles (FP64 kinds, whose two FP64 boxes would halve the resident
+//                 warps) or in a second box (FP32 bulk: a small box, and a coalesced load beats per-lane
+//                 reads).  The per-diagonal launches; the dataflow kernel but for:
+//   kFormWindows  (polish kinds in the dataflow kernel) the field in register windows too: a lane holds
+//                 its pencil's new value at jf-1 and old values at jf .. jf+3 (loads issued three steps
+//                 ahead); the upstream lanes' new values and the downstream lanes' old values come by
+//                 warp shuffle, the face halo pencils from owner lanes, and each changed node is stored
+//                 as it is updated.  The warp then needs no shared memory, so a block holds 24 (forward)
+//                 or 16 (adjoint) warps instead of 11, but a step takes 355 / 442 instructions instead
+//                 of 247 / 400 (ncu, warp instructions per tile and step).  For the forward with one
+//                 block per source on large grids, whose many ready tiles keep 24 warps busy (256 sources
+//                 of 256 x 256 x 128, 8192 tiles: 307 ms against 332 with boxes; 300 sources of 128 x 128 x 64,
+//                 1024 tiles: 50.5 against 43.1), for the adjoint also up to two blocks per source.
+//   kFormBoxes    (adjoint polish in clusters of four blocks or more) field and traveltime in boxes.
+// Elsewhere the latency of a tile bounds the polish, and the boxes are ahead: forward polish of 24
+// sources of 155 x 75 x 101 nodes 32.3 -> 25.3 ms, 64 of 128 x 128 x 64 26.9 -> 21.9, 9 of 90 x 71 x 53
+// 13.9 -> 9.9; adjoint polish of the 9 sources 14.5 -> 11.6 (of the 64: 27.9 -> 30.9, not taken).
+constexpr int kFormBox = 0, kFormWindows = 1, kFormBoxes = 2;
 
-// Whether the field itself is kept in register windows instead of a shared-memory halo box
-// (forward polish in the dataflow kernel, COHERENT).  A lane holds its pencil's new value at
-// jf-1 and old values at jf .. jf+3 (loads issued three steps ahead); the upstream lanes' new
-// values and the downstream lanes' old values come by warp shuffle, the face halo pencils from
-// owner lanes, and each changed node is stored as it is updated.  The warp then needs no shared
-// memory, so a dataflow block holds 24 (forward) or 16 (adjoint) warps instead of 11 boxes of
-// 17 KB (3D gradient workload: forward polish 167 -> 151 ms, adjoint polish 155 -> 125 ms).
-// The per-diagonal launches keep the box: with windows their forward polish ran slower
-// (159 -> 179 ms).
-template <int KIND, bool COHERENT>
+template <int KIND, int FORM>
+__host__ __device__ constexpr bool t_windows() {
+    return Traits<KIND>::adj && sizeof(typename Traits<KIND>::Aux) == 8 && FORM != kFormBoxes;
+}
+template <int KIND, int FORM>
 __host__ __device__ constexpr bool u_windows() {
-    return (KIND == kFwdPolish64 || KIND == kAdjPolish64) && COHERENT;
+    return FORM == kFormWindows;
 }
 
 // Shared memory per warp: the field's halo box, plus the FP32 bulk adjoint's traveltime
@@ -85,12 +93,12 @@ __host__ __device__ constexpr bool stage_slowness() {
     return KIND == kFwdFast32;
 }
 
-template <int KIND, class SH, bool COHERENT = false>
+template <int KIND, class SH, int FORM = kFormBox>
 __host__ __device__ constexpr int warp_smem_bytes() {
     using T = Traits<KIND>;
-    if (u_windows<KIND, COHERENT>()) return 16;   // no box
+    if (u_windows<KIND, FORM>()) return 16;   // no box
     return int(SH::HK * SH::PS * sizeof(typename T::Real) +
-               (T::adj && !t_windows<KIND>() ? SH::HK * SH::PS * sizeof(typename T::Aux) : 0) +
+               (T::adj && !t_windows<KIND, FORM>() ? SH::HK * SH::PS * sizeof(typename T::Aux) : 0) +
                (stage_slowness<KIND>() ? SH::TK * SH::SPS * sizeof(typename T::Aux) : 0));
 }
 
@@ -678,7 +686,7 @@ __device__ __forceinline__ bool tile_due(int dm, int dir) {
 // (dataflow schedule), so it is read through L2 instead of the read-only path.
 // The box is in the flipped coordinates of order dir (see load_box); the lanes (kf, if) walk
 // their pencils jf = 0..ej-1 so that step t updates the flipped hyperplane kf+if+jf = t.
-template <int KIND, bool COHERENT, class SH>
+template <int KIND, bool COHERENT, int FORM, class SH>
 __device__ __forceinline__ void process_tile(const Sweep3Args& A, const int inst, const int tid, const int tk,
                                              const int ti, const int tj, const int dir, const int iter,
                                              const int dmask, unsigned char* wsm, const int lane) {
@@ -714,8 +722,8 @@ __device__ __forceinline__ void process_tile(const Sweep3Args& A, const int inst
 
     Real* box = reinterpret_cast<Real*>(wsm);
     Aux* aux = reinterpret_cast<Aux*>(reinterpret_cast<unsigned char*>(box) + HK * PS * sizeof(Real));
-    constexpr bool TWIN = t_windows<KIND>();
-    constexpr bool UWIN = u_windows<KIND, COHERENT>();
+    constexpr bool TWIN = t_windows<KIND, FORM>();
+    constexpr bool UWIN = u_windows<KIND, FORM>();
     Real* fld = reinterpret_cast<Real*>(A.field) + inst * A.fstride;
 
     // ---- stage the field halo box (out-of-grid: +inf for the forward so that the
@@ -1127,7 +1135,7 @@ __global__ void __launch_bounds__(kWarps3 * 32) sweep3d_kernel(const Sweep3Args 
     const int dm = __ldcg(A.dirty + (long long)inst * A.ntiles + tid);
     if (!tile_due<KIND>(dm, A.dir)) return;   // locked tile for this order (warp-uniform)
     __syncwarp();
-    process_tile<KIND, false, SH>(A, inst, tid, tk, ti, tj, A.dir, iter, dm, smem_raw + warp * warp_smem_bytes<KIND, SH>(),
+    process_tile<KIND, false, kFormBox, SH>(A, inst, tid, tk, ti, tj, A.dir, iter, dm, smem_raw + warp * warp_smem_bytes<KIND, SH>(),
                               lane);
 }
 
@@ -1272,7 +1280,7 @@ __device__ __forceinline__ unsigned df_complete_warp(const TileGrid3& g, const D
 }
 
 // The warps' part of one outer iteration of instance inst; nw: warps of the block or cluster.
-template <int KIND, bool CL, class SH>
+template <int KIND, bool CL, int FORM, class SH>
 __device__ __forceinline__ void df_iteration(const Sweep3Args& A, const int inst, const int iter, const TileGrid3& g,
                                              const DataflowQueue& Q, unsigned char* wsm, const int lane, const int nw) {
     PFAST_TILE_SHAPE(SH);
@@ -1354,7 +1362,7 @@ __device__ __forceinline__ void df_iteration(const Sweep3Args& A, const int inst
             const int ex = __shfl_sync(0xffffffffu, x, mine), eo = __shfl_sync(0xffffffffu, o, mine);
             const int edm = __shfl_sync(0xffffffffu, dm, mine);
             const int tj = ex % g.nbj, ti = (ex / g.nbj) % g.nbi, tk = ex / (g.nbj * g.nbi);
-            process_tile<KIND, true, SH>(A, inst, ex, tk, ti, tj, eo, iter, edm, wsm, lane);
+            process_tile<KIND, true, FORM, SH>(A, inst, ex, tk, ti, tj, eo, iter, edm, wsm, lane);
             df_fence<CL>();   // the tile's field and lock words before its dependents start
             __syncwarp();
             next = df_complete_warp<CL>(g, Q, eo, ex, lane);
@@ -1375,12 +1383,10 @@ __device__ __forceinline__ void df_iteration(const Sweep3Args& A, const int inst
 // thread follows the block size.  The register-window kinds use no box: 24 warps for the
 // forward polish (85 registers a thread; 20 warps measured 2 % slower), 16 for the adjoint
 // polish, which also keeps the traveltime windows (128 registers; 20 warps measured 3 % slower).
-template <int KIND, class SH>
+template <int KIND, int FORM, class SH>
 __host__ __device__ constexpr int df_max_warps() {
-    return u_windows<KIND, true>() ? (KIND == kAdjPolish64 ? 16 : 24)
-           : (227 * 1024 - 256 - 40960) / warp_smem_bytes<KIND, SH, true>() < 24
-               ? (227 * 1024 - 256 - 40960) / warp_smem_bytes<KIND, SH, true>()
-               : 24;
+    constexpr int fit = (227 * 1024 - 256 - 40960) / warp_smem_bytes<KIND, SH, FORM>();
+    return u_windows<KIND, FORM>() ? (KIND == kAdjPolish64 ? 16 : 24) : (fit < 24 ? fit : 24);
 }
 
 // MULTI: instances of several grids in one launch.  Item q of the queue is models[items[q].x]'s
@@ -1391,8 +1397,8 @@ __host__ __device__ constexpr int df_max_warps() {
 // (counters, ring) of the first one through distributed shared memory, so that a survey with fewer
 // sources than SMs uses the SMs it would leave idle; the blocks of a cluster run at the same time
 // by construction, so their waits on one another end.
-template <int KIND, bool MULTI, bool CL, class SH>
-__global__ void __launch_bounds__(df_max_warps<KIND, SH>() * 32, 1) sweep3d_dataflow(const Sweep3Args A0,
+template <int KIND, bool MULTI, bool CL, int FORM, class SH>
+__global__ void __launch_bounds__(df_max_warps<KIND, FORM, SH>() * 32, 1) sweep3d_dataflow(const Sweep3Args A0,
                                                                       const Sweep3Args* __restrict__ models,
                                                                       const int2* __restrict__ items, const int nact,
                                                                       const int maxiter, int* __restrict__ queue,
@@ -1413,9 +1419,9 @@ __global__ void __launch_bounds__(df_max_warps<KIND, SH>() * 32, 1) sweep3d_data
         if constexpr (CL) cg::this_cluster().sync();
         else __syncthreads();
     };
-    unsigned char* wsm = smem_raw + warp * warp_smem_bytes<KIND, SH, true>();
+    unsigned char* wsm = smem_raw + warp * warp_smem_bytes<KIND, SH, FORM>();
     // after the warps' boxes: (MULTI: the current model's arguments,) the counters, the ring
-    unsigned char* dyn = smem_raw + (nthr >> 5) * warp_smem_bytes<KIND, SH, true>();
+    unsigned char* dyn = smem_raw + (nthr >> 5) * warp_smem_bytes<KIND, SH, FORM>();
     Sweep3Args& s_args = *reinterpret_cast<Sweep3Args*>(dyn);
     unsigned* cnt = reinterpret_cast<unsigned*>(dyn + (MULTI ? kDfArgsBytes : 0));
     DataflowQueue Q{cnt, cnt, (unsigned)qcap - 1u, &sh};
@@ -1476,7 +1482,7 @@ __global__ void __launch_bounds__(df_max_warps<KIND, SH>() * 32, 1) sweep3d_data
             }
             for (int t = cthr; t < ntiles; t += cnthr) diff[t] = 0;
             sync();
-            df_iteration<KIND, CL, SH>(A, inst, it, g, Q, wsm, lane, nw);
+            df_iteration<KIND, CL, FORM, SH>(A, inst, it, g, Q, wsm, lane, nw);
             sync();
             if (*(volatile int*)&Q.sh->abort) aborted = true;   // uniform: written before the barrier
             // convergence: some tile moved in this iteration / some tile still due in some order
@@ -1642,10 +1648,48 @@ pfast_status launch_one(const Sweep3Args& a, int d0, int tiles, int nact, cudaSt
     return PFAST_OK;
 }
 
+// The form of a dataflow phase: cluster blocks per source, grids of (up to) ntiles tiles.
+template <int KIND>
+constexpr int dataflow_form(int cluster, int ntiles) {
+    if (KIND == kFwdPolish64) return cluster == 1 && ntiles >= 4096 ? kFormWindows : kFormBox;
+    if (KIND == kAdjPolish64) return cluster >= 4 ? kFormBoxes : kFormWindows;
+    return kFormBox;
+}
+
+template <int KIND, int FORM, class SH>
+const void* dataflow_fn_of(bool multi, bool cluster) {
+    // the forms that occur (dataflow_form)
+    if constexpr (FORM == kFormBoxes)
+        return multi ? (const void*)sweep3d_dataflow<KIND, true, true, FORM, SH> : (const void*)sweep3d_dataflow<KIND, false, true, FORM, SH>;
+    else if constexpr (FORM == kFormWindows && KIND == kFwdPolish64)
+        return multi ? (const void*)sweep3d_dataflow<KIND, true, false, FORM, SH> : (const void*)sweep3d_dataflow<KIND, false, false, FORM, SH>;
+    else
+        return cluster ? (multi ? (const void*)sweep3d_dataflow<KIND, true, true, FORM, SH> : (const void*)sweep3d_dataflow<KIND, false, true, FORM, SH>)
+                       : (multi ? (const void*)sweep3d_dataflow<KIND, true, false, FORM, SH> : (const void*)sweep3d_dataflow<KIND, false, false, FORM, SH>);
+}
+
+// A dataflow kernel: its function, the warps a block holds at most and the bytes of a warp.
+struct DataflowKernel {
+    const void* fn;
+    int max_warps, warp_bytes;
+};
+
 template <int KIND, class SH>
-const void* dataflow_fn(bool multi, bool cluster) {
-    return cluster ? (multi ? (const void*)sweep3d_dataflow<KIND, true, true, SH> : (const void*)sweep3d_dataflow<KIND, false, true, SH>)
-                   : (multi ? (const void*)sweep3d_dataflow<KIND, true, false, SH> : (const void*)sweep3d_dataflow<KIND, false, false, SH>);
+DataflowKernel dataflow_kernel(bool multi, bool cluster, int form) {
+    if constexpr (KIND == kAdjPolish64) {
+        if (form == kFormBoxes)
+            return {dataflow_fn_of<KIND, kFormBoxes, SH>(multi, cluster), df_max_warps<KIND, kFormBoxes, SH>(),
+                    warp_smem_bytes<KIND, SH, kFormBoxes>()};
+    }
+    if constexpr (KIND == kFwdPolish64 || KIND == kAdjPolish64) {
+        if (KIND == kAdjPolish64 || form == kFormWindows)
+            return {dataflow_fn_of<KIND, kFormWindows, SH>(multi, cluster), df_max_warps<KIND, kFormWindows, SH>(),
+                    warp_smem_bytes<KIND, SH, kFormWindows>()};
+    }
+    if constexpr (KIND != kAdjPolish64)
+        return {dataflow_fn_of<KIND, kFormBox, SH>(multi, cluster), df_max_warps<KIND, kFormBox, SH>(),
+                warp_smem_bytes<KIND, SH, kFormBox>()};
+    return {};
 }
 
 template <int KIND, class SH>
@@ -1665,52 +1709,51 @@ pfast_status dataflow_shape_k(int ntiles, int nact, bool multi, DataflowShape* o
     PFAST_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     PFAST_CUDA_TRY(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     const long long room = (long long)smem_max - 256 - (long long)dataflow_extra_bytes(ntiles, multi);
-    const int wmax = (int)std::min<long long>(df_max_warps<KIND, SH>(), room / warp_smem_bytes<KIND, SH, true>());
+    constexpr bool kPlain = KIND == kFwdPlain64 || KIND == kAdjPlain64;
     *out = DataflowShape();
-    if (ntiles > kDataflowMaxTiles || wmax < 1) return PFAST_OK;
-    for (bool cluster : {false, true}) {
+    // the largest cluster size at which every instance has a cluster of its own at the same time
+    for (int cs = kMaxCluster; cs >= 1 && !out->warps; cs /= 2) {
+        if (cs > 1 && !cluster_wanted(cs, kPlain, nact, ntiles, sms)) continue;
+        const int form = dataflow_form<KIND>(cs, ntiles);
+        const DataflowKernel k = dataflow_kernel<KIND, SH>(multi, cs > 1, form);
+        const int wmax = (int)std::min<long long>(k.max_warps, room / k.warp_bytes);
+        if (ntiles > kDataflowMaxTiles || wmax < 1) return PFAST_OK;
         // the opt-in maximum (less the kernel's static shared memory), not this grid's size: a cached
         // shape of a larger grid launches later with more than a smaller grid's call would allow
-        const void* fn = dataflow_fn<KIND, SH>(multi, cluster);
         cudaFuncAttributes fa;
-        PFAST_CUDA_TRY(cudaFuncGetAttributes(&fa, fn));
-        PFAST_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        PFAST_CUDA_TRY(cudaFuncGetAttributes(&fa, k.fn));
+        PFAST_CUDA_TRY(cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             smem_max - (int)fa.sharedSizeBytes));
-        if (cluster) PFAST_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    }
-    auto smem_of = [&](int w) { return (size_t)w * warp_smem_bytes<KIND, SH, true>() + dataflow_extra_bytes(ntiles, multi); };
-    // the largest cluster size at which every instance has a cluster of its own at the same time
-    for (int cs = kMaxCluster; cs > 1 && !out->warps; cs /= 2) {
-        constexpr bool kPlain = KIND == kFwdPlain64 || KIND == kAdjPlain64;
-        if (!cluster_wanted(cs, kPlain, nact, ntiles, sms)) continue;
-        const int w = std::min(wmax, cluster_warps(cs, kPlain));
-        cudaLaunchConfig_t cfg = {};
-        cudaLaunchAttribute at = {};
-        at.id = cudaLaunchAttributeClusterDimension;
-        at.val.clusterDim.x = cs;
-        at.val.clusterDim.y = at.val.clusterDim.z = 1;
-        cfg.gridDim = dim3(cs);
-        cfg.blockDim = dim3(w * 32);
-        cfg.dynamicSmemBytes = smem_of(w);
-        cfg.attrs = &at;
-        cfg.numAttrs = 1;
+        const int w = cs > 1 ? std::min(wmax, cluster_warps(cs, kPlain)) : wmax;
+        const size_t smem = (size_t)w * k.warp_bytes + dataflow_extra_bytes(ntiles, multi);
         int resident = 0;
-        if (cudaOccupancyMaxActiveClusters(&resident, dataflow_fn<KIND, SH>(multi, true), &cfg) != cudaSuccess) {
-            cudaGetLastError();   // not available at this size: not used
-            continue;
+        if (cs > 1) {
+            PFAST_CUDA_TRY(cudaFuncSetAttribute(k.fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+            cudaLaunchConfig_t cfg = {};
+            cudaLaunchAttribute at = {};
+            at.id = cudaLaunchAttributeClusterDimension;
+            at.val.clusterDim.x = cs;
+            at.val.clusterDim.y = at.val.clusterDim.z = 1;
+            cfg.gridDim = dim3(cs);
+            cfg.blockDim = dim3(w * 32);
+            cfg.dynamicSmemBytes = smem;
+            cfg.attrs = &at;
+            cfg.numAttrs = 1;
+            if (cudaOccupancyMaxActiveClusters(&resident, k.fn, &cfg) != cudaSuccess) {
+                cudaGetLastError();   // not available at this size: not used
+                continue;
+            }
+            if (resident < nact) continue;
+        } else {
+            int per_sm = 0;
+            PFAST_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k.fn, w * 32, smem));
+            resident = std::max(1, per_sm) * sms;
         }
-        if (resident < nact) continue;
         out->warps = w;
         out->cluster = cs;
-        out->blocks = nact * cs;
-    }
-    if (!out->warps) {
-        int per_sm = 0;
-        PFAST_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dataflow_fn<KIND, SH>(multi, false),
-                                                                     wmax * 32, smem_of(wmax)));
-        out->warps = wmax;
-        out->cluster = 1;
-        out->blocks = std::max(1, std::min(nact, std::max(1, per_sm) * sms));
+        out->blocks = std::max(1, std::min(nact, resident)) * cs;
+        out->form = form;
+        out->smem = smem;
     }
     std::lock_guard<std::mutex> lk(mu);
     cache[std::make_tuple(dev, ntiles, nact, multi)] = *out;
@@ -1728,14 +1771,14 @@ pfast_status launch_dataflow_any(const Sweep3Args& a, const Sweep3Args* models, 
     at.val.clusterDim.y = at.val.clusterDim.z = 1;
     cfg.gridDim = dim3(ds.blocks);
     cfg.blockDim = dim3(ds.warps * 32);
-    cfg.dynamicSmemBytes = (size_t)ds.warps * warp_smem_bytes<KIND, SH, true>() + dataflow_extra_bytes(ntiles, multi);
+    cfg.dynamicSmemBytes = ds.smem;
     cfg.stream = st;
     cfg.attrs = &at;
     cfg.numAttrs = ds.cluster > 1 ? 1 : 0;
     int qcap = dataflow_qcap(ntiles);
     void* args[] = {(void*)&a, (void*)&models, (void*)&items, (void*)&nact, (void*)&maxiter, (void*)&queue,
                     (void*)&result, (void*)&qcap};
-    const cudaError_t e = cudaLaunchKernelExC(&cfg, dataflow_fn<KIND, SH>(multi, ds.cluster > 1), args);
+    const cudaError_t e = cudaLaunchKernelExC(&cfg, dataflow_kernel<KIND, SH>(multi, ds.cluster > 1, ds.form).fn, args);
     if (e != cudaSuccess) return cuda_fail(e, "dataflow sweep launch", __FILE__, __LINE__);
     return PFAST_OK;
 }
