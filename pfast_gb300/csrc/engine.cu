@@ -87,7 +87,7 @@ void HostBuf::release() {
 std::vector<DevBuf*> ctx_buffers(pfast_ctx* ctx) {
     return {&ctx->s64,  &ctx->s32,  &ctx->sq64,     &ctx->T32,    &ctx->tflags,    &ctx->T64,   &ctx->L64,
             &ctx->scratch, &ctx->mask, &ctx->act,  &ctx->changed, &ctx->ee,     &ctx->need,    &ctx->misc,
-            &ctx->grad_tmp, &ctx->vp_tmp, &ctx->picks_tmp, &ctx->f2a, &ctx->f2b, &ctx->f2c, &ctx->work,
+            &ctx->grad_tmp, &ctx->vp_tmp, &ctx->picks_tmp, &ctx->f2a, &ctx->f2b, &ctx->work,
             &ctx->queue, &ctx->out_a, &ctx->out_b, &ctx->out_c, &ctx->dyn, &ctx->multi, &ctx->multi_meta, &ctx->sv_src, &ctx->sv_rec, &ctx->sv_nxyz,
             &ctx->sv_tobs, &ctx->sv_last};
 }

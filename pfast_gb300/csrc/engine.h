@@ -47,7 +47,7 @@ struct pfast_ctx {
     cudaStream_t stream = nullptr;
     // device work buffers (reused across calls)
     pfast::DevBuf s64, s32, sq64, T32, tflags, T64, L64, scratch, mask, act, changed, ee, need, misc, grad_tmp, vp_tmp, picks_tmp;
-    pfast::DevBuf f2a, f2b, f2c;       // 2D field buffers
+    pfast::DevBuf f2a, f2b;            // 2D field buffers
     pfast::HostBuf h_act, h_changed, h_ee, h_need, h_work;
     pfast::DevBuf work;                 // executed node updates per instance (sweep kernels)
     pfast::DevBuf queue;                // work counter of the persistent sweep kernel

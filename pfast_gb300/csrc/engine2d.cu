@@ -173,6 +173,45 @@ pfast_status run_sweeps2(pfast_ctx* ctx, Sweep2Args a, int kind, const DiagTable
     PFAST_TRY2(ctx->h_work.ensure(sizeof(unsigned long long) * ninst));
     a.work = ctx->work.as<unsigned long long>();
     PFAST_CUDA_TRY(cudaMemsetAsync(a.work, 0, sizeof(unsigned long long) * ninst, st));
+    // One launch per phase where the grid's strips fit a block (up to 512 rows); taller grids launch
+    // per tile diagonal.
+    if (!active.empty() && strips_fit(kind, a.nr, a.nc)) {
+        const int nact = (int)active.size();
+        PFAST_TRY2(ctx->act.ensure(sizeof(int) * 2 * ninst));
+        PFAST_TRY2(ctx->h_act.ensure(sizeof(int) * 2 * ninst));
+        PFAST_TRY2(ctx->queue.ensure(2 * sizeof(int)));
+        PFAST_TRY2(ctx->h_dyn.ensure(2 * sizeof(int)));
+        h_act = ctx->h_act.as<int>();
+        for (int k = 0; k < nact; ++k) {
+            h_act[k] = active[k];
+            h_act[ninst + k] = caps[active[k]];
+        }
+        a.act = ctx->act.as<int>();
+        if (kind == kAdjFast32) {   // the instances' FP32 fields and split traveltimes share their offsets
+            const long long n = (long long)a.nr * a.nc;
+            PFAST_TRY2(ctx->T32.ensure(2 * sizeof(float) * n * ninst));
+            PFAST_LAUNCH(ctx, launch_split_inst(static_cast<const double*>(a.aux), ctx->T32.p, a.aux_off, a.inst_off, n,
+                                                ninst, st));
+            a.aux = ctx->T32.p;
+            a.aux_off = a.inst_off;
+        }
+        int* hq = ctx->h_dyn.as<int>();
+        PFAST_CUDA_TRY(cudaMemcpyAsync(const_cast<int*>(a.act), h_act, sizeof(int) * 2 * ninst, cudaMemcpyHostToDevice, st));
+        PFAST_CUDA_TRY(cudaMemsetAsync(ctx->queue.p, 0, 2 * sizeof(int), st));
+        PFAST_LAUNCH(ctx, launch_sweep2_strips(kind, a, nact, a.act + ninst, ctx->queue.as<int>(), a.changed, st));
+        PFAST_CUDA_TRY(cudaMemcpyAsync(hq, ctx->queue.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
+        PFAST_CUDA_TRY(cudaMemcpyAsync(h_chg, a.changed, sizeof(int) * ninst, cudaMemcpyDeviceToHost, st));
+        PFAST_CUDA_TRY(cudaStreamSynchronize(st));
+        if (hq[1]) {
+            set_last_error("strip sweep: a block made no progress for two seconds (internal error)");
+            return PFAST_ERR_CUDA;
+        }
+        for (int q : active) {
+            iters[q] = h_chg[q] & 0xffffff;
+            if ((h_chg[q] >> 30) && not_conv) ++*not_conv;
+        }
+        active.clear();
+    }
     int it = 0;
     cudaGraphExec_t exec = nullptr;
     if (ctx->graphs && !active.empty()) {
@@ -542,54 +581,60 @@ pfast_status adjoint2d_batch(pfast_ctx* ctx, pfast_survey2d* sv, int b0, int nb,
     const long long mwords = (long long)sv->nr * wpr;
     cudaStream_t s = ctx->stream;
     double* F = ctx->f2a.as<double>();
-    PFAST_TRY2(ctx->f2b.ensure(sizeof(double) * N * 2 * nb));      // lamT, UR per source
-    PFAST_TRY2(ctx->f2c.ensure(sizeof(double) * N * nb));          // lambda of the current reflector
+    PFAST_TRY2(ctx->f2b.ensure(sizeof(double) * N * 3 * nb));      // lamT, UR per source; lambda of the current reflector
     PFAST_TRY2(ctx->mask.ensure(sizeof(unsigned) * mwords * 2 * nb));
     PFAST_TRY2(ctx->ee.ensure(sizeof(double) * 2 * nb));
     PFAST_TRY2(ctx->h_ee.ensure(sizeof(double) * 2 * nb));
     double* LB = ctx->f2b.as<double>();
-    double* LC = ctx->f2c.as<double>();
+    const long long LC = 2 * N * nb;   // offset of the current reflector's lambda
     PFAST_CUDA_TRY(cudaMemsetAsync(LB, 0, sizeof(double) * N * 2 * nb, s));
     PFAST_CUDA_TRY(cudaMemsetAsync(ctx->mask.p, 0, sizeof(unsigned) * mwords * 2 * nb, s));
     PFAST_CUDA_TRY(cudaMemsetAsync(ctx->ee.p, 0, sizeof(double) * 2 * nb, s));
     double* d_eeT = ctx->ee.as<double>();
     double* d_eeR = d_eeT + nb;
-    // transmission adjoint, one instance per source
-    InstTables T;
-    for (int b = 0; b < nb; ++b) {
-        T.off.push_back((long long)(2 * b) * N);
-        T.aux_off.push_back(((long long)b * slots) * N);
-        T.mask_off.push_back((long long)(2 * b) * mwords);
-        T.gsrc.push_back(b0 + b);
-        T.ir.push_back(-1);
-    }
-    std::vector<int> caps(nb, maxswp), iters;
-    if (do_t) PFAST_TRY2(adj_phase2(ctx, sv, LB, F, T, precision, caps, iters, d_eeT, st));
-    // reflection adjoints, reflector by reflector; the iteration counter and the
-    // receiver mask carry over between reflectors (src/RT_padjoint2d.h:385-466)
-    std::vector<int> count(nb, 0);
-    for (int ir = 0; do_r && ir < R; ++ir) {
-        PFAST_CUDA_TRY(cudaMemsetAsync(LC, 0, sizeof(double) * N * nb, s));
-        InstTables Rt;
-        for (int b = 0; b < nb; ++b) {
-            Rt.off.push_back((long long)b * N);
-            Rt.aux_off.push_back(((long long)b * slots + 1 + R + ir) * N);
-            Rt.mask_off.push_back((long long)(2 * b + 1) * mwords);
-            Rt.gsrc.push_back(b0 + b);
-            Rt.ir.push_back(ir);
-            caps[b] = std::max(0, maxswp - count[b]);
+    // Transmission adjoint, one instance per source, together with the first reflector's, which does
+    // not depend on it (601 x 201 nodes, 40 sources, one reflector: 40 blocks twice in a row left most
+    // of the SMs idle); then reflector by reflector: the iteration counter and the receiver mask
+    // carry over between reflectors (src/RT_padjoint2d.h:385-466).
+    std::vector<int> count(nb, 0), iters;
+    for (int ir = 0; ir < std::max(1, do_r ? R : 0); ++ir) {
+        InstTables t;
+        std::vector<int> caps;
+        const bool with_t = ir == 0 && do_t, with_r = do_r && R > 0;
+        if (with_t)
+            for (int b = 0; b < nb; ++b) {
+                t.off.push_back((long long)(2 * b) * N);
+                t.aux_off.push_back(((long long)b * slots) * N);
+                t.mask_off.push_back((long long)(2 * b) * mwords);
+                t.gsrc.push_back(b0 + b);
+                t.ir.push_back(-1);
+                caps.push_back(maxswp);
+            }
+        const int r0 = (int)caps.size();
+        if (with_r) {
+            PFAST_CUDA_TRY(cudaMemsetAsync(LB + LC, 0, sizeof(double) * N * nb, s));
+            for (int b = 0; b < nb; ++b) {
+                t.off.push_back(LC + (long long)b * N);
+                t.aux_off.push_back(((long long)b * slots + 1 + R + ir) * N);
+                t.mask_off.push_back((long long)(2 * b + 1) * mwords);
+                t.gsrc.push_back(b0 + b);
+                t.ir.push_back(ir);
+                caps.push_back(std::max(0, maxswp - count[b]));
+            }
         }
-        // bc2 adds into d_eeR[b] (one running misfit sum over the reflectors of a source)
-        PFAST_TRY2(adj_phase2(ctx, sv, LC, F, Rt, precision, caps, iters, d_eeR, st));
-        for (int b = 0; b < nb; ++b) count[b] += iters[b] + 1;
-        std::vector<long long> dof(nb), sof(nb);
-        for (int b = 0; b < nb; ++b) { dof[b] = (long long)(2 * b + 1) * N; sof[b] = (long long)b * N; }
+        // bc2 adds an instance's misfit into its word: d_eeT[b] / d_eeR[b] (one running sum over the
+        // reflectors of a source); the two arrays lie one after the other
+        PFAST_TRY2(adj_phase2(ctx, sv, LB, F, t, precision, caps, iters, with_t ? d_eeT : d_eeR, st));
+        if (!with_r) break;
+        for (int b = 0; b < nb; ++b) count[b] += iters[r0 + b] + 1;
         InstTables add;
-        add.off = dof;
-        add.aux_off = sof;
+        for (int b = 0; b < nb; ++b) {
+            add.off.push_back((long long)(2 * b + 1) * N);
+            add.aux_off.push_back(LC + (long long)b * N);
+        }
         InstDev ad;
         PFAST_TRY2(upload_inst(ctx, ctx->misc, add, ad));
-        PFAST_LAUNCH(ctx, launch_addto2(LB, ad.off, LC, ad.aux_off, N, nb, s));
+        PFAST_LAUNCH(ctx, launch_addto2(LB, ad.off, LB, ad.aux_off, N, nb, s));
     }
     PFAST_CUDA_TRY(cudaMemcpyAsync(ctx->h_ee.p, ctx->ee.p, sizeof(double) * 2 * nb, cudaMemcpyDeviceToHost, s));
     PFAST_CUDA_TRY(cudaStreamSynchronize(s));

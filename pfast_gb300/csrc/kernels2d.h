@@ -59,6 +59,16 @@ struct DiagTable2 {
 pfast_status build_diag_table2(int nr, int nc, DiagTable2& t);
 void free_diag_table2(DiagTable2& t);
 pfast_status launch_sweep2(int kind, const Sweep2Args& a, int d, int tiles, int nact, cudaStream_t st);
+// Strips schedule (one launch per phase, a block per instance): solves the nact instances of a.act,
+// instance a.act[k] with at most caps[k] outer iterations, all device arrays; queue[0] = queue[1] = 0
+// by the caller; result[inst] = iterations | 1 << 30 when not converged (queue[1] set if a block
+// stalled: an internal error).  Same results as the per-diagonal launches.
+// The FP32 bulk adjoint takes its traveltimes split (launch_split_inst) at aux + aux_off[q] float2.
+bool strips_fit(int kind, int nr, int nc);
+pfast_status launch_split_inst(const double* a, void* b, const long long* oa, const long long* ob, long long n, int ninst,
+                               cudaStream_t st);
+pfast_status launch_sweep2_strips(int kind, const Sweep2Args& a, int nact, const int* caps, int* queue, int* result,
+                                  cudaStream_t st);
 // Opt-in near-source start (not in the reference): in each instance q with a point source
 // (inst_src[q] >= 0), the nodes within `radius` nodes (Euclidean) get the straight-ray time
 // 0.5 (s_src + s_node) * distance; a down-going instance (inst_lim[q] >= 0) only above its

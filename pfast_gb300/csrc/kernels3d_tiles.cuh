@@ -256,7 +256,8 @@ __device__ __forceinline__ double adj3_plain(double T0, double Txp, double Txm, 
         adj_axis_exact(T0, Typ, Tym, Lyp, Lym, sp.ex.axis[1], ey, ny);
         adj_axis_exact(T0, Tzp, Tzm, Lzp, Lzm, sp.ex.axis[2], ez, nz);
         const double den = ex + ey + ez;
-        return fabs(den) > 1e-9 ? (nx + ny + nz) / den : 0.0;
+        const double num = nx + ny + nz;   // den >= 0: a zero keeps its sign, and needs no division (its slow path)
+        return fabs(den) > 1e-9 ? (is_zero(num) ? num : here(num) / den) : 0.0;
     }
     const double dx = sp.d[0], dy = sp.d[1], dz = sp.d[2];
     const double gxp = -(Txp - T0) / dx, gxm = -(T0 - Txm) / dx;
