@@ -46,7 +46,7 @@ __device__ __forceinline__ float ref_min(float x, float y) { return (x < y) ? x 
 // for spacings outside its range the expressions as they stand).
 // a: x-neighbour minimum (spacing dx), b: z-neighbour minimum (dz).
 __device__ __forceinline__ double eik2_plain(double a, double b, double s, const Sweep2Args& K) {
-    if (K.ex.quick) return eik2_exact(a, b, s, K.ex);
+    if (K.ex.quick) return K.ex.fast ? eik2_exact<true>(a, b, s, K.ex) : eik2_exact<false>(a, b, s, K.ex);
     double da = K.dx, db = K.dz, ia = K.inv2x, ib = K.inv2z, t;
     if (b > a) { t = a; a = b; b = t; t = da; da = db; db = t; t = ia; ia = ib; ib = t; }
     double q = b + db * s;

@@ -111,8 +111,12 @@ __host__ __device__ constexpr int warp_smem_bytes() {
 // spacings outside the range of its identities take the expressions as they stand.  The ordering
 // tests run on the bit patterns (same outcome for non-negative values).
 __device__ __forceinline__ double eik3_plain(double a, double b, double c, double s, const Spacing3& sp) {
-    if (sp.ex.quick)
-        return sp.ex.iso ? eik3_exact<true>(a, b, c, s, sp.ex, sp.inv2) : eik3_exact<false>(a, b, c, s, sp.ex, sp.inv2);
+    if (sp.ex.quick) {
+        if (sp.ex.iso)
+            return sp.ex.fast ? eik3_exact<true, true>(a, b, c, s, sp.ex, sp.inv2)
+                              : eik3_exact<true, false>(a, b, c, s, sp.ex, sp.inv2);
+        return eik3_exact<false, false>(a, b, c, s, sp.ex, sp.inv2);
+    }
     double da = sp.d[0], db = sp.d[1], dc = sp.d[2];
     double ia = sp.inv2[0], ib = sp.inv2[1], ic = sp.inv2[2];
     double t;

@@ -58,13 +58,31 @@ static void report(const char* name, long long n, long long wrong) {
 }
 
 int main() {
-    const double spacings[] = {20.0, 5.0, 12.5, 16.7, 8.3, 0.1, 1.0 / 3.0, 1.0, 4096.0, 1e-7, 7.3e11};
+    const double spacings[] = {20.0, 5.0, 12.5, 16.7, 8.3, 0.1, 1.0 / 3.0, 1.0, 4096.0, 3e-6, 7.3e5};
+    {   // square root: random values, squares and their neighbours, powers of two, edges of the range
+        long long n = 0, wrong = 0;
+        for (int i = 0; i < 3000000; ++i) {
+            g_seed_error = (float)uni(1.0 - 4e-7, 1.0 + 4e-7);
+            double x = any_bits(-110, 110);
+            if (i % 4 == 1) { const double m = any_bits(-40, 40); x = m * m; }
+            if (i % 4 == 2) x = std::ldexp(1.0, (int)(rng() % 180) - 90);
+            if (i % 4 == 3) {   // next to a midpoint of two neighbouring roots
+                const double m = any_bits(-40, 40), h = std::ldexp(1.0, std::ilogb(m) - 53);
+                x = std::fma(m, m, 2 * m * h);
+            }
+            if (i % 3 == 1) x = std::nextafter(x, 0.0);
+            if (i % 3 == 2) x = std::nextafter(x, 1e300);
+            wrong += !same(sqrt_exact(x), std::sqrt(x)), ++n;
+        }
+        for (double x : {0.0, 0x1p-1074, 0x1p-101, 0x1p100, 1e300, (double)INFINITY}) wrong += !same(sqrt_exact(x), std::sqrt(x)), ++n;
+        report("sqrt", n, wrong);
+    }
     {   // division by a constant: random values, and values next to multiples and midpoints
         long long n = 0, wrong = 0;
         for (double d : spacings) {
             const DivBy k = div_by(d);
             for (int i = 0; i < 400000; ++i) {
-                double x = any_bits(-120, 120);
+                double x = any_bits(-90, 89);
                 if (i % 3 == 1) {   // a quotient next to a 54-bit midpoint, times the divisor
                     const double m = any_bits(-30, 30), h = std::ldexp(1.0, std::ilogb(m) - 53);
                     x = std::fma(m, d, h * d);
@@ -72,12 +90,14 @@ int main() {
                 } else if (i % 3 == 2) {
                     x = any_bits(-3, 3) * d;
                 }
-                wrong += !same(div_exact(x, k), x / d) || !same(div_exact4(x, k.d, k.rh, k.rl), x / d) ||
-                         !same(div_any(-x, k), -x / d);
+                if (k.fast) wrong += !same(div_exact<true>(x, k), x / d);
+                wrong += !same(div_exact<false>(x, k), x / d) || !same(div_mid(-x, k), -x / d) || !same(div_any(-x, k), -x / d);
+                const double y = any_bits(-1060, 950);
+                wrong += !same(div_any(y, k), y / d) || !same(div_mid(-y, k), -y / d);
                 ++n;
             }
             for (double x : {0.0, -0.0, 0x1p-1074, -0x1p-1060, 0x1p-950, 1e300, -1e308, (double)INFINITY})
-                wrong += !same(div_any(x, k), x / d), ++n;
+                wrong += !same(div_any(x, k), x / d) || !same(div_mid(x, k), x / d), ++n;
         }
         report("div", n, wrong);
     }
@@ -106,9 +126,9 @@ int main() {
             double inv2[3];
             for (int a = 0; a < 3; ++a) inv2[a] = 1.0 / d[a] / d[a];
             const double r = eik3_ref(v[0], v[1], v[2], s, d);
-            const double e = g.iso && mode % 2 == 0 ? eik3_exact<true>(v[0], v[1], v[2], s, g, inv2)
-                                                    : eik3_exact<false>(v[0], v[1], v[2], s, g, inv2);
-            wrong += !same(r, e);
+            wrong += !same(r, eik3_exact<false, false>(v[0], v[1], v[2], s, g, inv2));
+            if (g.iso) wrong += !same(r, eik3_exact<true, false>(v[0], v[1], v[2], s, g, inv2));
+            if (g.iso && g.fast) wrong += !same(r, eik3_exact<true, true>(v[0], v[1], v[2], s, g, inv2));
             ++n;
         }
         char name[32];
@@ -129,7 +149,9 @@ int main() {
             if (c == 3) b = 0.0;
             if (c == 4) a = b = kUnreached;
             if (c == 5) { const double f = std::ldexp(1.0, (int)(rng() % 1200) - 600); a *= f; b *= f; s *= f; }
-            wrong += !same(eik2_ref(a, b, s, dx, dz), eik2_exact(a, b, s, exact_grid2(dx, dz)));
+            const ExactGrid2 g = exact_grid2(dx, dz);
+            const double r = eik2_ref(a, b, s, dx, dz);
+            wrong += !same(r, eik2_exact<false>(a, b, s, g)) || (g.fast && !same(r, eik2_exact<true>(a, b, s, g)));
             ++n;
         }
         report("eik2", n, wrong);

@@ -22,7 +22,7 @@ def test_exact_updates_match_the_expressions(tmp_path):
     subprocess.run([gxx, "-std=c++17", "-O2", "-ffp-contract=off", "-I", os.path.join(ROOT, "pfast_gb300", "csrc"),
                     os.path.join(HERE, "native", "exact_arith_check.cpp"), "-o", exe], check=True)
     out = subprocess.run([exe], capture_output=True, text=True, timeout=300)
-    assert out.returncode == 0 and "FAIL" not in out.stdout and out.stdout.count("ok ") == 9, out.stdout
+    assert out.returncode == 0 and "FAIL" not in out.stdout and out.stdout.count("ok ") == 10, out.stdout
 
 
 def _bits(a):
