@@ -58,6 +58,15 @@ PFAST_HD int dep_count(const TileGrid3& g, int o, int x) {
     return c;
 }
 
+// dep_count of all eight orders, 4 bits each: from order 1 on every neighbour counts, upstream in this
+// order or downstream in the one before.
+PFAST_HD unsigned dep_counts(const TileGrid3& g, int x) {
+    unsigned n = 0;
+    for (int a = 0; a < 3; ++a)
+        for (int s = 0; s < 2; ++s) n += tile_neighbour(g, x, a, s) >= 0;
+    return (unsigned)dep_count(g, 0, x) | (n + 1) * 0x11111110u;
+}
+
 // The items that wait for (o, x), at most 13: tile[k], order[k] for k < the returned count.
 //   (o+1, x)                                    for o < 7,
 //   (o, n)   for each neighbour n that x is upstream of in order o,

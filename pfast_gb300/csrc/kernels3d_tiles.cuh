@@ -132,34 +132,42 @@ __device__ __forceinline__ double eik3_plain(double a, double b, double c, doubl
 //   1 term:  x = dc*s
 //   2 terms: x = (wb*B + sqrt((wb+wc) s^2 - wb wc B^2)) / (wb+wc),         B = b-c
 //   3 terms: x = (wa*A + wb*B + sqrt(W s^2 - wa wb (A-B)^2 - wa wc A^2 - wb wc B^2)) / W,  A = a-c
+// Without branches, as the isotropic form below.  Candidates from unreached neighbours may be inf or
+// NaN; they are never selected.
 __device__ __forceinline__ float eik3_fast(float a, float b, float c, float s, const Spacing3& K) {
     float da = K.df[0], db = K.df[1], dc = K.df[2];
     float wa = K.wf[0], wb = K.wf[1], wc = K.wf[2];
     float ra = K.rpf[0], rb = K.rpf[1], rc = K.rpf[2];
-    float t;
-    if (b > a) { t = a; a = b; b = t; t = da; da = db; db = t; t = wa; wa = wb; wb = t; t = ra; ra = rb; rb = t; }
-    if (c > a) { t = a; a = c; c = t; t = da; da = dc; dc = t; t = wa; wa = wc; wc = t; t = ra; ra = rc; rc = t; }
-    if (c > b) { t = b; b = c; c = t; t = db; db = dc; dc = t; t = wb; wb = wc; wc = t; t = rb; rb = rc; rc = t; }
-    float q = fmaf(dc, s, c);
-    if (q <= b) return q;
+    auto order = [](float& x, float& y, float& dx, float& dy, float& wx, float& wy, float& rx, float& ry) {
+        const bool sw = y > x;
+        float t;
+        t = sw ? y : x; y = sw ? x : y; x = t;
+        t = sw ? dy : dx; dy = sw ? dx : dy; dx = t;
+        t = sw ? wy : wx; wy = sw ? wx : wy; wx = t;
+        t = sw ? ry : rx; ry = sw ? rx : ry; rx = t;
+    };
+    order(a, b, da, db, wa, wb, ra, rb);
+    order(a, c, da, dc, wa, wc, ra, rc);
+    order(b, c, db, dc, wb, wc, rb, rc);
+    const float q1 = fmaf(dc, s, c);
     const float s2 = s * s;
     const float B = b - c;
     const float wbB = wb * B;
     const float D = fmaf(wb + wc, s2, -wbB * wc * B);
-    q = (D >= 0.f) ? c + (wbB + sqrtf(D)) * ra : (float)kInf;
-    if (q <= a) return q;
+    const float q2 = (D >= 0.f) ? c + (wbB + sqrtf(D)) * ra : (float)kInf;
     const float A = a - c;
     const float AB = A - B;
     const float W = wa + wb + wc;
     const float D3 = W * s2 - (wa * wb * AB * AB + wa * wc * A * A + wb * wc * B * B);
-    return (D3 >= 0.f) ? c + (fmaf(wa, A, wbB) + sqrtf(D3)) * K.rWf : (float)kInf;
+    const float q3 = (D3 >= 0.f) ? c + (fmaf(wa, A, wbB) + sqrtf(D3)) * K.rWf : (float)kInf;
+    return q1 <= b ? q1 : (q2 <= a ? q2 : q3);
 }
 
-// Square root by the hardware approximation (PTX sqrt.approx.f32, a few ulps): the FP32 bulk
+// Square root by the hardware approximation (PTX sqrt.approx.ftz.f32, a few ulps): the FP32 bulk
 // result is only the starting point of the FP64 polish.
 __device__ __forceinline__ float sqrt_approx(float x) {
     float r;
-    asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
 
@@ -710,6 +718,7 @@ __device__ __forceinline__ void process_tile(const Sweep3Args& A, const int inst
     // instruction).  The plain kinds compare with a snapshot taken at the tile's first
     // processing in the iteration, as the reference's isconv does.
     constexpr bool kSnap = KIND == kFwdPlain64 || KIND == kAdjPlain64;
+    constexpr bool kBulk = KIND == kFwdFast32 || KIND == kAdjFast32;
     // The tile's lock word as lane 0 last wrote it.  Face neighbours are never processed at the
     // same time (per-diagonal: other launches; dataflow: the dependencies), so it is composed
     // here without reading it back.
@@ -759,6 +768,11 @@ __device__ __forceinline__ void process_tile(const Sweep3Args& A, const int inst
             const unsigned fb = A.mask[inst * A.mask_stride + ((long long)(k0 + lk) * nr + (i0 + li)) * A.wpr + (j0 >> 5)];
             fixed_bits = px ? fb : (__brev(fb) >> (32 - ej));
         }
+        // the grid's faces are not updated either
+        const int gk_ = k0 + lk, gi_ = i0 + li;
+        if (!(gk_ >= 1 && gk_ <= nz - 2 && gi_ >= 1 && gi_ <= nr - 2)) fixed_bits = 0xffffffffu;
+        if (j0 == 0) fixed_bits |= 1u << (px ? 0 : ej - 1);
+        if (j0 + ej == nc) fixed_bits |= 1u << (px ? ej - 1 : 0);
     }
 
     // ---- snapshot at the tile's first processing in this outer iteration (its values are
@@ -795,7 +809,6 @@ __device__ __forceinline__ void process_tile(const Sweep3Args& A, const int inst
         near_src = ddk * ddk + ddi * ddi + ddj * ddj <= A.src_r2;
         qkqi = (gk - sk) * (gk - sk) + (gi - si) * (gi - si);
     }
-    const bool row_interior = ADJ ? (gk >= 1 && gk <= nz - 2 && gi >= 1 && gi <= nr - 2) : true;
     unsigned sel = 0;   // polish: orders (flipped coordinates) in which some node of this lane's pencil is selected
     const long long rowbase = gk * plane + (long long)gi * nc;
     const Aux* srow = ADJ ? nullptr : reinterpret_cast<const Aux*>(A.aux) + rowbase;
@@ -876,6 +889,88 @@ __device__ __forceinline__ void process_tile(const Sweep3Args& A, const int inst
         uh0 = uload(uhrow, -hpos, 0, ej - 1); uhq1 = uload(uhrow, 1 - hpos, 0, ej - 1); uhq2 = uload(uhrow, 2 - hpos, 0, ej - 1);
     }
 
+    bool f_klo = false, f_khi = false, f_ilo = false, f_ihi = false, f_jlo = false, f_jhi = false;   // grid face marks
+    if constexpr (kBulk) {
+        // ---- FP32 bulk: every lane takes every step, the inactive ones on box entries of no
+        // consequence (all within the box), so that a step is straight-line code: 4 x 8 x 32 tiles
+        // took 169 (forward) and 208 (adjoint) warp instructions a step with the branches and
+        // the face tests of the other kinds.  What a step keeps is one bit per changed node;
+        // which faces that marks is found at the end, from the box.
+        const float* bp = box + cl;
+        const float* tp_ = aux + cl;        // adjoint
+        const float* sp_ = stile + sl;      // forward
+        unsigned chb = 0;                   // changed nodes of this lane's pencil, bit jf
+        const bool inK = lkf > 0, inI = lif > 0;
+#pragma unroll 1
+        for (int t = 0; t < steps; ++t) {
+            const int ljf = t - toff;
+            bool upd = (unsigned)ljf < (unsigned)ej;
+            const float xu = bp[t - 1], xd = bp[t + 1], yu = bp[t - HJ], yd = bp[t + HJ], zu = bp[t - PS], zd = bp[t + PS];
+            const float old = bp[t];
+            const bool inJ = ljf > 0;
+            float nv;
+            bool ch, feeds;   // feeds: some in-tile node that this pass visited before depends on this one
+            if constexpr (!ADJ) {
+                if (near_src) {   // the source node (and the opt-in fixed region) stays
+                    const int gj = gjA + dj * ljf;
+                    upd = upd & (qkqi + (gj - sj) * (gj - sj) > A.src_r2);
+                }
+                // field values are >= +0 or +inf: fminf is the reference's MIN here
+                const float xa = fminf(xd, xu), yb = fminf(yd, yu), zc = fminf(zd, zu), s = sp_[t];
+                nv = fminf(old, A.sp.iso ? eik3_fast_iso(xa, yb, zc, s * A.sp.df[0]) : eik3_fast(xa, yb, zc, s, A.sp));
+                ch = upd & (nv < old);
+                feeds = nv < fmaxf(fmaxf(inK ? zu : 0.0f, inI ? yu : 0.0f), inJ ? xu : 0.0f);
+            } else {
+                const float T0 = tp_[t], Txu = tp_[t - 1], Txd = tp_[t + 1], Tyu = tp_[t - HJ], Tyd = tp_[t + HJ];
+                const float Tzu = tp_[t - PS], Tzd = tp_[t + PS];
+                upd = upd & !((fixed_bits >> (ljf & 31)) & 1u);
+                // the update is symmetric in the two neighbours of an axis
+                nv = adj3_bulk(T0, Txd, Txu, Tyd, Tyu, Tzd, Tzu, xd, xu, yd, yu, zd, zu, old, A.sp);
+                ch = upd & (__float_as_uint(nv) != __float_as_uint(old));
+                feeds = T0 > fminf(fminf(inK ? Tzu : INFINITY, inI ? Tyu : INFINITY), inJ ? Txu : INFINITY);
+            }
+            if (ch) box[cl + t] = nv;
+            chb |= ch ? 1u << (ljf & 31) : 0u;
+            stale |= ch & feeds;
+            moved |= ch & (fabsf(old - nv) > A.tol_abs_f + A.tol_rel_f * fabsf(nv));
+            __syncwarp();
+        }
+        chg = chb != 0;
+        const unsigned who = __ballot_sync(0xffffffffu, chg);
+        if (!who) return;
+        // ---- a changed face node marks the neighbour whose node across the face depends on it
+        // (depends_on): box values and traveltimes of the node and of the halo entry beyond it
+        auto dep = [&](int c, int n) -> bool {
+            if constexpr (ADJ) return aux[c] > aux[n];
+            else return box[c] < box[n];
+        };
+        auto face = [&](int pencil, int step) -> bool {   // the pencil's nodes, lane = column
+            const unsigned m = __shfl_sync(0xffffffffu, chb, pencil);
+            const int c = (pencil / TI + 1) * PS + (pencil % TI + 1) * HJ + 1 + lane;
+            return ((m >> lane) & 1u) && dep(c, c + step);
+        };
+        bool zlo = false, zhi = false, ylo = false, yhi = false;   // flipped: upstream / downstream
+        constexpr unsigned kRow0 = TI == 8 ? 0x01010101u : 0x11111111u;   // pencils with if = 0
+        if (who & ((1u << TI) - 1))
+#pragma unroll
+            for (int i = 0; i < TI; ++i) zlo |= face(i, -PS);
+        if ((who >> ((ek - 1) * TI)) & ((1u << TI) - 1))
+#pragma unroll
+            for (int i = 0; i < TI; ++i) zhi |= face((ek - 1) * TI + i, PS);
+        if (who & kRow0)
+#pragma unroll
+            for (int k = 0; k < TK; ++k) ylo |= face(k * TI, -HJ);
+        if ((who >> (ei - 1)) & kRow0)
+#pragma unroll
+            for (int k = 0; k < TK; ++k) yhi |= face(k * TI + ei - 1, HJ);
+        const int c0 = (lkf + 1) * PS + (lif + 1) * HJ + 1;   // lane = pencil
+        const bool xlo = (chb & 1u) && dep(c0, c0 - 1), xhi = ((chb >> (ej - 1)) & 1u) && dep(c0 + ej - 1, c0 + ej);
+        const unsigned faces = __reduce_or_sync(0xffffffffu, (zlo ? 1u : 0u) | (zhi ? 2u : 0u) | (ylo ? 4u : 0u) | (yhi ? 8u : 0u) |
+                                                                 (xlo ? 16u : 0u) | (xhi ? 32u : 0u));
+        f_klo = faces & (pz ? 1u : 2u); f_khi = faces & (pz ? 2u : 1u);
+        f_ilo = faces & (py ? 4u : 8u); f_ihi = faces & (py ? 8u : 4u);
+        f_jlo = faces & (px ? 16u : 32u); f_jhi = faces & (px ? 32u : 16u);
+    } else {
 #pragma unroll 1
     for (int t = 0; t < steps; ++t) {
         const int ljf = t - toff;
@@ -919,7 +1014,7 @@ __device__ __forceinline__ void process_tile(const Sweep3Args& A, const int inst
             const Real old = UWIN ? u0 : box[c];
             Real nv = old;
             float dstep = INFINITY;   // polish: the size of this node's change
-            if constexpr (ADJ && !TWIN) {   // FP32 bulk: the traveltimes from the staged box
+            if constexpr (ADJ && !TWIN) {   // the traveltimes from the staged box
                 t0 = aux[c]; Txu = aux[c - 1]; Txd = aux[c + 1]; Tyu = aux[c - HJ]; Tyd = aux[c + HJ];
                 Tzu = aux[c - PS]; Tzd = aux[c + PS];
             }
@@ -928,16 +1023,10 @@ __device__ __forceinline__ void process_tile(const Sweep3Args& A, const int inst
                 bool free_node = true;   // the source node (and the opt-in fixed region) stays
                 if (near_src) free_node = qkqi + (gj - sj) * (gj - sj) > A.src_r2;
                 if (free_node) {
-                    Aux s;
-                    if constexpr (stage_slowness<KIND>()) s = stile[sl + t];
-                    else s = __ldg(srow + gj);
+                    const Aux s = __ldg(srow + gj);
                     // the neighbour minima are symmetric in the two neighbours of an axis
                     if constexpr (KIND == kFwdPlain64) {
                         nv = min_nonneg(old, eik3_plain(min_nonneg(xd, xu), min_nonneg(yd, yu), min_nonneg(zd, zu), s, A.sp));
-                    } else if constexpr (KIND == kFwdFast32) {
-                        // field values are >= +0 or +inf: fminf is the reference's MIN here
-                        const float xa = fminf(xd, xu), yb = fminf(yd, yu), zc = fminf(zd, zu);
-                        nv = fminf(old, A.sp.iso ? eik3_fast_iso(xa, yb, zc, s * A.sp.df[0]) : eik3_fast(xa, yb, zc, s, A.sp));
                     } else {   // polish: one Newton step of the local Godunov equation (aux holds s^2, (s h)^2 when isotropic)
                         // Octant selection: if an axis is active (U0 above its smaller neighbour) and
                         // that neighbour is the one this sweep visits after the node, the update would
@@ -959,8 +1048,7 @@ __device__ __forceinline__ void process_tile(const Sweep3Args& A, const int inst
                     }
                 }
             } else {
-                const int gj = gjA + dj * ljf;
-                if (row_interior && gj >= 1 && gj <= nc - 2 && !((fixed_bits >> ljf) & 1u)) {
+                if (!((fixed_bits >> ljf) & 1u)) {
                     if constexpr (KIND == kAdjPlain64) {
                         // the reference's operand order, in grid orientation (m: index - 1, p: index + 1)
                         const Real Lxp = px ? xd : xu, Lxm = px ? xu : xd, Lyp = py ? yd : yu, Lym = py ? yu : yd;
@@ -968,9 +1056,6 @@ __device__ __forceinline__ void process_tile(const Sweep3Args& A, const int inst
                         const Aux Txp = px ? Txd : Txu, Txm = px ? Txu : Txd, Typ = py ? Tyd : Tyu, Tym = py ? Tyu : Tyd;
                         const Aux Tzp = pz ? Tzd : Tzu, Tzm = pz ? Tzu : Tzd;
                         nv = adj3_plain(t0, Txp, Txm, Typ, Tym, Tzp, Tzm, Lxp, Lxm, Lyp, Lym, Lzp, Lzm, A.sp);
-                    } else if constexpr (KIND == kAdjFast32) {
-                        // the update is symmetric in the two neighbours of an axis
-                        nv = adj3_bulk(t0, Txd, Txu, Tyd, Tyu, Tzd, Tzu, xd, xu, yd, yu, zd, zu, old, A.sp);
                     } else {
                         // Octant selection (see the forward polish): lambda at a node depends on the
                         // neighbours with a larger traveltime.  Where on some axis only the neighbour
@@ -1004,8 +1089,6 @@ __device__ __forceinline__ void process_tile(const Sweep3Args& A, const int inst
                 chg = true;
                 if constexpr (kSelective) {
                     if (dstep > tol_step) moved = true;
-                } else if constexpr (!kSnap) {
-                    if (fabsf(old - nv) > A.tol_abs_f + A.tol_rel_f * fabsf(nv)) moved = true;
                 }
                 // does the neighbour across a face (value vn, traveltime tn) depend on this node?
                 // The neighbour values were read before this step's stores, none of which
@@ -1047,12 +1130,13 @@ __device__ __forceinline__ void process_tile(const Sweep3Args& A, const int inst
 
     // ---- unlock this tile and every face neighbour that sees a changed face node (flipped
     // faces mapped back to grid faces)
-    const unsigned f_klo = __ballot_sync(0xffffffffu, pz ? m_zu : m_zd);
-    const unsigned f_khi = __ballot_sync(0xffffffffu, pz ? m_zd : m_zu);
-    const unsigned f_ilo = __ballot_sync(0xffffffffu, py ? m_yu : m_yd);
-    const unsigned f_ihi = __ballot_sync(0xffffffffu, py ? m_yd : m_yu);
-    const unsigned f_jlo = __ballot_sync(0xffffffffu, px ? m_xu : m_xd);
-    const unsigned f_jhi = __ballot_sync(0xffffffffu, px ? m_xd : m_xu);
+    f_klo = __any_sync(0xffffffffu, pz ? m_zu : m_zd);
+    f_khi = __any_sync(0xffffffffu, pz ? m_zd : m_zu);
+    f_ilo = __any_sync(0xffffffffu, py ? m_yu : m_yd);
+    f_ihi = __any_sync(0xffffffffu, py ? m_yd : m_yu);
+    f_jlo = __any_sync(0xffffffffu, px ? m_xu : m_xd);
+    f_jhi = __any_sync(0xffffffffu, px ? m_xd : m_xu);
+    }
     // Own re-marking.  A polish sweep in order o leaves every node that selects o consistent
     // with the values it reads (its active neighbours come before it in o), so after small
     // updates the tile is due again in o only when a neighbour or another order changes
@@ -1157,7 +1241,8 @@ __global__ void __launch_bounds__(kWarps3 * 32) sweep3d_kernel(const Sweep3Args 
 //   lock words.  A tile that is not due in the item's order (tile locking) completes at once,
 //   lane by lane; of the due items the warp processes one (process_tile) and returns the
 //   others to the ring for idle warps.  Completing (o, x) re-arms x's counter of parity o for
-//   order o + 2 and decrements its dependents' counters; those that reach zero join the ring.
+//   order o + 2 (clusters keep all eight orders' counters instead) and decrements its dependents'
+//   counters; those that reach zero join the ring.
 //   The iteration ends when all 8 x ntiles items completed; the block then tests convergence
 //   as the per-diagonal schedule's reduction does (any tile moved / any tile still due).
 // Every tile processing sees exactly the neighbour values and lock words it sees in the
@@ -1222,11 +1307,14 @@ __device__ __forceinline__ int df_dependent(const TileGrid3& g, int o, int x, in
     return o < 7 && !side_upstream(o + 1, a, 1 - s) ? (y << 3) | (o + 1) : -1;
 }
 
-// Item e has one missing dependency fewer; returns its count before.
+// Item e has one missing dependency fewer; returns its count before.  A block keeps two 4-bit
+// counters per tile, four tiles per word; a cluster, whose completions would wait for the re-arming
+// of one, all eight orders' counters, one word per tile.
+template <bool CL>
 __device__ __forceinline__ unsigned df_notify(const DataflowQueue& Q, int e) {
     const int y = e >> 3;
-    const unsigned shf = 8u * (unsigned)(y & 3) + 4u * (unsigned)(e & 1);
-    return (atomicSub(Q.cnt + (y >> 2), 1u << shf) >> shf) & 15u;
+    const unsigned shf = CL ? 4u * (unsigned)(e & 7) : 8u * (unsigned)(y & 3) + 4u * (unsigned)(e & 1);
+    return (atomicSub(Q.cnt + (CL ? y : y >> 2), 1u << shf) >> shf) & 15u;
 }
 
 // Re-arm x's counter of parity o for order o + 2 (it is zero: it fired for (o, x), and no
@@ -1241,14 +1329,16 @@ __device__ __forceinline__ void df_rearm(const TileGrid3& g, const DataflowQueue
 // go on with; the others join the ring.
 template <bool CL>
 __device__ __forceinline__ unsigned df_complete(const TileGrid3& g, const DataflowQueue& Q, int o, int x) {
-    df_rearm(g, Q, o, x);
-    df_fence<CL>();
+    if constexpr (!CL) {
+        df_rearm(g, Q, o, x);
+        df_fence<CL>();
+    }
     int dep[13];
     unsigned old[13];
 #pragma unroll
     for (int k = 0; k < 13; ++k) {
         dep[k] = df_dependent(g, o, x, k);
-        old[k] = dep[k] >= 0 ? df_notify(Q, dep[k]) : 2u;
+        old[k] = dep[k] >= 0 ? df_notify<CL>(Q, dep[k]) : 2u;
     }
     unsigned keep = kSlotEmpty;
 #pragma unroll
@@ -1267,16 +1357,15 @@ __device__ __forceinline__ unsigned df_complete(const TileGrid3& g, const Datafl
 // became ready.
 template <bool CL>
 __device__ __forceinline__ unsigned df_complete_warp(const TileGrid3& g, const DataflowQueue& Q, int o, int x, int lane) {
-    if (lane == 0) {
-        df_rearm(g, Q, o, x);
-        df_fence<CL>();
+    if constexpr (!CL) {
+        if (lane == 0) df_rearm(g, Q, o, x);
     }
     __syncwarp();
     unsigned keep = kSlotEmpty;
     const int dep = lane < 13 ? df_dependent(g, o, x, lane) : -1;
     if (dep >= 0) {
-        df_fence<CL>();   // the warp's tile (seen by this lane through the warp barrier) first
-        const unsigned old = df_notify(Q, dep);
+        df_fence<CL>();   // what the warp wrote (seen by this lane through the warp barrier) first
+        const unsigned old = df_notify<CL>(Q, dep);
         if (old == 1u) keep = (unsigned)dep;
         else if (old == 0u) *(volatile int*)&Q.sh->abort = 1;
     }
@@ -1368,8 +1457,6 @@ __device__ __forceinline__ void df_iteration(const Sweep3Args& A, const int inst
             const int edm = __shfl_sync(0xffffffffu, dm, mine);
             const int tj = ex % g.nbj, ti = (ex / g.nbj) % g.nbi, tk = ex / (g.nbj * g.nbi);
             process_tile<KIND, true, FORM, SH>(A, inst, ex, tk, ti, tj, eo, iter, edm, wsm, lane);
-            df_fence<CL>();   // the tile's field and lock words before its dependents start
-            __syncwarp();
             next = df_complete_warp<CL>(g, Q, eo, ex, lane);
             if (lane == 0) ++ncomp;
         }
@@ -1388,10 +1475,12 @@ __device__ __forceinline__ void df_iteration(const Sweep3Args& A, const int inst
 // thread follows the block size.  The register-window kinds use no box: 24 warps for the
 // forward polish (85 registers a thread; 20 warps measured 2 % slower), 16 for the adjoint
 // polish, which also keeps the traveltime windows (128 registers; 20 warps measured 3 % slower).
-template <int KIND, int FORM, class SH>
+// Clusters hold at most 12.
+template <int KIND, int FORM, bool CL, class SH>
 __host__ __device__ constexpr int df_max_warps() {
     constexpr int fit = (227 * 1024 - 256 - 40960) / warp_smem_bytes<KIND, SH, FORM>();
-    return u_windows<KIND, FORM>() ? (KIND == kAdjPolish64 ? 16 : 24) : (fit < 24 ? fit : 24);
+    constexpr int most = u_windows<KIND, FORM>() ? (KIND == kAdjPolish64 ? 16 : 24) : (fit < 24 ? fit : 24);
+    return CL && most > 12 ? 12 : most;
 }
 
 // MULTI: instances of several grids in one launch.  Item q of the queue is models[items[q].x]'s
@@ -1403,7 +1492,7 @@ __host__ __device__ constexpr int df_max_warps() {
 // sources than SMs uses the SMs it would leave idle; the blocks of a cluster run at the same time
 // by construction, so their waits on one another end.
 template <int KIND, bool MULTI, bool CL, int FORM, class SH>
-__global__ void __launch_bounds__(df_max_warps<KIND, FORM, SH>() * 32, 1) sweep3d_dataflow(const Sweep3Args A0,
+__global__ void __launch_bounds__(df_max_warps<KIND, FORM, CL, SH>() * 32, 1) sweep3d_dataflow(const Sweep3Args A0,
                                                                       const Sweep3Args* __restrict__ models,
                                                                       const int2* __restrict__ items, const int nact,
                                                                       const int maxiter, int* __restrict__ queue,
@@ -1456,7 +1545,7 @@ __global__ void __launch_bounds__(df_max_warps<KIND, FORM, SH>() * 32, 1) sweep3
             inst = A0.act[item];
         }
         const Sweep3Args& A = MULTI ? s_args : A0;
-        const int ntiles = A.ntiles, ncw = (ntiles + 3) >> 2;
+        const int ntiles = A.ntiles, ncw = CL ? ntiles : (ntiles + 3) >> 2;
         Q.slots = Q.cnt + ncw;
         const TileGrid3 g{A.nbk, A.nbi, A.nbj};
         int* diff = A.diff + (long long)inst * ntiles;
@@ -1464,9 +1553,10 @@ __global__ void __launch_bounds__(df_max_warps<KIND, FORM, SH>() * 32, 1) sweep3
         int it = A.iter;   // the first outer iteration (a continuation starts past 0); maxiter is absolute
         bool moved = true, aborted = false;
         while (it < maxiter) {
-            // counters of orders 0 and 1, an empty ring, cleared per-tile change flags
-            if (rank == 0) {
-                unsigned* slots = cnt + ncw;
+            // counters (a block: of orders 0 and 1), an empty ring, cleared per-tile change flags
+            if constexpr (CL) {
+                for (int x = cthr; x < ntiles; x += cnthr) Q.cnt[x] = dep_counts(g, x);
+            } else {
                 for (int w = threadIdx.x; w < ncw; w += nthr) {
                     unsigned v = 0;
                     for (int b = 0; b < 4; ++b) {
@@ -1475,15 +1565,15 @@ __global__ void __launch_bounds__(df_max_warps<KIND, FORM, SH>() * 32, 1) sweep3
                     }
                     cnt[w] = v;
                 }
-                // the ring starts with (order 0, first tile)
-                for (int q = threadIdx.x; q < qcap; q += nthr) slots[q] = q ? kSlotEmpty : (unsigned)first_tile(g) << 3;
-                if (threadIdx.x == 0) {
-                    sh.head = 0;
-                    sh.tail = 1;
-                    sh.done = 0;
-                    sh.abort = 0;
-                    sh.flags[it & 1] = 0;
-                }
+            }
+            // the ring starts with (order 0, first tile)
+            for (int q = cthr; q < qcap; q += cnthr) Q.slots[q] = q ? kSlotEmpty : (unsigned)first_tile(g) << 3;
+            if (cthr == 0) {
+                sh.head = 0;
+                sh.tail = 1;
+                sh.done = 0;
+                sh.abort = 0;
+                sh.flags[it & 1] = 0;
             }
             for (int t = cthr; t < ntiles; t += cnthr) diff[t] = 0;
             sync();
@@ -1635,8 +1725,8 @@ inline int dataflow_qcap(int ntiles) {
     return q;
 }
 
-inline size_t dataflow_extra_bytes(int ntiles, bool multi) {
-    return (size_t)4 * ((ntiles + 3) / 4) + (size_t)4 * dataflow_qcap(ntiles) + (multi ? kDfArgsBytes : 0);
+inline size_t dataflow_extra_bytes(int ntiles, bool multi, bool cluster) {
+    return (size_t)4 * (cluster ? ntiles : (ntiles + 3) / 4) + (size_t)4 * dataflow_qcap(ntiles) + (multi ? kDfArgsBytes : 0);
 }
 
 template <int KIND, class SH>
@@ -1683,16 +1773,16 @@ template <int KIND, class SH>
 DataflowKernel dataflow_kernel(bool multi, bool cluster, int form) {
     if constexpr (KIND == kAdjPolish64) {
         if (form == kFormBoxes)
-            return {dataflow_fn_of<KIND, kFormBoxes, SH>(multi, cluster), df_max_warps<KIND, kFormBoxes, SH>(),
+            return {dataflow_fn_of<KIND, kFormBoxes, SH>(multi, cluster), cluster ? df_max_warps<KIND, kFormBoxes, true, SH>() : df_max_warps<KIND, kFormBoxes, false, SH>(),
                     warp_smem_bytes<KIND, SH, kFormBoxes>()};
     }
     if constexpr (KIND == kFwdPolish64 || KIND == kAdjPolish64) {
         if (KIND == kAdjPolish64 || form == kFormWindows)
-            return {dataflow_fn_of<KIND, kFormWindows, SH>(multi, cluster), df_max_warps<KIND, kFormWindows, SH>(),
+            return {dataflow_fn_of<KIND, kFormWindows, SH>(multi, cluster), cluster ? df_max_warps<KIND, kFormWindows, true, SH>() : df_max_warps<KIND, kFormWindows, false, SH>(),
                     warp_smem_bytes<KIND, SH, kFormWindows>()};
     }
     if constexpr (KIND != kAdjPolish64)
-        return {dataflow_fn_of<KIND, kFormBox, SH>(multi, cluster), df_max_warps<KIND, kFormBox, SH>(),
+        return {dataflow_fn_of<KIND, kFormBox, SH>(multi, cluster), cluster ? df_max_warps<KIND, kFormBox, true, SH>() : df_max_warps<KIND, kFormBox, false, SH>(),
                 warp_smem_bytes<KIND, SH, kFormBox>()};
     return {};
 }
@@ -1713,7 +1803,6 @@ pfast_status dataflow_shape_k(int ntiles, int nact, bool multi, DataflowShape* o
     }
     PFAST_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     PFAST_CUDA_TRY(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    const long long room = (long long)smem_max - 256 - (long long)dataflow_extra_bytes(ntiles, multi);
     constexpr bool kPlain = KIND == kFwdPlain64 || KIND == kAdjPlain64;
     *out = DataflowShape();
     // the largest cluster size at which every instance has a cluster of its own at the same time
@@ -1721,8 +1810,13 @@ pfast_status dataflow_shape_k(int ntiles, int nact, bool multi, DataflowShape* o
         if (cs > 1 && !cluster_wanted(cs, kPlain, nact, ntiles, sms)) continue;
         const int form = dataflow_form<KIND>(cs, ntiles);
         const DataflowKernel k = dataflow_kernel<KIND, SH>(multi, cs > 1, form);
-        const int wmax = (int)std::min<long long>(k.max_warps, room / k.warp_bytes);
-        if (ntiles > kDataflowMaxTiles || wmax < 1) return PFAST_OK;
+        if (ntiles > kDataflowMaxTiles) return PFAST_OK;
+        const long long extra = (long long)dataflow_extra_bytes(ntiles, multi, cs > 1);
+        const int wmax = (int)std::min<long long>(k.max_warps, ((long long)smem_max - 256 - extra) / k.warp_bytes);
+        if (wmax < 1) {
+            if (cs > 1) continue;
+            return PFAST_OK;
+        }
         // the opt-in maximum (less the kernel's static shared memory), not this grid's size: a cached
         // shape of a larger grid launches later with more than a smaller grid's call would allow
         cudaFuncAttributes fa;
@@ -1730,7 +1824,7 @@ pfast_status dataflow_shape_k(int ntiles, int nact, bool multi, DataflowShape* o
         PFAST_CUDA_TRY(cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             smem_max - (int)fa.sharedSizeBytes));
         const int w = cs > 1 ? std::min(wmax, cluster_warps(cs, kPlain)) : wmax;
-        const size_t smem = (size_t)w * k.warp_bytes + dataflow_extra_bytes(ntiles, multi);
+        const size_t smem = (size_t)(w * (long long)k.warp_bytes + extra);
         int resident = 0;
         if (cs > 1) {
             PFAST_CUDA_TRY(cudaFuncSetAttribute(k.fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));

@@ -78,7 +78,7 @@ inline bool cluster_wanted(int cs, bool plain, int nact, int ntiles, int sms) {
 // 41.3 (6); 64 sources of 128 x 128 x 64, mixed gradient, 2 blocks: 97 (8), 83 (12), 81 (24).
 inline int cluster_warps(int cs, bool plain) {
     if (plain || cs >= 8) return 4;
-    return cs >= 4 ? 6 : 24;
+    return cs >= 4 ? 6 : 12;
 }
 
 // The candidate of a phase that has not been timed, among `allowed` (tune_allowed): the dataflow
