@@ -423,95 +423,122 @@ __device__ __forceinline__ void load_box(T* box, const T* __restrict__ g, int k0
 }
 
 // Vector form of load_box, for grids whose rows start on 16-byte boundaries (ncols a multiple of
-// V = 16 / sizeof(T) and a 16-byte aligned field): box rows are read as aligned V-element vectors
-// from grid column j0 - V on, so the halo columns j0 - 1 and j0 + ej come with their vectors
-// (a vector lies wholly inside or outside the grid).  The first MV = TJ / V vectors of each row
-// (columns j0 - V .. j0 + TJ - V - 1) are read by 32 / MV rows of lanes at a time; the last two
-// (columns j0 + TJ - V .. j0 + TJ + V - 1) by 16 rows of lane pairs.  A lane's columns, and so its
-// flipped box positions, are fixed for the whole load.
+// V = 16 / sizeof(T) and a 16-byte aligned field; a tile's columns are then whole vectors).  The
+// tile's columns are read as MV = TJ / V aligned vectors per row, 32 / MV rows of lanes at a time: two
+// rows of one plane (FP64) or of two (FP32), so that a lane's row and plane parity, its columns and its
+// flipped positions are fixed for the whole load; the two halo columns one element per lane.  With
+// halo columns inside misaligned vectors and the rows decoded per pass, what a tile cost beside its
+// wavefront was 2500 instructions (FP32 forward), 42 % of the total.
 template <typename T, bool COHERENT, class SH>
 __device__ __forceinline__ void load_box_vec(T* box, const T* __restrict__ g, int k0, int i0, int j0, int ek, int ei,
                                              int ej, bool pz, bool py, bool px, int nz, int nr, int nc, T fill,
                                              int lane) {
     PFAST_TILE_SHAPE(SH);
     using VT = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
-    constexpr int V = 16 / sizeof(T);
-    constexpr int MV = TJ / V;          // main vectors per row: 8 (FP32) or 16 (FP64)
-    constexpr int RPI = 32 / MV;        // rows per main pass: 4 or 2
-    constexpr int NROW = HK * HI;
+    constexpr int V = 16 / sizeof(T), MV = TJ / V;
+    constexpr int RY = 2, RZ = 32 / MV / RY;        // rows x planes of a pass: 2 x 2 (FP32) or 2 x 1
+    constexpr int NY = HI / RY, ZB = RZ == 2 ? 1 : 2;   // passes per plane step; plane steps per batch
+    static_assert(HI % RY == 0 && HK % (RZ * ZB) == 0, "whole batches");
     const long long plane = (long long)nr * nc;
+    // flipped position of box plane z / row y: origin + z*sz + y*sy
+    const int sz = pz ? PS : -PS, sy = py ? HJ : -HJ;
+    const int origin = (pz ? 0 : (ek + 1) * PS) + (py ? 0 : (ei + 1) * HJ);
+    {
+        const int q = lane % MV, dy = (lane / MV) % RY, dz = lane / MV / RY;
+        unsigned rows = 0, have = 0;                // bit u: row 2u + dy is in the box / in the grid
 #pragma unroll
-    for (int part = 0; part < 2; ++part) {
-        const int q = part == 0 ? lane % MV : MV + (lane & 1);   // the lane's vector in the row
-        const int rsub = part == 0 ? lane / MV : lane >> 1;      // its row within a pass
-        const int rstep = part == 0 ? RPI : 16;
-        const int gx = j0 - V + q * V;                           // grid column of the vector's first element
-        const bool vin = gx >= 0 && gx < nc;
-        int xf[V];
-        bool xs[V];
-#pragma unroll
-        for (int e = 0; e < V; ++e) {
-            const int bx = gx + e - (j0 - 1);                    // halo-box column
-            xs[e] = bx >= 0 && bx <= ej + 1;
-            xf[e] = px ? bx : ej + 1 - bx;
+        for (int u = 0; u < NY; ++u) {
+            const int y = u * RY + dy;
+            if (q * V < ej && y <= ei + 1) {
+                rows |= 1u << u;
+                if ((unsigned)(i0 - 1 + y) < (unsigned)nr) have |= 1u << u;
+            }
         }
-        constexpr int BATCH = 8;
+        const T* src = g + (k0 - 1 + dz) * plane + (long long)(i0 - 1 + dy) * nc + j0 + q * V;
+        const int bx = px ? 1 + q * V : ej - q * V, dx = px ? 1 : -1;
+        T* dst = box + origin + dz * sz + dy * sy + bx;
 #pragma unroll 1
-        for (int r0 = 0; r0 < NROW; r0 += BATCH * rstep) {
-            VT v[BATCH];
+        for (int z = 0; z < HK; z += RZ * ZB) {
+            VT v[ZB * NY];
 #pragma unroll
-            for (int u = 0; u < BATCH; ++u) {
-                const int r = r0 + u * rstep + rsub, z = r / HI, y = r - z * HI;
-                const int gk = k0 - 1 + z, gi = i0 - 1 + y;
-                const bool ok = vin && r < NROW && z <= ek + 1 && y <= ei + 1 && (unsigned)gk < (unsigned)nz &&
-                                (unsigned)gi < (unsigned)nr;
-                const VT* src = reinterpret_cast<const VT*>(g + gk * plane + (long long)gi * nc + gx);
-                if (ok) v[u] = COHERENT ? __ldcg(src) : __ldg(src);
-                else {
-                    T* f = reinterpret_cast<T*>(&v[u]);
+            for (int w = 0; w < ZB; ++w) {
+                const int zz = z + w * RZ + dz;
+                const bool zin = zz <= ek + 1 && (unsigned)(k0 - 1 + zz) < (unsigned)nz;
+#pragma unroll
+                for (int u = 0; u < NY; ++u) {
+                    T* f = reinterpret_cast<T*>(&v[w * NY + u]);
 #pragma unroll
                     for (int e = 0; e < V; ++e) f[e] = fill;
+                    const VT* at = reinterpret_cast<const VT*>(src + w * RZ * plane + u * RY * nc);
+                    if (zin && (have >> u & 1u)) v[w * NY + u] = COHERENT ? __ldcg(at) : __ldg(at);
                 }
             }
 #pragma unroll
-            for (int u = 0; u < BATCH; ++u) {
-                const int r = r0 + u * rstep + rsub, z = r / HI, y = r - z * HI;
-                if (r >= NROW || z > ek + 1 || y > ei + 1) continue;
-                T* brow = box + (pz ? z : ek + 1 - z) * PS + (py ? y : ei + 1 - y) * HJ;
-                const T* f = reinterpret_cast<const T*>(&v[u]);
+            for (int w = 0; w < ZB; ++w)
 #pragma unroll
-                for (int e = 0; e < V; ++e)
-                    if (xs[e]) brow[xf[e]] = f[e];
-            }
+                for (int u = 0; u < NY; ++u)
+                    if (z + w * RZ + dz <= ek + 1 && (rows >> u & 1u)) {
+                        const T* f = reinterpret_cast<const T*>(&v[w * NY + u]);
+                        T* at = dst + w * RZ * sz + u * RY * sy;
+#pragma unroll
+                        for (int e = 0; e < V; ++e) at[e * dx] = f[e];
+                    }
+            src += RZ * ZB * plane;
+            dst += RZ * ZB * sz;
+        }
+    }
+    {   // the halo columns j0 - 1 and j0 + ej: lane = (row, side)
+        constexpr int NROW = HK * HI, NP = (NROW + 15) / 16;
+        const int side = lane & 1, gj = side ? j0 + ej : j0 - 1, bx = (side != 0) == px ? ej + 1 : 0;
+        const bool vin = (unsigned)gj < (unsigned)nc;
+        T v[NP];
+#pragma unroll
+        for (int u = 0; u < NP; ++u) {
+            const int r = u * 16 + (lane >> 1), z = r / HI, y = r - z * HI;
+            const bool ok = vin && z <= ek + 1 && y <= ei + 1 && (unsigned)(k0 - 1 + z) < (unsigned)nz &&
+                            (unsigned)(i0 - 1 + y) < (unsigned)nr;
+            v[u] = fill;
+            const T* at = g + (k0 - 1 + z) * plane + (long long)(i0 - 1 + y) * nc + gj;
+            if (ok) v[u] = COHERENT ? __ldcg(at) : __ldg(at);
+        }
+#pragma unroll
+        for (int u = 0; u < NP; ++u) {
+            const int r = u * 16 + (lane >> 1), z = r / HI, y = r - z * HI;
+            if (z <= ek + 1 && y <= ei + 1) box[origin + z * sz + y * sy + bx] = v[u];
         }
     }
 }
 
-// Vector write-back of the tile's interior (same alignment condition; ej is then a multiple of
-// V): lane (row of a pass, vector) gathers V flipped box entries and stores them at once.
+// Vector write-back of the tile's interior (same alignment condition): lane (row of a pass,
+// vector) gathers V flipped box entries and stores them at once.
 template <typename T, class SH>
 __device__ __forceinline__ void store_tile_vec(T* __restrict__ fld, const T* box, int k0, int i0, int j0, int ek,
                                                int ei, int ej, bool pz, bool py, bool px, int nr, int nc, int lane) {
     PFAST_TILE_SHAPE(SH);
     using VT = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
-    constexpr int V = 16 / sizeof(T);
-    constexpr int MV = TJ / V, RPI = 32 / MV;
+    constexpr int V = 16 / sizeof(T), MV = TJ / V, RPI = 32 / MV;
+    constexpr int NY = TI / RPI;   // passes per plane
+    static_assert(TI % RPI == 0, "a pass stays in its plane");
     const long long plane = (long long)nr * nc;
     const int q = lane % MV, rsub = lane / MV;
-    const bool qok = q * V < ej;
-#pragma unroll 4
-    for (int r0 = 0; r0 < TK * TI; r0 += RPI) {
-        const int r = r0 + rsub, rk = r / TI, ri = r - rk * TI;
-        if (!qok || rk >= ek || ri >= ei) continue;
-        const int base = ((pz ? rk : ek - 1 - rk) + 1) * PS + ((py ? ri : ei - 1 - ri) + 1) * HJ + 1;
-        VT v;
-        T* f = reinterpret_cast<T*>(&v);
+    const int sz = pz ? PS : -PS, sy = py ? HJ : -HJ, dx = px ? 1 : -1;
+    const T* src = box + (pz ? PS : ek * PS) + (py ? HJ : ei * HJ) + rsub * sy + (px ? 1 + q * V : ej - q * V);
+    T* dst = fld + k0 * plane + (long long)(i0 + rsub) * nc + j0 + q * V;
+    const int ny = q * V < ej ? ei - rsub : 0;   // this lane's rows: ri + rsub < ei
+#pragma unroll 1
+    for (int rk = 0; rk < ek; ++rk) {
 #pragma unroll
-        for (int e = 0; e < V; ++e) {
-            const int rj = q * V + e;
-            f[e] = box[base + (px ? rj : ej - 1 - rj)];
+        for (int u = 0; u < NY; ++u) {
+            if (u * RPI >= ny) continue;
+            const T* at = src + u * RPI * sy;
+            VT v;
+            T* f = reinterpret_cast<T*>(&v);
+#pragma unroll
+            for (int e = 0; e < V; ++e) f[e] = at[e * dx];
+            *reinterpret_cast<VT*>(dst + u * RPI * nc) = v;
         }
-        *reinterpret_cast<VT*>(fld + (k0 + rk) * plane + (long long)(i0 + ri) * nc + j0 + q * V) = v;
+        src += sz;
+        dst += plane;
     }
 }
 
@@ -526,31 +553,35 @@ __device__ __forceinline__ void load_interior(T* dst, const T* __restrict__ g, i
     const long long plane = (long long)nr * nc;
     if (vec) {
         using VT = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
-        constexpr int V = 16 / sizeof(T);
-        constexpr int MV = TJ / V, RPI = 32 / MV;
+        constexpr int V = 16 / sizeof(T), MV = TJ / V, RPI = 32 / MV;
+        constexpr int NY = TI / RPI, ZB = TK % 4 == 0 && NY == 1 ? 4 : 2;   // passes per plane, planes per batch
+        static_assert(TI % RPI == 0 && TK % ZB == 0, "whole batches");
         const int q = lane % MV, rsub = lane / MV;
-        const bool qok = q * V < ej;
+        const int sz = pz ? SPS : -SPS, sy = py ? SJ : -SJ, dx = px ? 1 : -1;
+        const T* src = g + k0 * plane + (long long)(i0 + rsub) * nc + j0 + q * V;
+        T* to = dst + (pz ? 0 : (ek - 1) * SPS) + (py ? 0 : (ei - 1) * SJ) + rsub * sy + (px ? q * V : ej - 1 - q * V);
+        const int ny = q * V < ej ? ei - rsub : 0;
 #pragma unroll 1
-        for (int r0 = 0; r0 < TK * TI; r0 += 4 * RPI) {
-            VT v[4];
+        for (int rk = 0; rk < ek; rk += ZB) {
+            VT v[ZB * NY];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int r = r0 + u * RPI + rsub, rk = r / TI, ri = r - rk * TI;
-                if (qok && rk < ek && ri < ei)
-                    v[u] = __ldg(reinterpret_cast<const VT*>(g + (k0 + rk) * plane + (long long)(i0 + ri) * nc + j0 + q * V));
-            }
+            for (int w = 0; w < ZB; ++w)
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int r = r0 + u * RPI + rsub, rk = r / TI, ri = r - rk * TI;
-                if (!(qok && rk < ek && ri < ei)) continue;
-                T* row = dst + (pz ? rk : ek - 1 - rk) * SPS + (py ? ri : ei - 1 - ri) * SJ;
-                const T* f = reinterpret_cast<const T*>(&v[u]);
+                for (int u = 0; u < NY; ++u)
+                    if (rk + w < ek && u * RPI < ny)
+                        v[w * NY + u] = __ldg(reinterpret_cast<const VT*>(src + w * plane + u * RPI * nc));
 #pragma unroll
-                for (int e = 0; e < V; ++e) {
-                    const int rj = q * V + e;
-                    row[px ? rj : ej - 1 - rj] = f[e];
-                }
-            }
+            for (int w = 0; w < ZB; ++w)
+#pragma unroll
+                for (int u = 0; u < NY; ++u)
+                    if (rk + w < ek && u * RPI < ny) {
+                        const T* f = reinterpret_cast<const T*>(&v[w * NY + u]);
+                        T* at = to + w * sz + u * RPI * sy;
+#pragma unroll
+                        for (int e = 0; e < V; ++e) at[e * dx] = f[e];
+                    }
+            src += ZB * plane;
+            to += ZB * sz;
         }
     } else {
         const int jf = px ? lane : ej - 1 - lane;
