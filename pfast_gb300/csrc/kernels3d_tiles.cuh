@@ -375,51 +375,67 @@ __device__ __forceinline__ double adj3_polish(double T0, double Txp, double Txm,
 // conflicts).  Halo position z = 0..ek+1 around a tile of ek planes (grid plane k0-1+z) lies
 // at flipped zf = z where the sweep ascends along z, else ek+1-z; likewise rows and columns.
 //
-// load_box: the halo box at origin (k0-1, i0-1, j0-1), one box row per warp instruction
-// (lanes along the row, coalesced); out-of-grid entries get `fill`; the rows and columns
-// beyond a partial tile's halo are neither loaded nor stored (never read).  Twelve rows are
-// loaded before they are stored, to keep many loads in flight.
+// The halo columns j0 - 1 and j0 + ej of the box, one element per lane: lane = (row, side).
+template <typename T, bool COHERENT, class SH>
+__device__ __forceinline__ void load_box_sides(T* box, const T* __restrict__ g, int k0, int i0, int j0, int ek, int ei,
+                                               int ej, bool pz, bool py, bool px, int nz, int nr, int nc, T fill,
+                                               int lane) {
+    PFAST_TILE_SHAPE(SH);
+    constexpr int NROW = HK * HI, NP = (NROW + 15) / 16;
+    const long long plane = (long long)nr * nc;
+    const int sz = pz ? PS : -PS, sy = py ? HJ : -HJ;
+    const int origin = (pz ? 0 : (ek + 1) * PS) + (py ? 0 : (ei + 1) * HJ);
+    const int side = lane & 1, gj = side ? j0 + ej : j0 - 1, bx = (side != 0) == px ? ej + 1 : 0;
+    const bool vin = (unsigned)gj < (unsigned)nc;
+    T v[NP];
+#pragma unroll
+    for (int u = 0; u < NP; ++u) {
+        const int r = u * 16 + (lane >> 1), z = r / HI, y = r - z * HI;
+        const bool ok = vin && z <= ek + 1 && y <= ei + 1 && (unsigned)(k0 - 1 + z) < (unsigned)nz &&
+                        (unsigned)(i0 - 1 + y) < (unsigned)nr;
+        v[u] = fill;
+        const T* at = g + (k0 - 1 + z) * plane + (long long)(i0 - 1 + y) * nc + gj;
+        if (ok) v[u] = COHERENT ? __ldcg(at) : __ldg(at);
+    }
+#pragma unroll
+    for (int u = 0; u < NP; ++u) {
+        const int r = u * 16 + (lane >> 1), z = r / HI, y = r - z * HI;
+        if (z <= ek + 1 && y <= ei + 1) box[origin + z * sz + y * sy + bx] = v[u];
+    }
+}
+
+// load_box: the halo box at origin (k0-1, i0-1, j0-1), one tile row per warp instruction
+// (lane = column, coalesced), a plane's rows in flight together; out-of-grid entries get `fill`;
+// the rows and columns beyond a partial tile's halo are neither loaded nor stored (never read).
 // COHERENT: the field, which the dataflow kernel itself writes (other warps of the block
 // stored the neighbouring tiles): read through L2, not the read-only path.
 template <typename T, bool COHERENT, class SH>
 __device__ __forceinline__ void load_box(T* box, const T* __restrict__ g, int k0, int i0, int j0, int ek, int ei,
                                          int ej, bool pz, bool py, bool px, int nz, int nr, int nc, T fill, int lane) {
     PFAST_TILE_SHAPE(SH);
-    constexpr int NROW = HK * HI;
-    constexpr int RB = 12;
-    static_assert(NROW % RB == 0 && HJ - 32 <= 32, "row batching");
     const long long plane = (long long)nr * nc;
-    const int gj0 = j0 - 1 + lane, gj1 = j0 + 31 + lane;
-    const bool s0 = lane <= ej + 1, s1 = lane < HJ - 32 && lane + 32 <= ej + 1;   // within the halo
-    const bool c0 = s0 && (unsigned)gj0 < (unsigned)nc;
-    const bool c1 = s1 && (unsigned)gj1 < (unsigned)nc;
-    const int xf0 = px ? lane : ej + 1 - lane, xf1 = px ? lane + 32 : ej - 31 - lane;
+    const int sz = pz ? PS : -PS, sy = py ? HJ : -HJ;
+    const int y0 = i0 ? 0 : 1, y1 = min(ei + 2, nr - i0 + 1);   // box rows in the grid
+    const bool in = lane < ej;
+    const T* src = g + (k0 - 1) * plane + (long long)(i0 - 1) * nc + j0 + (in ? lane : 0);
+    T* dst = box + (pz ? 0 : (ek + 1) * PS) + (py ? 0 : (ei + 1) * HJ) + (px ? 1 + lane : ej - lane);
 #pragma unroll 1
-    for (int rb = 0; rb < NROW; rb += RB) {
-        T v0[RB], v1[RB];
+    for (int z = 0; z <= ek + 1; ++z) {
+        const bool zin = (unsigned)(k0 - 1 + z) < (unsigned)nz;
+        T v[HI];
 #pragma unroll
-        for (int u = 0; u < RB; ++u) {
-            const int r = rb + u, z = r / HI, y = r - z * HI;
-            const int gk = k0 - 1 + z, gi = i0 - 1 + y;
-            const bool rok = z <= ek + 1 && y <= ei + 1 && (unsigned)gk < (unsigned)nz && (unsigned)gi < (unsigned)nr;
-            const T* row = g + gk * plane + (long long)gi * nc;
-            if constexpr (COHERENT) {
-                v0[u] = (rok && c0) ? __ldcg(row + gj0) : fill;
-                v1[u] = (rok && c1) ? __ldcg(row + gj1) : fill;
-            } else {
-                v0[u] = (rok && c0) ? __ldg(row + gj0) : fill;
-                v1[u] = (rok && c1) ? __ldg(row + gj1) : fill;
-            }
+        for (int y = 0; y < HI; ++y) {
+            v[y] = fill;
+            const T* at = src + y * nc;
+            if (zin && y >= y0 && y < y1) v[y] = COHERENT ? __ldcg(at) : __ldg(at);
         }
 #pragma unroll
-        for (int u = 0; u < RB; ++u) {
-            const int r = rb + u, z = r / HI, y = r - z * HI;
-            if (z > ek + 1 || y > ei + 1) continue;
-            T* brow = box + (pz ? z : ek + 1 - z) * PS + (py ? y : ei + 1 - y) * HJ;
-            if (s0) brow[xf0] = v0[u];
-            if (s1) brow[xf1] = v1[u];
-        }
+        for (int y = 0; y < HI; ++y)
+            if (in && y <= ei + 1) dst[y * sy] = v[y];
+        src += plane;
+        dst += sz;
     }
+    load_box_sides<T, COHERENT, SH>(box, g, k0, i0, j0, ek, ei, ej, pz, py, px, nz, nr, nc, fill, lane);
 }
 
 // Vector form of load_box, for grids whose rows start on 16-byte boundaries (ncols a multiple of
@@ -487,25 +503,26 @@ __device__ __forceinline__ void load_box_vec(T* box, const T* __restrict__ g, in
             dst += RZ * ZB * sz;
         }
     }
-    {   // the halo columns j0 - 1 and j0 + ej: lane = (row, side)
-        constexpr int NROW = HK * HI, NP = (NROW + 15) / 16;
-        const int side = lane & 1, gj = side ? j0 + ej : j0 - 1, bx = (side != 0) == px ? ej + 1 : 0;
-        const bool vin = (unsigned)gj < (unsigned)nc;
-        T v[NP];
+    load_box_sides<T, COHERENT, SH>(box, g, k0, i0, j0, ek, ei, ej, pz, py, px, nz, nr, nc, fill, lane);
+}
+
+// Write-back with one row per warp instruction, for the other grids.
+template <typename T, class SH>
+__device__ __forceinline__ void store_tile(T* __restrict__ fld, const T* box, int k0, int i0, int j0, int ek, int ei, int ej,
+                                           bool pz, bool py, bool px, int nr, int nc, int lane) {
+    PFAST_TILE_SHAPE(SH);
+    if (lane >= ej) return;
+    const long long plane = (long long)nr * nc;
+    const int sz = pz ? PS : -PS, sy = py ? HJ : -HJ;
+    const T* src = box + (pz ? PS : ek * PS) + (py ? HJ : ei * HJ) + (px ? 1 + lane : ej - lane);
+    T* dst = fld + k0 * plane + (long long)i0 * nc + j0 + lane;
+#pragma unroll 1
+    for (int rk = 0; rk < ek; ++rk) {
 #pragma unroll
-        for (int u = 0; u < NP; ++u) {
-            const int r = u * 16 + (lane >> 1), z = r / HI, y = r - z * HI;
-            const bool ok = vin && z <= ek + 1 && y <= ei + 1 && (unsigned)(k0 - 1 + z) < (unsigned)nz &&
-                            (unsigned)(i0 - 1 + y) < (unsigned)nr;
-            v[u] = fill;
-            const T* at = g + (k0 - 1 + z) * plane + (long long)(i0 - 1 + y) * nc + gj;
-            if (ok) v[u] = COHERENT ? __ldcg(at) : __ldg(at);
-        }
-#pragma unroll
-        for (int u = 0; u < NP; ++u) {
-            const int r = u * 16 + (lane >> 1), z = r / HI, y = r - z * HI;
-            if (z <= ek + 1 && y <= ei + 1) box[origin + z * sz + y * sy + bx] = v[u];
-        }
+        for (int ri = 0; ri < TI; ++ri)
+            if (ri < ei) dst[ri * nc] = src[ri * sy];
+        src += sz;
+        dst += plane;
     }
 }
 
@@ -584,21 +601,21 @@ __device__ __forceinline__ void load_interior(T* dst, const T* __restrict__ g, i
             to += ZB * sz;
         }
     } else {
-        const int jf = px ? lane : ej - 1 - lane;
+        if (lane >= ej) return;
+        const int sz = pz ? SPS : -SPS, sy = py ? SJ : -SJ;
+        const T* src = g + k0 * plane + (long long)i0 * nc + j0 + lane;
+        T* to = dst + (pz ? 0 : (ek - 1) * SPS) + (py ? 0 : (ei - 1) * SJ) + (px ? lane : ej - 1 - lane);
 #pragma unroll 1
-        for (int m0 = 0; m0 < TK * TI; m0 += 8) {
-            T v[8];
+        for (int rk = 0; rk < ek; ++rk) {
+            T v[TI];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const int rk = (m0 + u) / TI, ri = (m0 + u) % TI;
-                if (rk < ek && ri < ei && lane < ej) v[u] = __ldg(g + (k0 + rk) * plane + (long long)(i0 + ri) * nc + j0 + lane);
-            }
+            for (int ri = 0; ri < TI; ++ri)
+                if (ri < ei) v[ri] = __ldg(src + ri * nc);
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const int rk = (m0 + u) / TI, ri = (m0 + u) % TI;
-                if (rk < ek && ri < ei && lane < ej)
-                    dst[(pz ? rk : ek - 1 - rk) * SPS + (py ? ri : ei - 1 - ri) * SJ + jf] = v[u];
-            }
+            for (int ri = 0; ri < TI; ++ri)
+                if (ri < ei) to[ri * sy] = v[ri];
+            src += plane;
+            to += sz;
         }
     }
 }
@@ -1192,17 +1209,9 @@ __device__ __forceinline__ void process_tile(const Sweep3Args& A, const int inst
     // ---- write back (UWIN: stored as updated); the FP64 kinds compare with the iteration-start
     // snapshot
     if constexpr (!kSnap) {
-        if constexpr (UWIN) {
-        } else if (A.vec_rows) {
-            store_tile_vec<Real, SH>(fld, box, k0, i0, j0, ek, ei, ej, pz, py, px, nr, nc, lane);
-        } else {
-#pragma unroll 8
-            for (int m = 0; m < 32; ++m) {
-                const int rk = m / TI, ri = m % TI;
-                if (rk < ek && ri < ei && lane < ej)
-                    fld[(k0 + rk) * plane + (long long)(i0 + ri) * nc + j0 + lane] =
-                        box[box_index<SH>(rk, ri, lane, ek, ei, ej, pz, py, px)];
-            }
+        if constexpr (!UWIN) {
+            if (A.vec_rows) store_tile_vec<Real, SH>(fld, box, k0, i0, j0, ek, ei, ej, pz, py, px, nr, nc, lane);
+            else store_tile<Real, SH>(fld, box, k0, i0, j0, ek, ei, ej, pz, py, px, nr, nc, lane);
         }
         if (__any_sync(0xffffffffu, moved) && lane == 0) A.diff[(long long)inst * A.ntiles + tid] = 1;
     } else {
