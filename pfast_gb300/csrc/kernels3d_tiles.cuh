@@ -881,12 +881,20 @@ __device__ __forceinline__ void process_tile(const Sweep3Args& A, const int inst
     // outside the tile are tracked by owner lanes at their consumer's position: lanes 0..TI-1
     // the flipped k-1 face, the next TI the k+1 face, then TK lanes each for the i-1 and i+1
     // faces (24 lanes in both tile shapes).
-    const Aux* Tb = TWIN ? reinterpret_cast<const Aux*>(A.aux) + inst * A.fstride : nullptr;
-    const Aux* trow = (TWIN && lane_ok) ? Tb + rowbase : nullptr;
-    const Aux* hrow = nullptr;
-    const Real* urow = (UWIN && lane_ok) ? fld + rowbase : nullptr;   // the field's windows (UWIN)
-    const Real* uhrow = nullptr;
+    // The adjoint's windows load without conditions: the column is clamped into the grid, a lane
+    // without a row reads the tile's first.  What such a load returns is never used, as the nodes
+    // of the grid's faces are fixed (adjoint polish of 256 sources of 256 x 256 x 128 nodes: 249 to
+    // 243 ms, of a batch of 8 grids of 0.2-0.9 million nodes with 4-40 sources: 21.7 to 20.7).  The forward needs the fill outside the
+    // grid; selecting it where it is used, after the same unconditional loads, was slower (305
+    // to 328 ms), so its loads keep their conditions.
+    const long long wrow = lane_ok ? rowbase : k0 * plane + (long long)i0 * nc;
+    auto wcol = [&](int p) { return min(max(gjA + dj * p, 0), nc - 1); };
+    const Aux* trow = TWIN ? reinterpret_cast<const Aux*>(A.aux) + inst * A.fstride + wrow : nullptr;
+    const Aux* hrow = trow;
+    const Real* urow = UWIN ? fld + wrow : nullptr;   // the field's windows (UWIN)
+    const Real* uhrow = urow;
     int hpos = 0;
+    bool hvalid = false;
     if constexpr (TWIN || UWIN) {
         int lkh = 0, lih = 0;
         bool own = false;
@@ -903,38 +911,34 @@ __device__ __forceinline__ void process_tile(const Sweep3Args& A, const int inst
             hpos = lo ? y : y + ei - 1;
         }
         const int gkh = k0 + lkh, gih = i0 + lih;
-        if (own && (unsigned)gkh < (unsigned)nz && (unsigned)gih < (unsigned)nr) {
-            if constexpr (TWIN) hrow = Tb + gkh * plane + (long long)gih * nc;
-            if constexpr (UWIN) uhrow = fld + gkh * plane + (long long)gih * nc;
-        }
+        hvalid = own && (unsigned)gkh < (unsigned)nz && (unsigned)gih < (unsigned)nr;
+        const long long hoff = hvalid ? gkh * plane + (long long)gih * nc - wrow : 0;
+        hrow += TWIN ? hoff : 0;
+        uhrow += UWIN ? hoff : 0;
     }
-    // traveltime of pencil row r at flipped position p, zero outside [plo, phi] or the grid
-    auto tload = [&](const Aux* r, int p, int plo, int phi) -> Aux {
-        const int g = j0 + (px ? p : ej - 1 - p);
-        return (r != nullptr && p >= plo && p <= phi && (unsigned)g < (unsigned)nc) ? __ldg(r + g) : Aux(0);
-    };
     const int jf0 = -lkf - lif;
     Aux tm = Aux(0), t0 = Aux(0), tp = Aux(0), q1 = Aux(0), q2 = Aux(0), h0 = Aux(0), hq1 = Aux(0), hq2 = Aux(0);
     if constexpr (TWIN) {
-        tm = tload(trow, jf0 - 1, -1, ej); t0 = tload(trow, jf0, -1, ej); tp = tload(trow, jf0 + 1, -1, ej);
-        q1 = tload(trow, jf0 + 2, -1, ej); q2 = tload(trow, jf0 + 3, -1, ej);
-        h0 = tload(hrow, -hpos, 0, ej - 1); hq1 = tload(hrow, 1 - hpos, 0, ej - 1); hq2 = tload(hrow, 2 - hpos, 0, ej - 1);
+        tm = __ldg(trow + wcol(jf0 - 1)); t0 = __ldg(trow + wcol(jf0)); tp = __ldg(trow + wcol(jf0 + 1));
+        q1 = __ldg(trow + wcol(jf0 + 2)); q2 = __ldg(trow + wcol(jf0 + 3));
+        h0 = __ldg(hrow + wcol(-hpos)); hq1 = __ldg(hrow + wcol(1 - hpos)); hq2 = __ldg(hrow + wcol(2 - hpos));
     }
-    // field of pencil row r at flipped position p: the fill outside [plo, phi] or the grid (UWIN)
-    auto uload = [&](const Real* r, int p, int plo, int phi) -> Real {
-        const int g = j0 + (px ? p : ej - 1 - p);
-        if (r == nullptr || p < plo || p > phi || (unsigned)g >= (unsigned)nc) return fill;
-        if constexpr (COHERENT) return __ldcg(r + g);
-        else return __ldg(r + g);
+    // field of pencil row `row` at flipped position p (UWIN); forward: the fill outside the tile's
+    // box (its last position `end`) or the grid
+    auto uread = [&](const Real* at) -> Real { return COHERENT ? __ldcg(at) : __ldg(at); };
+    auto uload = [&](const Real* row, bool own, int p, int end) -> Real {
+        if constexpr (ADJ) return uread(row + wcol(p));
+        const int g = gjA + dj * p;
+        return own && p >= end - ej - 1 && p <= end && (unsigned)g < (unsigned)nc ? uread(row + g) : fill;
     };
     // UWIN: um = new value at jf-1, u0 / up / uq1 / uq2 = old values at jf .. jf+3; uh*: the
     // owned halo pencil at the consumer's position and two ahead
     Real um = Real(0), u0 = Real(0), up = Real(0), uq1 = Real(0), uq2 = Real(0);
     Real uh0 = Real(0), uhq1 = Real(0), uhq2 = Real(0);
     if constexpr (UWIN) {
-        um = uload(urow, jf0 - 1, -1, ej); u0 = uload(urow, jf0, -1, ej); up = uload(urow, jf0 + 1, -1, ej);
-        uq1 = uload(urow, jf0 + 2, -1, ej); uq2 = uload(urow, jf0 + 3, -1, ej);
-        uh0 = uload(uhrow, -hpos, 0, ej - 1); uhq1 = uload(uhrow, 1 - hpos, 0, ej - 1); uhq2 = uload(uhrow, 2 - hpos, 0, ej - 1);
+        um = uload(urow, lane_ok, jf0 - 1, ej); u0 = uload(urow, lane_ok, jf0, ej); up = uload(urow, lane_ok, jf0 + 1, ej);
+        uq1 = uload(urow, lane_ok, jf0 + 2, ej); uq2 = uload(urow, lane_ok, jf0 + 3, ej);
+        uh0 = uload(uhrow, hvalid, -hpos, ej - 1); uhq1 = uload(uhrow, hvalid, 1 - hpos, ej - 1); uhq2 = uload(uhrow, hvalid, 2 - hpos, ej - 1);
     }
 
     bool f_klo = false, f_khi = false, f_ilo = false, f_ihi = false, f_jlo = false, f_jhi = false;   // grid face marks
@@ -1056,7 +1060,8 @@ __device__ __forceinline__ void process_tile(const Sweep3Args& A, const int inst
         Real res = u0;   // UWIN: this lane's value at jf after the step
         if ((unsigned)ljf < (unsigned)ej) {
             const int c = cl + t;
-            const Real xu = UWIN ? um : box[c - 1], xd = UWIN ? up : box[c + 1];
+            const Real xu = UWIN ? um : box[c - 1];
+            const Real xd = UWIN ? up : box[c + 1];
             const Real yu = UWIN ? wyu : box[c - HJ], yd = UWIN ? wyd : box[c + HJ];
             const Real zu = UWIN ? wzu : box[c - PS], zd = UWIN ? wzd : box[c + PS];
             const Real old = UWIN ? u0 : box[c];
@@ -1157,12 +1162,12 @@ __device__ __forceinline__ void process_tile(const Sweep3Args& A, const int inst
             }
         }
         if constexpr (TWIN) {   // slide the windows to step t + 1
-            tm = t0; t0 = tp; tp = q1; q1 = q2; q2 = tload(trow, t + 4 - lkf - lif, -1, ej);
-            h0 = hq1; hq1 = hq2; hq2 = tload(hrow, t + 3 - hpos, 0, ej - 1);
+            tm = t0; t0 = tp; tp = q1; q1 = q2; q2 = __ldg(trow + wcol(t + 4 - lkf - lif));
+            h0 = hq1; hq1 = hq2; hq2 = __ldg(hrow + wcol(t + 3 - hpos));
         }
         if constexpr (UWIN) {
-            um = res; u0 = up; up = uq1; uq1 = uq2; uq2 = uload(urow, t + 4 - lkf - lif, -1, ej);
-            uh0 = uhq1; uhq1 = uhq2; uhq2 = uload(uhrow, t + 3 - hpos, 0, ej - 1);
+            um = res; u0 = up; up = uq1; uq1 = uq2; uq2 = uload(urow, lane_ok, t + 4 - lkf - lif, ej);
+            uh0 = uhq1; uhq1 = uhq2; uhq2 = uload(uhrow, hvalid, t + 3 - hpos, ej - 1);
         }
         if constexpr (!UWIN) __syncwarp();
     }
