@@ -1851,7 +1851,7 @@ pfast_status dataflow_shape_k(int ntiles, int nact, bool multi, DataflowShape* o
     constexpr bool kPlain = KIND == kFwdPlain64 || KIND == kAdjPlain64;
     *out = DataflowShape();
     // the largest cluster size at which every instance has a cluster of its own at the same time
-    for (int cs = kMaxCluster; cs >= 1 && !out->warps; cs /= 2) {
+    for (int cs = kMaxCluster; cs >= 1 && !out->warps; --cs) {
         if (cs > 1 && !cluster_wanted(cs, kPlain, nact, ntiles, sms)) continue;
         const int form = dataflow_form<KIND>(cs, ntiles);
         const DataflowKernel k = dataflow_kernel<KIND, SH>(multi, cs > 1, form);

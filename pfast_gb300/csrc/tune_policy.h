@@ -62,10 +62,14 @@ inline int tune_pick(const TuneEntry* e, unsigned allowed, int nact, int sms) {
 // Measured (ms of a mixed gradient of 128 x 128 x 64 nodes, blocks per source): 64 sources 95 (1), 81
 // (2); 40 sources 71 (2), 70 (4); 100 sources 99 (1), 103 (2); plain, 96 x 96 x 48: 16 sources 602
 // (1), 331 (2), 202 (4), 175 (8), 287 (16); 40 sources 331 (2), 299 (4).
+// Any size, not powers of two alone, which left up to half of the SMs idle just above a step
+// (plain gradient of 128 x 128 x 100: 21 sources 628 ms with 4 blocks, 395 with 7; 96 x 96 x 48: 42
+// sources 314 (2), 223 (3); mixed, 128 x 128 x 100: 13 sources 53 (8), 46 (15)).  Sizes of 9 to 15 only on
+// grids of 100 tiles a block: 12 sources of 96 x 96 x 48 (432 tiles) took 126 ms with 8 blocks, 162 with 13.
 constexpr int kMaxCluster = 16;
 
 inline bool cluster_wanted(int cs, bool plain, int nact, int ntiles, int sms) {
-    return 10LL * nact * cs <= (plain ? 11LL : 13LL) * sms && ntiles >= 8 * cs;
+    return 10LL * nact * cs <= (plain ? 11LL : 13LL) * sms && ntiles >= (cs > 8 && cs < kMaxCluster ? 100 : 8) * cs;
 }
 
 // Warps per block of a cluster.  Few: the ready tiles of a source are few as well, and what
@@ -82,19 +86,24 @@ inline int cluster_warps(int cs, bool plain) {
 }
 
 // The candidate of a phase that has not been timed, among `allowed` (tune_allowed): the dataflow
-// kernel, except where one launch per tile diagonal is ahead: the plain kinds with one block per
-// instance and fewer instances than SMs (100 sources of 96 x 96 x 48: 566 against 706 ms; 200 sources
-// 880 against 722), and the FP32 bulk kinds with one block per instance where a diagonal
-// holds many tiles (256 sources of 256 x 256 x 128, 30,000 tiles a diagonal: forward 193 against 214 ms;
-// 300 sources of 128 x 128 x 64, 9,000: 30 against 26).  cluster: blocks per instance of the dataflow
-// kernel; plain / fp32: the phase's kind (neither: polish).
+// kernel, except where one launch per tile diagonal is ahead:
+// - the plain kinds, whose FP64 pipe needs one warp per SM sub-partition only, with at most three
+//   blocks per instance that leave SMs idle, where a diagonal holds enough tiles for all SMs.
+//   Gradients, ms per diagonal / dataflow (tiles a diagonal): 84 sources of 96 x 96 x 48 393 / 552
+//   (1450), 61 of 226 x 35 x 68 723 / 924 (1480), 49 of 100 x 171 x 47 738 / 790-880 (1440), 64 of
+//   96 x 96 x 48 352 / 333 (1110), 84 of 64 x 64 x 32 165 / 151 (670); one block each from three
+//   quarters of the SMs on: 119 of 67 x 137 x 26 504 / 427 (2100), 123 of 104 x 125 x 25 579 / 493
+//   (2200); two or three each from all SMs on: forward of 79 of 37 x 126 x 108 575 / 472 (1590);
+// - the FP32 bulk kinds with one block per instance where a diagonal holds many tiles (256 sources
+//   of 256 x 256 x 128, 30,000 tiles a diagonal: forward 165 / 176, adjoint 242 / 250; 256
+//   sources of 96 x 96 x 48, 4,400: 12.3 / 8.8, 14.6 / 11.6).
+// cluster: blocks per instance of the dataflow kernel; plain / fp32: the phase's kind (neither: polish).
 inline int untuned_pick(unsigned allowed, bool plain, bool fp32, int cluster, int nact, long long ntiles, int ndiag,
                         int sms) {
     bool dataflow = true;
-    if (cluster <= 1) {
-        if (plain) dataflow = nact >= sms;
-        if (fp32) dataflow = ntiles * nact < 16384LL * ndiag;
-    }
+    if (plain)
+        dataflow = cluster > 3 || 4 * nact * cluster >= (cluster > 1 ? 4 : 3) * sms || ntiles * nact < 1200LL * ndiag;
+    if (fp32 && cluster <= 1) dataflow = ntiles * nact < 16384LL * ndiag;
     const int order[2][kTuneCandidates] = {{0, 1, 2, 3, 4, 5}, {2, 3, 4, 5, 0, 1}};
     for (int c : order[dataflow])
         if (allowed >> c & 1) return c;

@@ -1,7 +1,7 @@
 """The dataflow schedule with a thread-block cluster per source: the policy that picks the cluster
 size and the untuned schedule (pfast_gb300/csrc/tune_policy.h, compiled with g++), and on the GPU
-the same bits as one launch per tile diagonal for source counts that give clusters of 16, 8, 4, 2
-and 1 blocks, whole and ragged tiles, equal and unequal spacings."""
+the same bits as one launch per tile diagonal for source counts that give clusters of 1 to 9
+blocks and of the tile count's most, whole and ragged tiles, equal and unequal spacings."""
 import os
 import shutil
 import subprocess
@@ -19,18 +19,23 @@ using namespace pfast;
 static int n = 0;
 static void eq(long long got, long long want) { ++n; std::printf("%s %d: %lld %lld\n", got == want ? "ok" : "FAIL", n, got, want); }
 static int size(bool plain, int nact, int ntiles) {
-    for (int cs = kMaxCluster; cs > 1; cs /= 2) if (cluster_wanted(cs, plain, nact, ntiles, 152)) return cs;
+    for (int cs = kMaxCluster; cs > 1; --cs) if (cluster_wanted(cs, plain, nact, ntiles, 152)) return cs;
     return 1;
 }
 int main() {
     eq(size(true, 1, 1024), 16); eq(size(true, 16, 432), 8); eq(size(true, 40, 432), 4); eq(size(true, 100, 432), 1);
-    eq(size(false, 9, 378), 16); eq(size(false, 24, 1300), 8); eq(size(false, 64, 1024), 2); eq(size(false, 256, 8192), 1);
+    eq(size(false, 9, 378), 16); eq(size(false, 24, 1300), 8); eq(size(false, 64, 1024), 3); eq(size(false, 256, 8192), 1);
     eq(size(false, 1, 80), 8); eq(size(false, 1, 15), 1);
+    eq(size(true, 21, 1600), 7); eq(size(true, 42, 432), 3); eq(size(true, 12, 432), 8); eq(size(true, 12, 1300), 13);
     for (int cs = 2; cs <= 16; cs *= 2) eq(cluster_warps(cs, true) >= 4 && cluster_warps(cs, false) <= 24, 1);
     // schedule: candidate 2 = dataflow 4x8x32, 0 = per diagonal 4x8x32
     eq(untuned_pick(0x3f, true, false, 16, 1, 1024, 34, 152), 2);
     eq(untuned_pick(0x3f, true, false, 1, 100, 432, 26, 152), 0);
     eq(untuned_pick(0x3f, true, false, 1, 200, 432, 26, 152), 2);
+    eq(untuned_pick(0x3f, true, false, 1, 84, 128, 16, 152), 2);      // few tiles a diagonal
+    eq(untuned_pick(0x3f, true, false, 2, 61, 680, 28, 152), 0);
+    eq(untuned_pick(0x3f, true, false, 2, 79, 864, 43, 152), 2);
+    eq(untuned_pick(0x3f, true, false, 7, 23, 1736, 44, 152), 2);
     eq(untuned_pick(0x3f, false, true, 1, 256, 8192, 70, 152), 0);
     eq(untuned_pick(0x3f, false, true, 1, 300, 1024, 34, 152), 2);
     eq(untuned_pick(0x3f, false, false, 1, 256, 8192, 70, 152), 2);
@@ -53,13 +58,14 @@ def test_cluster_and_schedule_policy(tmp_path):
     src.write_text(CHECK)
     subprocess.run([gxx, "-std=c++17", "-O1", "-I", os.path.join(ROOT, "pfast_gb300", "csrc"), str(src), "-o", exe], check=True)
     out = subprocess.run([exe], capture_output=True, text=True, timeout=60).stdout
-    assert "FAIL" not in out and out.count("ok ") == 26, out
+    assert "FAIL" not in out and out.count("ok ") == 34, out
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("nsrc", [1, 9, 30, 60, 170])
-@pytest.mark.parametrize("shape,d", [((16, 33, 64), (20.0, 20.0, 20.0)), ((21, 41, 70), (16.7, 12.5, 20.0))])
-def test_cluster_dataflow_same_bits(nsrc, shape, d):
+@pytest.mark.parametrize("shape,d,nsrc", [((16, 33, 64), (20.0, 20.0, 20.0), n) for n in (1, 30, 45, 170)] +
+                         [((21, 41, 70), (16.7, 12.5, 20.0), n) for n in (1, 9, 22, 27, 60)] +
+                         [((40, 72, 320), (20.0, 20.0, 20.0), 17)])
+def test_cluster_dataflow_same_bits(shape, d, nsrc):
     import torch
     import pfast_gb300 as pg
     nz, nr, nc = shape
