@@ -52,10 +52,12 @@ typedef struct {
                              1e-9 convergence tolerance. */
     int schedule;         /* 3D sweeps: 0 = automatic (per sweep kind, the fastest schedule and
                              tile shape measured by pfast_survey3d_autotune for this grid shape and
-                             source count; untuned: persistent from 2 sources per SM), 1 = one launch
+                             source count; untuned: persistent, except where a rule on source count
+                             and grid expects 1 to be ahead), 1 = one launch
                              per tile diagonal (every tile of every source spread over all SMs), 2 =
-                             persistent: one dataflow launch per phase, one block solves one source
-                             with its sweep orders overlapping as the tile dependencies allow (grids
+                             persistent: one dataflow launch per phase; a block, or a cluster of up to
+                             16 blocks where there are fewer sources than SMs, solves one source with
+                             its sweep orders overlapping as the tile dependencies allow (grids
                              of at most 8192 tiles; larger grids use 1), 3 = hybrid: the first outer
                              iteration per tile diagonal, the rest in the dataflow kernel.  Same
                              results. */

@@ -252,17 +252,18 @@ pfast_status run_sweeps3(pfast_ctx* ctx, Sweep3Args a, int kind, int nb, std::ve
                          int* iters, long long nodes_per_sweep, long long* node_updates, int* not_conv,
                          double* ms_acc) {
     // Three schedules.  Per-diagonal launches spread every tile of every active instance over
-    // all SMs (one warp per tile) and suit surveys with few instances; the dataflow kernel
-    // (one block solves one instance, its sweep orders overlapping as their tile dependencies
-    // allow, no host round trip per iteration) suits runs with about one instance per SM or
-    // more; the hybrid runs the first, dense outer iteration per diagonal and the sparse rest
+    // all SMs (one warp per tile) and suit phases whose diagonals hold many tiles; in the
+    // dataflow kernel a block or a cluster of blocks solves one instance, its sweep orders
+    // overlapping as their tile dependencies allow, with no host round trip per iteration; the
+    // hybrid runs the first, dense outer iteration per diagonal and the sparse rest
     // in the dataflow kernel.  Two tile shapes, 4x8x32 and 8x4x32 nodes in sweep-order axes.
-    // Automatic: the autotuner above.  Grids whose tiles do not fit the dataflow kernel's
-    // shared memory use the per-diagonal launches.
+    // Automatic: the autotuner above, and untuned_pick before it has run.  Grids whose tiles do
+    // not fit the dataflow kernel's shared memory use the per-diagonal launches.
     int dev = 0, sms = 1;
     PFAST_CUDA_TRY(cudaGetDevice(&dev));
     PFAST_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const auto tkey = std::make_tuple(dev, kind, a.nz, a.nr, a.nc, (int)active.size());
+    const int load = (int)active.size() * ctx->share();
     DataflowShape dshape[kTileShapes];
     bool fits[kTileShapes] = {};
     for (int shape = 0; shape < kTileShapes; ++shape) {
@@ -270,7 +271,7 @@ pfast_status run_sweeps3(pfast_ctx* ctx, Sweep3Args a, int kind, int nb, std::ve
         DiagTable3* t = nullptr;
         PFAST_TRY(ctx_diag3(ctx, a.nz, a.nr, a.nc, shape, &t));
         const int ntl = t->nbk * t->nbi * t->nbj;
-        if (!active.empty()) PFAST_TRY(dataflow_shape(kind, shape, ntl, (int)active.size(), &dshape[shape]));
+        if (!active.empty()) PFAST_TRY(dataflow_shape(kind, shape, ntl, (int)active.size(), load, &dshape[shape]));
         fits[shape] = dshape[shape].warps > 0;
     }
     const unsigned allowed = tune_allowed(ctx->schedule, ctx->tile_shape, fits);
@@ -280,7 +281,7 @@ pfast_status run_sweeps3(pfast_ctx* ctx, Sweep3Args a, int kind, int nb, std::ve
         DiagTable3* t = nullptr;
         PFAST_TRY(ctx_diag3(ctx, a.nz, a.nr, a.nc, shape, &t));
         cand = untuned_pick(allowed, kind == kFwdPlain64 || kind == kAdjPlain64, kind == kFwdFast32 || kind == kAdjFast32,
-                            dshape[shape].cluster, (int)active.size(), (long long)t->nbk * t->nbi * t->nbj, t->ndiag, sms);
+                            dshape[shape].cluster, load, (long long)t->nbk * t->nbi * t->nbj, t->ndiag, sms);
     }
     ctx->candidates = (ctx->candidates & ~(15 << 4 * kind)) | (cand + 1) << 4 * kind;
     const bool persistent = cand >> 1 == 1, hybrid = cand >> 1 == 2;
@@ -940,10 +941,14 @@ static pfast_status survey3d_create_impl(pfast_ctx* ctx, int nrows, int ncols, i
         return PFAST_OK;
     }
     auto up = [&](void** dst, const void* h, size_t bytes) -> pfast_status {
-        PFAST_CUDA_TRY(cudaMalloc(dst, std::max<size_t>(bytes, 16)));
-        if (bytes) PFAST_CUDA_TRY(cudaMemcpy(*dst, h, bytes, cudaMemcpyHostToDevice));
+        if (sv->astream) PFAST_CUDA_TRY(cudaMallocAsync(dst, std::max<size_t>(bytes, 16), sv->astream));
+        else PFAST_CUDA_TRY(cudaMalloc(dst, std::max<size_t>(bytes, 16)));
+        if (!(bytes)) return PFAST_OK;
+        if (sv->astream) PFAST_CUDA_TRY(cudaMemcpyAsync(*dst, h, bytes, cudaMemcpyHostToDevice, sv->astream));
+        else PFAST_CUDA_TRY(cudaMemcpy(*dst, h, bytes, cudaMemcpyHostToDevice));
         return PFAST_OK;
     };
+    sv->astream = ctx->resident_stream;
     if (!stt) stt = up((void**)&sv->d_src_kij, kij.data(), sizeof(int) * 3 * nsrc);
     if (!stt) stt = up((void**)&sv->d_src_lin, lin.data(), sizeof(long long) * nsrc);
     if (!stt) stt = up((void**)&sv->d_ch0, sv->h_ch0.data(), sizeof(int) * (nsrc + 1));
@@ -952,6 +957,11 @@ static pfast_status survey3d_create_impl(pfast_ctx* ctx, int nrows, int ncols, i
     if (!stt) stt = up((void**)&sv->d_nxyz, sv->has_picks ? nxyz : nullptr, sv->has_picks ? sizeof(double) * 3 * nrec : 0);
     if (!stt) stt = up((void**)&sv->d_tobs, sv->has_picks ? T_obs : nullptr, sv->has_picks ? sizeof(double) * nrec : 0);
     if (!stt) stt = up((void**)&sv->d_last, last.data(), sizeof(unsigned char) * nrec);
+    // the host tables above are freed when this function returns
+    if (!stt && sv->astream) {
+        const cudaError_t e = cudaStreamSynchronize(sv->astream);
+        if (e != cudaSuccess) stt = cuda_fail(e, "survey upload", __FILE__, __LINE__);
+    }
     if (stt) { pfast_survey3d_destroy(sv); return stt; }
     *out = sv;
     return PFAST_OK;
@@ -970,7 +980,8 @@ pfast_status pfast_survey3d_destroy(pfast_survey3d* sv) {
     if (sv->borrowed) { delete sv; return PFAST_OK; }   // the context's buffers
     for (void* p : {(void*)sv->d_src_kij, (void*)sv->d_src_lin, (void*)sv->d_ch0, (void*)sv->d_srnum, (void*)sv->d_rec,
                     (void*)sv->d_nxyz, (void*)sv->d_tobs, (void*)sv->d_last})
-        if (p) cudaFree(p);
+        if (p && sv->astream) cudaFreeAsync(p, sv->astream);
+        else if (p) cudaFree(p);
     delete sv;
     return PFAST_OK;
 }

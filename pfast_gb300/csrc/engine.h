@@ -2,6 +2,8 @@
 // buffers, surveys and the sweep driver.
 #pragma once
 
+#include <algorithm>
+#include <atomic>
 #include <map>
 #include <tuple>
 #include <vector>
@@ -79,10 +81,17 @@ struct pfast_ctx {
     int tile_shape = PFAST_TILE_AUTO;           // of the current 3D evaluation (pfast_options)
     int candidates = 0;                         // per sweep kind: 1 + candidate of its last phase (pfast_stats)
     int near_radius = 0;                        // of the current 3D evaluation (pfast_options)
+    // request server: requests that run at the same time (read at the start of each sweep phase)
+    const std::atomic<int>* running = nullptr;
+    int share() const { return running ? std::max(1, running->load(std::memory_order_relaxed)) : 1; }
+    // request server: the stream on which arrays of surveys created on this context are allocated and
+    // freed, as cudaMalloc and cudaFree wait for the sweeps of every other stream
+    cudaStream_t resident_stream = nullptr;
     bool tuning = false;                        // record phase times for the schedule autotuner
 };
 
 struct pfast_survey3d {
+    cudaStream_t astream = nullptr;   // arrays allocated on this stream (pfast_ctx::resident_stream)
     pfast_ctx* ctx = nullptr;
     int nz = 0, nr = 0, nc = 0;
     double dx = 0, dy = 0, dz = 0;
@@ -101,6 +110,7 @@ struct pfast_survey3d {
 };
 
 struct pfast_survey2d {
+    cudaStream_t astream = nullptr;   // arrays allocated on this stream (pfast_ctx::resident_stream)
     pfast_ctx* ctx = nullptr;
     int nr = 0, nc = 0;
     double dx = 0, dz = 0;

@@ -915,10 +915,14 @@ pfast_status pfast_survey2d_create(pfast_ctx* ctx, int nrows, int ncols, double 
         }
     }
     auto up = [&](void** dst, const void* h, size_t bytes) -> pfast_status {
-        PFAST_CUDA_TRY(cudaMalloc(dst, std::max<size_t>(bytes, 16)));
-        if (bytes && h) PFAST_CUDA_TRY(cudaMemcpy(*dst, h, bytes, cudaMemcpyHostToDevice));
+        if (sv->astream) PFAST_CUDA_TRY(cudaMallocAsync(dst, std::max<size_t>(bytes, 16), sv->astream));
+        else PFAST_CUDA_TRY(cudaMalloc(dst, std::max<size_t>(bytes, 16)));
+        if (!(bytes && h)) return PFAST_OK;
+        if (sv->astream) PFAST_CUDA_TRY(cudaMemcpyAsync(*dst, h, bytes, cudaMemcpyHostToDevice, sv->astream));
+        else PFAST_CUDA_TRY(cudaMemcpy(*dst, h, bytes, cudaMemcpyHostToDevice));
         return PFAST_OK;
     };
+    sv->astream = ctx->resident_stream;
     pfast_status r = PFAST_OK;
     if (!r) r = up((void**)&sv->d_src_ij, src, sizeof(int) * 2 * nsrc);
     if (!r) r = up((void**)&sv->d_ch0, sv->h_ch0.data(), sizeof(int) * (nsrc + 1));
@@ -932,6 +936,11 @@ pfast_status pfast_survey2d_create(pfast_ctx* ctx, int nrows, int ncols, double 
     if (!r) r = up((void**)&sv->d_last_r, last_r.data(), last_r.size());
     if (!r) r = up((void**)&sv->d_Z, (NumofR && Z) ? Z : nullptr, (NumofR && Z) ? sizeof(double) * 3 * (size_t)NumofR * ncols : 0);
     if (!r) r = up((void**)&sv->d_k2vec, tab.data(), sizeof(int) * tab.size());
+    // the host tables above are freed when this function returns
+    if (!r && sv->astream) {
+        const cudaError_t e = cudaStreamSynchronize(sv->astream);
+        if (e != cudaSuccess) r = cuda_fail(e, "survey upload", __FILE__, __LINE__);
+    }
     if (r) { pfast_survey2d_destroy(sv); return r; }
     *out = sv;
     return PFAST_OK;
@@ -942,7 +951,8 @@ pfast_status pfast_survey2d_destroy(pfast_survey2d* sv) {
     for (void* p : {(void*)sv->d_src_ij, (void*)sv->d_ch0, (void*)sv->d_srnum, (void*)sv->d_rec, (void*)sv->d_nxy,
                     (void*)sv->d_ttobs, (void*)sv->d_trobs, (void*)sv->d_last_t, (void*)sv->d_last_r, (void*)sv->d_Z,
                     (void*)sv->d_k2vec})
-        if (p) cudaFree(p);
+        if (p && sv->astream) cudaFreeAsync(p, sv->astream);
+        else if (p) cudaFree(p);
     delete sv;
     return PFAST_OK;
 }

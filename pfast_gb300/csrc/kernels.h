@@ -87,7 +87,8 @@ struct DataflowShape {
     int warps = 0, cluster = 1, blocks = 0, form = 0;
     size_t smem = 0;
 };
-pfast_status dataflow_shape(int kind, int shape, int ntiles, int nact, DataflowShape* out, bool multi = false);
+// load: instances that want SMs at the same time, those of other streams included (>= nact).
+pfast_status dataflow_shape(int kind, int shape, int ntiles, int nact, int load, DataflowShape* out, bool multi = false);
 // Dataflow sweep kernel (one launch per phase): blocks or clusters take the
 // nact instances of a.act from queue[0] (zeroed by the caller) and solve each to convergence
 // (maxiter outer iterations at most); result[inst] = iterations | 1<<30 if not converged
@@ -98,7 +99,7 @@ pfast_status launch_sweep3_dataflow(int kind, const Sweep3Args& a, int nact, int
 // The dataflow kernel over instances of several grids: item q is instance items[q].y of the grid
 // whose arguments are models[items[q].x] (a device array; each model's result goes to its own
 // `changed` array); max_ntiles: the largest grid's tile count (<= kDataflowMaxTiles); ds
-// from dataflow_shape(kind, shape, max_ntiles, nitems, &ds, true).
+// from dataflow_shape(kind, shape, max_ntiles, nitems, load, &ds, true).
 pfast_status launch_sweep3_dataflow_multi(int kind, int shape, const Sweep3Args* models, const int2* items, int nitems,
                                           int max_ntiles, int maxiter, int* queue, const DataflowShape& ds,
                                           cudaStream_t st);
@@ -112,7 +113,7 @@ struct ShapeLaunchers {
                                  const DataflowShape& ds, cudaStream_t st);
     static pfast_status dataflow_multi(int kind, const Sweep3Args* models, const int2* items, int nitems,
                                        int max_ntiles, int maxiter, int* queue, const DataflowShape& ds, cudaStream_t st);
-    static pfast_status dataflow_shape(int kind, int ntiles, int nact, bool multi, DataflowShape* out);
+    static pfast_status dataflow_shape(int kind, int ntiles, int nact, int load, bool multi, DataflowShape* out);
     static pfast_status seed(int kind, const Sweep3Args& a, int nact, cudaStream_t st);
     static pfast_status orders(int kind, const Sweep3Args& a, int nact, cudaStream_t st);
 };

@@ -3,8 +3,9 @@
 //
 // Same scheme as the 3D kernels: the 4 sweep orders of the reference
 // (src/RT_pfsm2d.h:168-181, src/RT_padjoint2d.h:351-369) are run as wavefronts of
-// T2I x T2J tiles (one launch per tile anti-diagonal); inside a tile lane = row,
-// and step t updates the node anti-diagonal li + lj = t.  Upstream neighbours are
+// T2I x T2J tiles, with one launch per phase in which a warp streams along each strip of
+// T2I rows (up to 512 rows; taller grids take one launch per tile anti-diagonal); lane =
+// row, and step t updates the node anti-diagonal li + lj = t.  Upstream neighbours are
 // final and downstream ones untouched when a node is updated, exactly as in the
 // reference's lexicographic loop, so the plain FP64 flavour is bit-identical.
 

@@ -113,10 +113,10 @@ pfast_status launch_sweep3_dataflow_multi(int kind, int shape, const Sweep3Args*
                  : ShapeLaunchers<Shape48>::dataflow_multi(kind, models, items, nitems, max_ntiles, maxiter, queue, ds, st);
 }
 
-pfast_status dataflow_shape(int kind, int shape, int ntiles, int nact, DataflowShape* out, bool multi) {
+pfast_status dataflow_shape(int kind, int shape, int ntiles, int nact, int load, DataflowShape* out, bool multi) {
     if (!known_shape(shape)) return PFAST_ERR_INVALID;
-    return shape ? ShapeLaunchers<Shape84>::dataflow_shape(kind, ntiles, nact, multi, out)
-                 : ShapeLaunchers<Shape48>::dataflow_shape(kind, ntiles, nact, multi, out);
+    return shape ? ShapeLaunchers<Shape84>::dataflow_shape(kind, ntiles, nact, load, multi, out)
+                 : ShapeLaunchers<Shape48>::dataflow_shape(kind, ntiles, nact, load, multi, out);
 }
 
 pfast_status launch_seed_tiles3(int kind, const Sweep3Args& a, int nact, cudaStream_t st) {

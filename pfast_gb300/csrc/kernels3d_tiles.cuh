@@ -58,15 +58,18 @@ template <> struct Traits<kAdjPolish64>  { using Real = double; using Aux = doub
 //                 ahead); the upstream lanes' new values and the downstream lanes' old values come by
 //                 warp shuffle, the face halo pencils from owner lanes, and each changed node is stored
 //                 as it is updated.  The warp then needs no shared memory, so a block holds 24 (forward)
-//                 or 16 (adjoint) warps instead of 11, but a step takes 355 / 442 instructions instead
-//                 of 247 / 400 (ncu, warp instructions per tile and step).  For the forward with one
-//                 block per source on large grids, whose many ready tiles keep 24 warps busy (256 sources
-//                 of 256 x 256 x 128, 8192 tiles: 307 ms against 332 with boxes; 300 sources of 128 x 128 x 64,
-//                 1024 tiles: 50.5 against 43.1), for the adjoint also up to two blocks per source.
-//   kFormBoxes    (adjoint polish in clusters of four blocks or more) field and traveltime in boxes.
+//                 or 16 (adjoint) warps instead of 11, at more instructions a step (ncu, first
+//                 version: 355 / 442 warp instructions per tile and step against 247 / 400).  For the
+//                 forward with one block per source on large grids, whose many ready tiles keep 24 warps
+//                 busy (256 sources of 256 x 256 x 128, 8192 tiles: 303 ms against 317 with boxes; 152
+//                 sources of 128 x 128 x 100, 1600 tiles: 35.1 against 30.9); for the adjoint with one
+//                 block per source (the 256 sources: 243 against 292 with a field box) or up to three on
+//                 grids of 1024 tiles or more.
+//   kFormBoxes    (adjoint polish in clusters otherwise) field and traveltime in boxes.
 // Elsewhere the latency of a tile bounds the polish, and the boxes are ahead: forward polish of 24
 // sources of 155 x 75 x 101 nodes 32.3 -> 25.3 ms, 64 of 128 x 128 x 64 26.9 -> 21.9, 9 of 90 x 71 x 53
-// 13.9 -> 9.9; adjoint polish of the 9 sources 14.5 -> 11.6 (of the 64: 27.9 -> 30.9, not taken).
+// 13.9 -> 9.9; adjoint polish of the 9 sources 14.5 -> 11.6, 42 of 96 x 96 x 48 (432 tiles, 3 blocks)
+// 12.1 -> 9.7, but 55 of 128 x 128 x 100 (1600 tiles, 2 blocks) 28.0 -> 32.2.
 constexpr int kFormBox = 0, kFormWindows = 1, kFormBoxes = 2;
 
 template <int KIND, int FORM>
@@ -1792,7 +1795,7 @@ pfast_status launch_one(const Sweep3Args& a, int d0, int tiles, int nact, cudaSt
 template <int KIND>
 constexpr int dataflow_form(int cluster, int ntiles) {
     if (KIND == kFwdPolish64) return cluster == 1 && ntiles >= 4096 ? kFormWindows : kFormBox;
-    if (KIND == kAdjPolish64) return cluster >= 4 ? kFormBoxes : kFormWindows;
+    if (KIND == kAdjPolish64) return cluster >= 4 || (cluster > 1 && ntiles < 1024) ? kFormBoxes : kFormWindows;
     return kFormBox;
 }
 
@@ -1833,14 +1836,14 @@ DataflowKernel dataflow_kernel(bool multi, bool cluster, int form) {
 }
 
 template <int KIND, class SH>
-pfast_status dataflow_shape_k(int ntiles, int nact, bool multi, DataflowShape* out) {
-    static std::map<std::tuple<int, int, int, bool>, DataflowShape> cache;   // (device, ntiles, nact, multi)
+pfast_status dataflow_shape_k(int ntiles, int nact, int load, bool multi, DataflowShape* out) {
+    static std::map<std::tuple<int, int, int, int, bool>, DataflowShape> cache;   // (device, ntiles, nact, load, multi)
     static std::mutex mu;
     int dev = 0, sms = 0, smem_max = 0;
     PFAST_CUDA_TRY(cudaGetDevice(&dev));
     {
         std::lock_guard<std::mutex> lk(mu);
-        auto it = cache.find(std::make_tuple(dev, ntiles, nact, multi));
+        auto it = cache.find(std::make_tuple(dev, ntiles, nact, load, multi));
         if (it != cache.end()) {
             *out = it->second;
             return PFAST_OK;
@@ -1852,7 +1855,7 @@ pfast_status dataflow_shape_k(int ntiles, int nact, bool multi, DataflowShape* o
     *out = DataflowShape();
     // the largest cluster size at which every instance has a cluster of its own at the same time
     for (int cs = kMaxCluster; cs >= 1 && !out->warps; --cs) {
-        if (cs > 1 && !cluster_wanted(cs, kPlain, nact, ntiles, sms)) continue;
+        if (cs > 1 && !cluster_wanted(cs, kPlain, load, ntiles, sms)) continue;
         const int form = dataflow_form<KIND>(cs, ntiles);
         const DataflowKernel k = dataflow_kernel<KIND, SH>(multi, cs > 1, form);
         if (ntiles > kDataflowMaxTiles) return PFAST_OK;
@@ -1887,7 +1890,7 @@ pfast_status dataflow_shape_k(int ntiles, int nact, bool multi, DataflowShape* o
                 cudaGetLastError();   // not available at this size: not used
                 continue;
             }
-            if (resident < nact) continue;
+            if (resident < load) continue;
         } else {
             int per_sm = 0;
             PFAST_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k.fn, w * 32, smem));
@@ -1900,7 +1903,7 @@ pfast_status dataflow_shape_k(int ntiles, int nact, bool multi, DataflowShape* o
         out->smem = smem;
     }
     std::lock_guard<std::mutex> lk(mu);
-    cache[std::make_tuple(dev, ntiles, nact, multi)] = *out;
+    cache[std::make_tuple(dev, ntiles, nact, load, multi)] = *out;
     return PFAST_OK;
 }
 
@@ -1964,8 +1967,8 @@ pfast_status ShapeLaunchers<SH>::dataflow_multi(int kind, const Sweep3Args* mode
 }
 
 template <class SH>
-pfast_status ShapeLaunchers<SH>::dataflow_shape(int kind, int ntiles, int nact, bool multi, DataflowShape* out) {
-    PFAST_KIND_SWITCH(kind, (dataflow_shape_k<K, SH>(ntiles, nact, multi, out)));
+pfast_status ShapeLaunchers<SH>::dataflow_shape(int kind, int ntiles, int nact, int load, bool multi, DataflowShape* out) {
+    PFAST_KIND_SWITCH(kind, (dataflow_shape_k<K, SH>(ntiles, nact, load, multi, out)));
 }
 
 template <class SH>

@@ -38,6 +38,7 @@ struct Model {
     double dx = 0, dy = 0, dz = 0;
     double* d_vp = nullptr;
     double* d_wr = nullptr;
+    cudaStream_t astream = nullptr;   // of the arrays
     size_t bytes = 0;
     int refs = 0;
     bool dropped = false;
@@ -69,8 +70,8 @@ struct Job {
 };
 
 void free_model(Model& m) {
-    if (m.d_vp) cudaFree(m.d_vp);
-    if (m.d_wr) cudaFree(m.d_wr);
+    if (m.d_vp) cudaFreeAsync(m.d_vp, m.astream);
+    if (m.d_wr) cudaFreeAsync(m.d_wr, m.astream);
     m.d_vp = m.d_wr = nullptr;
 }
 
@@ -89,6 +90,7 @@ struct pfast_server {
     std::condition_variable cv_work, cv_done;
     std::unique_ptr<serve::Policy> policy;
     std::vector<pfast_ctx*> ctxs;
+    std::atomic<int> running{0};   // policy->running(), read by the contexts without the lock
     std::vector<std::thread> workers;
     pfast_ctx* admin = nullptr;   // context for registration copies
     std::map<long long, std::shared_ptr<Model>> models;
@@ -211,6 +213,7 @@ void worker_main(pfast_server* srv, int slot) {
         job->batch = d.batch;
         job->bytes = d.bytes;
         job->t_start = Clock::now();
+        srv->running = srv->policy->running();
         srv->peak = std::max(srv->peak, srv->policy->used());
         lk.unlock();
         pfast_status st = run_job(ctx, *job);
@@ -223,6 +226,7 @@ void worker_main(pfast_server* srv, int slot) {
         job->message = msg;
         job->done = true;
         srv->policy->finish(job->bytes);
+        srv->running = srv->policy->running();
         srv->completed += 1;
         if (st != PFAST_OK) srv->failed += 1;
         job->model->refs -= 1;
@@ -271,11 +275,13 @@ pfast_status pfast_server_create(const pfast_server_config* cfg, pfast_server** 
     srv->policy.reset(new serve::Policy((size_t)cfg->hbm_budget_bytes, cfg->slots,
                                         cfg->max_bypass > 0 ? cfg->max_bypass : 8));
     pfast_status s = pfast_ctx_create(cfg->device, &srv->admin);
+    if (s == PFAST_OK) srv->admin->resident_stream = srv->admin->own_stream;
     for (int k = 0; s == PFAST_OK && k < cfg->slots; ++k) {
         pfast_ctx* c = nullptr;
         s = pfast_ctx_create(cfg->device, &c);
         if (s == PFAST_OK) {
             ctx_stream_ordered(c);
+            c->running = &srv->running;
             srv->ctxs.push_back(c);
         }
     }
@@ -332,10 +338,12 @@ pfast_status pfast_server_put_model(pfast_server* srv, long long model_id, int d
         }
     }
     PFAST_CUDA_TRY(cudaSetDevice(srv->cfg.device));
-    cudaError_t e = cudaMalloc(&m->d_vp, N * 8);
-    if (e == cudaSuccess && WR) e = cudaMalloc(&m->d_wr, N * 8);
-    if (e == cudaSuccess) e = cudaMemcpy(m->d_vp, vp, N * 8, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && WR) e = cudaMemcpy(m->d_wr, WR, N * 8, cudaMemcpyHostToDevice);
+    m->astream = srv->admin->own_stream;
+    cudaError_t e = cudaMallocAsync(&m->d_vp, N * 8, m->astream);
+    if (e == cudaSuccess && WR) e = cudaMallocAsync(&m->d_wr, N * 8, m->astream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(m->d_vp, vp, N * 8, cudaMemcpyHostToDevice, m->astream);
+    if (e == cudaSuccess && WR) e = cudaMemcpyAsync(m->d_wr, WR, N * 8, cudaMemcpyHostToDevice, m->astream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(m->astream);
     std::lock_guard<std::mutex> g(srv->mu);
     if (e != cudaSuccess) {
         free_model(*m);

@@ -35,7 +35,7 @@ inline unsigned tune_allowed(int schedule_opt, int shape_opt, const bool dataflo
 // The candidate of a phase: once every allowed candidate has been timed (e non-null), the one
 // with the smallest mean phase time (the first of equal ones); before that, the dataflow kernel
 // with 4x8x32 tiles from two active instances per SM, else one launch per tile diagonal
-// (falling back to the lowest allowed candidate).
+// (falling back to the lowest allowed candidate).  The sweeps ask untuned_pick below until then.
 inline int tune_pick(const TuneEntry* e, unsigned allowed, int nact, int sms) {
     if (e) {
         int best = -1;
