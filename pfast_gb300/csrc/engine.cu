@@ -263,7 +263,7 @@ pfast_status run_sweeps3(pfast_ctx* ctx, Sweep3Args a, int kind, int nb, std::ve
     PFAST_CUDA_TRY(cudaGetDevice(&dev));
     PFAST_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const auto tkey = std::make_tuple(dev, kind, a.nz, a.nr, a.nc, (int)active.size());
-    const int load = (int)active.size() * ctx->share();
+    const int load = (int)active.size() * SweepScope::count(dev);
     DataflowShape dshape[kTileShapes];
     bool fits[kTileShapes] = {};
     for (int shape = 0; shape < kTileShapes; ++shape) {
@@ -995,6 +995,7 @@ static pfast_status survey3d_run(pfast_ctx* ctx, pfast_survey3d* sv, const doubl
     pfast_options o = resolve_impl(opt, 100);
     ctx->polish_floor = o.polish_floor > 0.0 ? (float)o.polish_floor : kPolishFloor;
     ctx->schedule = o.schedule;
+    const SweepScope scope(ctx->device);
     ctx->tile_shape = o.tile_shape;
     ctx->near_radius = o.near_source_radius;
     stats_begin_impl(stats);
@@ -1158,6 +1159,7 @@ pfast_status pfast_fsm3d(double* vp, double* U, int* src, int srcid, int MAXSwp,
     }
     if (!r) r = prepare_slowness(ctx, ctx->vp_tmp.as<double>(), N, false);
     ctx->schedule = PFAST_SCHEDULE_AUTO;
+    const SweepScope scope(ctx->device);
     ctx->near_radius = 0;
     if (!r) r = forward3d_batch(ctx, sv, 0, 1, PFAST_PLAIN_FP64, MAXSwp, nullptr);
     if (!r) {
@@ -1193,6 +1195,7 @@ pfast_status pfast_adjoint_fsm3d(double* U, double* T, double* T_obs, int* rec, 
     }
     double ee = 0.0;
     ctx->schedule = PFAST_SCHEDULE_AUTO;
+    const SweepScope scope(ctx->device);
     if (!r) r = adjoint3d_batch(ctx, sv, 0, 1, PFAST_PLAIN_FP64, MAXSwp, &ee, nullptr);
     if (!r) {
         cudaError_t e = cudaMemcpyAsync(U, ctx->L64.p, sizeof(double) * N, cudaMemcpyDeviceToHost, s);

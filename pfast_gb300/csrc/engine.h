@@ -81,13 +81,29 @@ struct pfast_ctx {
     int tile_shape = PFAST_TILE_AUTO;           // of the current 3D evaluation (pfast_options)
     int candidates = 0;                         // per sweep kind: 1 + candidate of its last phase (pfast_stats)
     int near_radius = 0;                        // of the current 3D evaluation (pfast_options)
-    // request server: requests that run at the same time (read at the start of each sweep phase)
-    const std::atomic<int>* running = nullptr;
-    int share() const { return running ? std::max(1, running->load(std::memory_order_relaxed)) : 1; }
     // request server: the stream on which arrays of surveys created on this context are allocated and
     // freed, as cudaMalloc and cudaFree wait for the sweeps of every other stream
     cudaStream_t resident_stream = nullptr;
     bool tuning = false;                        // record phase times for the schedule autotuner
+};
+
+// A 3D evaluation or solve of this process under way on a device, in whatever thread and context.
+// Phases that run side by side share the SMs, so none spreads its sources over all of them (48
+// uneven models through a request server's 8 slots: 2.10 s when each did, 1.70 s; mixed gradients
+// of 12 sources of 96 x 96 x 48 nodes, 12 in each of 8 threads: 1067 ms and 611).
+struct SweepScope {
+    std::atomic<int>& n;
+    explicit SweepScope(int device) : n(running(device)) { ++n; }
+    ~SweepScope() { --n; }
+    SweepScope(const SweepScope&) = delete;
+    SweepScope& operator=(const SweepScope&) = delete;
+    static int count(int device) { return std::max(1, running(device).load(std::memory_order_relaxed)); }
+
+private:
+    static std::atomic<int>& running(int device) {
+        static std::atomic<int> counts[64];
+        return counts[std::min(std::max(device, 0), 63)];
+    }
 };
 
 struct pfast_survey3d {

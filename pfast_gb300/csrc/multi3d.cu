@@ -124,7 +124,7 @@ pfast_status multi_phase(pfast_ctx* ctx, std::vector<Model>& ms, std::vector<Swe
         PFAST_CUDA_TRY(cudaMemcpyAsync(d_args, args.data(), sizeof(Sweep3Args) * nm, cudaMemcpyHostToDevice, st));
         PFAST_CUDA_TRY(cudaMemcpyAsync(d_items, items.data(), sizeof(int2) * nitems, cudaMemcpyHostToDevice, st));
         DataflowShape ds;
-        PFAST_TRY(dataflow_shape(kind, 0, max_ntiles, nitems, nitems * ctx->share(), &ds, true));
+        PFAST_TRY(dataflow_shape(kind, 0, max_ntiles, nitems, nitems * SweepScope::count(ctx->device), &ds, true));
         if (ds.warps <= 0) {
             set_last_error("multi-model evaluation: a grid of %d tiles does not fit the dataflow kernel", max_ntiles);
             return PFAST_ERR_INVALID;
@@ -178,6 +178,7 @@ pfast_status multi_phase(pfast_ctx* ctx, std::vector<Model>& ms, std::vector<Swe
 
 // The evaluation of one group of models that fits in device memory at once.
 pfast_status eval_group(pfast_ctx* ctx, std::vector<Model>& ms, const pfast_options& o, pfast_stats* stats) {
+    const SweepScope scope(ctx->device);
     cudaStream_t st = ctx->stream;
     const bool mixed = o.precision == PFAST_MIXED;
     const int nm = (int)ms.size();

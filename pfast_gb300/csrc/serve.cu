@@ -90,7 +90,6 @@ struct pfast_server {
     std::condition_variable cv_work, cv_done;
     std::unique_ptr<serve::Policy> policy;
     std::vector<pfast_ctx*> ctxs;
-    std::atomic<int> running{0};   // policy->running(), read by the contexts without the lock
     std::vector<std::thread> workers;
     pfast_ctx* admin = nullptr;   // context for registration copies
     std::map<long long, std::shared_ptr<Model>> models;
@@ -213,7 +212,6 @@ void worker_main(pfast_server* srv, int slot) {
         job->batch = d.batch;
         job->bytes = d.bytes;
         job->t_start = Clock::now();
-        srv->running = srv->policy->running();
         srv->peak = std::max(srv->peak, srv->policy->used());
         lk.unlock();
         pfast_status st = run_job(ctx, *job);
@@ -226,7 +224,6 @@ void worker_main(pfast_server* srv, int slot) {
         job->message = msg;
         job->done = true;
         srv->policy->finish(job->bytes);
-        srv->running = srv->policy->running();
         srv->completed += 1;
         if (st != PFAST_OK) srv->failed += 1;
         job->model->refs -= 1;
@@ -281,7 +278,6 @@ pfast_status pfast_server_create(const pfast_server_config* cfg, pfast_server** 
         s = pfast_ctx_create(cfg->device, &c);
         if (s == PFAST_OK) {
             ctx_stream_ordered(c);
-            c->running = &srv->running;
             srv->ctxs.push_back(c);
         }
     }
