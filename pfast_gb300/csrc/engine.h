@@ -90,7 +90,7 @@ struct pfast_ctx {
 // A 3D evaluation or solve of this process under way on a device, in whatever thread and context.
 // Phases that run side by side share the SMs, so none spreads its sources over all of them (48
 // uneven models through a request server's 8 slots: 2.10 s when each did, 1.70 s; mixed gradients
-// of 12 sources of 96 x 96 x 48 nodes, 12 in each of 8 threads: 1067 ms and 611).
+// of 12 sources of 96 x 96 x 48 nodes, 12 in each of 8 threads: 1067 ms and 650).
 struct SweepScope {
     std::atomic<int>& n;
     explicit SweepScope(int device) : n(running(device)) { ++n; }
