@@ -233,6 +233,10 @@ inline ExactGrid3 exact_grid3(const double d[3]) {
 
 // |v| in [2^-34, 2^34]: traveltimes for which every quotient above stays in its range
 PFAST_HD bool in_range(double v) { return (unsigned)(exponent_of(v) - 989) <= 67u; }
+// Slownesses below 2^34 as well: the terms with s*s enter the same sums, and where they overflow (from
+// about 2^450 on, velocities below 1e-136 of an impermeable body) the one-step quotient of an infinite
+// numerator is NaN, where x / d is infinite and the minimum with the node's value drops it.
+PFAST_HD bool slow_in_range(double s) { return exponent_of(s) <= 1056; }
 
 // Magnitude of a value >= +0 as FP32 (truncated; +inf and beyond give a huge finite value).
 PFAST_HD float approx32(double v) {
@@ -286,7 +290,7 @@ PFAST_HD double eik3_exact(double x, double y, double z, double s, const ExactGr
     if (bits_of(q) <= bits_of(b)) return q;
     const double db = pick(kb, g.axis[0].d, g.axis[1].d, g.axis[2].d);
     const bool ainf = bits_of(a) >= 0x7ff0000000000000ll;
-    if (!(in_range(b) && (is_zero(c) || in_range(c)) && (ainf || in_range(a)))) {
+    if (!(in_range(b) && (is_zero(c) || in_range(c)) && (ainf || in_range(a)) && slow_in_range(s))) {
         const double da = pick(ka, g.axis[0].d, g.axis[1].d, g.axis[2].d);
         return eik3_tail_ref(a, b, c, da, db, dc, pick(ka, inv2[0], inv2[1], inv2[2]),
                              pick(kb, inv2[0], inv2[1], inv2[2]), pick(kc, inv2[0], inv2[1], inv2[2]), s);
@@ -405,7 +409,7 @@ PFAST_HD double eik2_exact(double x, double z, double s, const ExactGrid2& g) {
     const double q = lo + dlo * s;
     if (bits_of(q) <= bits_of(hi)) return q;
     double S, C;
-    if (in_range(hi) && (is_zero(lo) || in_range(lo))) {
+    if (in_range(hi) && (is_zero(lo) || in_range(lo)) && slow_in_range(s)) {
         auto dv = [](double v, const DivBy& k) {   // one of the two may be 0 beside the source
             const double r = div_exact<FAST>(v, k);
             return is_zero(v) ? v : r;

@@ -1,0 +1,86 @@
+// The plain FP64 updates of exact_arith.h against the reference's expressions, bit for bit (NaN for
+// NaN), on arguments far outside those of a survey: slownesses from 0 over the whole exponent range
+// to infinity.  Prints "ok <name> <cases>" or "FAIL ..." lines.
+#include <algorithm>
+#include <cstdio>
+#include <random>
+
+#include "exact_arith.h"
+
+using namespace pfast;
+
+static std::mt19937_64 rng(977);
+static double uni(double a, double b) { return std::uniform_real_distribution<double>(a, b)(rng); }
+static bool same(double a, double b) { return bits_of(a) == bits_of(b) || (std::isnan(a) && std::isnan(b)); }
+
+static double eik3_ref(double a, double b, double c, double s, const double* d) {
+    double da = d[0], db = d[1], dc = d[2], t;
+    if (b > a) { t = a; a = b; b = t; t = da; da = db; db = t; }
+    if (c > a) { t = a; a = c; c = t; t = da; da = dc; dc = t; }
+    if (c > b) { t = b; b = c; c = t; t = db; db = dc; dc = t; }
+    double q = dc * s + c;
+    if (q <= b) return q;
+    double A = dc * dc + db * db, B = -2. * (b * dc * dc + c * db * db);
+    double C = dc * dc * b * b + db * db * c * c - db * db * dc * dc * s * s;
+    double D = B * B - 4. * A * C;
+    q = (D >= 0) ? (-B + std::sqrt(D)) / 2. / A : kUnreached;
+    if (q <= a) return q;
+    A = 1.0 / da / da + 1.0 / db / db + 1.0 / dc / dc;
+    B = -2.0 * (a / da / da + b / db / db + c / dc / dc);
+    C = a * a / da / da + b * b / db / db + c * c / dc / dc - s * s;
+    D = B * B - 4. * A * C;
+    return (D >= 0) ? (-B + std::sqrt(D)) / 2. / A : kUnreached;
+}
+static double eik2_ref(double a, double b, double s, double dx, double dz) {
+    double da = dx, db = dz, t;
+    if (b > a) { t = a; a = b; b = t; t = da; da = db; db = t; }
+    double q = b + db * s;
+    if (q <= a) return q;
+    const double A = 1.0 / da / da + 1.0 / db / db, B = -2. * (a / da / da + b / db / db);
+    const double C = a * a / da / da + b * b / db / db - s * s, D = B * B - 4 * A * C;
+    return (D >= 0) ? (-B + std::sqrt(D)) / 2. / A : kUnreached;
+}
+
+static int bad = 0;
+static void report(const char* name, long long n, long long wrong) {
+    std::printf("%s %s %lld\n", wrong ? "FAIL" : "ok", name, wrong ? wrong : n);
+    bad += wrong != 0;
+}
+
+int main() {
+    const double spacings[] = {20.0, 5.0, 12.5, 16.7, 8.3, 0.1, 1.0 / 3.0, 1.0, 4096.0, 3e-6, 7.3e5};
+    {   // neighbour minima of a solve (0 at the source, up to the unreached value, infinite at the grid's faces)
+        long long n3 = 0, w3 = 0, n2 = 0, w2 = 0;
+        for (int dec = -324; dec <= 310; ++dec)
+            for (int i = 0; i < 4000; ++i) {
+                double s = std::pow(10.0, dec + uni(0.0, 1.0));   // 0 below the range, infinite above it
+                double d[3];
+                const double h = spacings[rng() % 11];
+                for (double& v : d) v = i % 2 ? spacings[rng() % 11] : h;
+                const double base = rng() % 3 ? std::pow(10.0, uni(-9.0, 7.0)) : 0.0;
+                double v[3];
+                for (double& x : v) {
+                    x = std::min(kUnreached, base * (1.0 + uni(0.0, 1.0) * (rng() % 2 ? 1e-3 : 1.0)));
+                    const unsigned c = rng() % 24;
+                    if (c == 0) x = 0.0;
+                    if (c == 1) x = kUnreached;
+                    if (c == 2) x = INFINITY;
+                }
+                const ExactGrid3 g = exact_grid3(d);
+                double inv2[3];
+                for (int a = 0; a < 3; ++a) inv2[a] = 1.0 / d[a] / d[a];
+                const double r = eik3_ref(v[0], v[1], v[2], s, d);
+                w3 += !same(r, eik3_exact<false, false>(v[0], v[1], v[2], s, g, inv2));
+                if (g.iso) w3 += !same(r, eik3_exact<true, false>(v[0], v[1], v[2], s, g, inv2));
+                if (g.iso && g.fast) w3 += !same(r, eik3_exact<true, true>(v[0], v[1], v[2], s, g, inv2));
+                ++n3;
+                const ExactGrid2 g2 = exact_grid2(d[0], d[1]);
+                const double r2 = eik2_ref(v[0], v[1], s, d[0], d[1]);
+                w2 += !same(r2, eik2_exact<false>(v[0], v[1], s, g2)) || (g2.fast && !same(r2, eik2_exact<true>(v[0], v[1], s, g2)));
+                ++n2;
+            }
+        report("eik3_slowness", n3, w3);
+        report("eik2_slowness", n2, w2);
+    }
+    return bad ? 1 : 0;
+}
