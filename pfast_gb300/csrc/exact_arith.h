@@ -361,6 +361,13 @@ PFAST_HD double sub_sparse(double p, double m) {
 PFAST_HD void adj_axis_exact(double T0, double Tp, double Tm, double Lp, double Lm, const DivBy& k, double& den,
                              double& num) {
     const double gp = div_mid(-(Tp - T0), k), gm = div_mid(-(T0 - Tm), k);
+    if (exponent_of(gp) >= 0x7fe || exponent_of(gm) >= 0x7fe) {
+        // x + |x| overflows, is NaN for -inf (x - |x| for +inf), and a NaN has no sign to go by
+        const double p = here(gp), m = here(gm);
+        den = ((p + fabs(p)) / 2.0 - (m - fabs(m)) / 2.0) / k.d;
+        num = ((m + fabs(m)) / 2.0 * Lm - (p - fabs(p)) / 2.0 * Lp) / k.d;
+        return;
+    }
     const double pp = pos_part(gp), nm = neg_part(gm), pm = pos_part(gm), np = neg_part(gp);
     den = div_mid(sub_sparse(pp, nm), k);
     // pm * Lm - np * Lp

@@ -1,6 +1,6 @@
 // The plain FP64 updates of exact_arith.h against the reference's expressions, bit for bit (NaN for
 // NaN), on arguments far outside those of a survey: slownesses from 0 over the whole exponent range
-// to infinity.  Prints "ok <name> <cases>" or "FAIL ..." lines.
+// to infinity; traveltimes of a caller's field that are NaN, infinite or huge.  Prints "ok <name> <cases>" or "FAIL ..." lines.
 #include <algorithm>
 #include <cstdio>
 #include <random>
@@ -39,6 +39,13 @@ static double eik2_ref(double a, double b, double s, double dx, double dz) {
     const double A = 1.0 / da / da + 1.0 / db / db, B = -2. * (a / da / da + b / db / db);
     const double C = a * a / da / da + b * b / db / db - s * s, D = B * B - 4 * A * C;
     return (D >= 0) ? (-B + std::sqrt(D)) / 2. / A : kUnreached;
+}
+static double posr(double x) { return (x + std::fabs(x)) / 2.0; }
+static double negr(double x) { return (x - std::fabs(x)) / 2.0; }
+static void axis_ref(double T0, double Tp, double Tm, double Lp, double Lm, double d, double& den, double& num) {
+    const double gp = -(Tp - T0) / d, gm = -(T0 - Tm) / d;
+    den = (posr(gp) - negr(gm)) / d;
+    num = (posr(gm) * Lm - negr(gp) * Lp) / d;
 }
 
 static int bad = 0;
@@ -81,6 +88,27 @@ int main() {
             }
         report("eik3_slowness", n3, w3);
         report("eik2_slowness", n2, w2);
+    }
+    {   // adjoint terms of one axis
+        const double nan = std::nan("");
+        const double Ts[] = {nan, -nan, -(double)INFINITY, -1.7e308, -1e308, -1e300, -2e100, -0.4, -0.0, 0.0, 0.3, 9e6};
+        long long n = 0, wrong = 0;
+        for (double d : spacings) {
+            const DivBy k = div_by(d);
+            for (double T0 : Ts) for (double Tp : Ts) for (double Tm : Ts)
+                for (int i = 0; i < 40; ++i) {
+                    auto L = [&]() -> double {
+                        const unsigned c = rng() % 10;
+                        return c == 0 ? 0.0 : c == 1 ? -0.0 : c == 2 ? INFINITY : c == 3 ? 1e308 : uni(-3.0, 3.0);
+                    };
+                    const double Lp = L(), Lm = L();
+                    double dr, nr, de, ne;
+                    axis_ref(T0, Tp, Tm, Lp, Lm, d, dr, nr);
+                    adj_axis_exact(T0, Tp, Tm, Lp, Lm, k, de, ne);
+                    wrong += !same(dr, de) || !same(nr, ne), ++n;
+                }
+        }
+        report("adj_axis_any_time", n, wrong);
     }
     return bad ? 1 : 0;
 }

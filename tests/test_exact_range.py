@@ -1,7 +1,8 @@
 """The plain FP64 updates (pfast_gb300/csrc/exact_arith.h) outside the range of a survey's values: on the
 CPU against the reference's expressions (tests/native/exact_range_check.cpp), and whole solves on the
-GPU against the oracle, bit for bit, around bodies of almost no velocity (any positive finite
-velocity is accepted)."""
+GPU against the oracle, bit for bit (NaN for NaN): forward around bodies of almost no velocity (any
+positive finite velocity is accepted), adjoint on fields with traveltimes that are no numbers,
+infinite or huge (a caller's field is taken as it is)."""
 import os
 import shutil
 import subprocess
@@ -26,7 +27,7 @@ def check_lines(tmp_path_factory):
     return subprocess.run([exe], capture_output=True, text=True, timeout=300).stdout.splitlines()
 
 
-@pytest.mark.parametrize("name", ["eik3_slowness", "eik2_slowness"])
+@pytest.mark.parametrize("name", ["eik3_slowness", "eik2_slowness", "adj_axis_any_time"])
 def test_updates_match_the_expressions(check_lines, name):
     line = [x for x in check_lines if x.split()[1] == name]
     assert line and line[0].startswith("ok "), check_lines
@@ -64,3 +65,40 @@ def test_solves_around_impermeable_bodies(v0):
         assert bits_equal(Tr.cpu().numpy(), Tr0)
         sv.close()
     ctx.close()
+
+
+def same_or_nan(a, b):
+    a, b = np.ascontiguousarray(a), np.ascontiguousarray(b)
+    n = np.isnan(a)
+    return np.array_equal(n, np.isnan(b)) and bits_equal(np.where(n, 0.0, a), np.where(n, 0.0, b))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("v", [np.nan, -np.nan, -np.inf, -1.7e308])
+def test_adjoints_of_fields_with_any_time(v):
+    import pfast_gb300 as pg
+    from oracle import port
+    rng = np.random.default_rng(11)
+    nz, nr, nc = 6, 13, 40
+    T = rng.uniform(0.0, 1.0, (nz, nr, nc))
+    at = rng.random(T.shape) < 0.01
+    at[0] = False                         # the receivers' plane keeps its times
+    T[0] += 1.0                           # lambda enters from the receivers
+    T[at] = v
+    assert np.signbit(T[at]).all() == np.signbit(v) and at.sum() > 10
+    src = np.array([[0, nc // 2, 0]], np.int32)
+    rec = np.array([(i, j, 0) for i in range(nr) for j in range(nc)], np.int32)
+    srnum = np.array([len(rec)], np.int32)
+    n3 = np.tile([0.3, 0.1, -0.9], (len(rec), 1))
+    tobs = T[0].ravel() + rng.normal(0.0, 0.02, len(rec))
+    for d in ((20.0, 20.0, 20.0), (16.7, 8.3, 12.5)):
+        L0, e0, _ = port.adjoint3d(T, tobs, rec, n3, src, srnum, 0, 40, *d)
+        L = np.empty(T.shape)
+        e = pg.adjoint_fsm3d(L, T, tobs, rec, n3, src, srnum, 0, 40, *d, nr, nc, nz)
+        assert same_or_nan(L, L0) and e == e0
+    T2 = np.ascontiguousarray(np.concatenate([T[0, :1], T[1], T[2], T[3]]))
+    rec, n2, tobs, srnum, src = rec[:nc, :2].copy(), n3[:nc, :2].copy(), tobs[:nc].copy(), np.array([nc], np.int32), src[:, :2].copy()
+    L0, e0, _ = port.tadjoint2d(T2, tobs, rec, n2, src, srnum, 0, 40, 20.0, 16.7)
+    L = np.empty(T2.shape)
+    e = pg.Tadjoint_fsm2d(L, T2, tobs, rec, n2, src, srnum, 0, 40, 20.0, 16.7, *T2.shape)
+    assert same_or_nan(L, L0) and e == e0
