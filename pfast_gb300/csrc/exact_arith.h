@@ -385,6 +385,14 @@ PFAST_HD void adj_axis_exact(double T0, double Tp, double Tm, double Lp, double 
     num = div_any(n, k);
 }
 
+// Whether the plain adjoint update of a node (traveltime tn, value vn) can change in any bit when its
+// neighbour of traveltime t0 goes from `old` to `nv`.  A neighbour of smaller or equal traveltime
+// enters as +0 * lambda, which changes no bit of a nonzero sum of finite terms.  A zero lambda (the
+// sign of a zero sum) counts as a dependency, and so does a neighbour that is or was not finite: 0 *
+// inf has made the sum NaN, and it stays so until the node is updated again.
+PFAST_HD bool adj_depends_exact(double t0, double tn, double vn, double old, double nv) {
+    return ordered(t0) > ordered(tn) || is_zero(vn) || exponent_of(nv) == 0x7ff || exponent_of(old) == 0x7ff;
+}
 
 // ------------------------------------------------------------------ 2D
 struct ExactGrid2 {

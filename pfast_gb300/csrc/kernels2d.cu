@@ -522,7 +522,7 @@ __global__ void __launch_bounds__(kWarps2 * 32) sweep2d_kernel(const Sweep2Args 
                         // (FP32 bulk: offsets from the tile's corner, compared as values)
                         auto dep = [&](Aux tn, int n) {
                             if constexpr (KIND == kAdjPlain64)
-                                return ordered(T0) > ordered(tn) || is_zero(box[n]) || exponent_of(r) == 0x7ff;
+                                return adj_depends_exact(T0, tn, box[n], old, r);
                             else if constexpr (sizeof(Aux) == 8) return obits2(T0) > obits2(tn);
                             else return T0 > tn;
                         };
@@ -986,7 +986,7 @@ __global__ void __launch_bounds__(kStripMax * 32) sweep2d_strips(const Sweep2Arg
                                         constexpr long long kMargin = KIND == kFwdPlain64 ? 1ll << 33 : 0;
                                         return min(obits2(old), obits2(nv)) < obits2(vn) + kMargin;
                                     } else if constexpr (KIND == kAdjPlain64) {
-                                        return (ordered(oT0) > ordered(tn)) | is_zero(vn) | (exponent_of(nv) == 0x7ff);
+                                        return adj_depends_exact(oT0, tn, vn, old, nv);
                                     } else if constexpr (sizeof(Aux) == 8) {
                                         return obits2(oT0) > obits2(tn);
                                     } else {

@@ -685,7 +685,7 @@ __device__ __forceinline__ long long obits(double x) { return __double_as_longlo
 __device__ __forceinline__ int obits(float x) { return __float_as_int(x); }
 
 // Whether the update of a neighbour (value vn, traveltime tn) can depend on a node that changed
-// to nv; lo: the smaller of the node's old and new value (ordered bits), t0: its traveltime.
+// from old to nv; lo: the smaller of the node's old and new value (ordered bits), t0: its traveltime.
 // Forward: the Godunov update and its Newton form exclude neighbours above the node's value.
 // Adjoint: lambda at a node weighs its neighbours with max(T_neighbour - T_node, 0).
 // The plain kinds skip tiles only where that leaves every bit as it is:
@@ -693,14 +693,11 @@ __device__ __forceinline__ int obits(float x) { return __float_as_int(x); }
 //   worst (its discriminant cancels), so a neighbour value more than 2^-20 relative above the
 //   node's can neither lower the minimum of the node's value and the formula's nor take part in
 //   it; closer values count as a dependency;
-//   adjoint: a neighbour of smaller or equal traveltime enters as +0 * lambda, which can change
-//   no bit of a nonzero sum of finite terms; a zero lambda (the sign of a zero sum) and a
-//   non-finite change count as dependencies.
+//   adjoint: adj_depends_exact (exact_arith.h).
 template <int KIND, typename B, typename Real, typename Aux>
-__device__ __forceinline__ bool depends_on(B lo, Real nv, Aux t0, Real vn, Aux tn) {
+__device__ __forceinline__ bool depends_on(B lo, Real old, Real nv, Aux t0, Real vn, Aux tn) {
     if constexpr (KIND == kFwdPlain64) return lo < obits(vn) + (1ll << 33);
-    else if constexpr (KIND == kAdjPlain64)
-        return ordered(t0) > ordered(tn) || is_zero(vn) || exponent_of(nv) == 0x7ff;
+    else if constexpr (KIND == kAdjPlain64) return adj_depends_exact(t0, tn, vn, old, nv);
     else if constexpr (Traits<KIND>::adj) return obits(t0) > obits(tn);
     else return lo < obits(vn);
 }
@@ -1150,7 +1147,7 @@ __device__ __forceinline__ void process_tile(const Sweep3Args& A, const int inst
                 // The neighbour values were read before this step's stores, none of which
                 // touches them (they lie on the hyperplanes t - 1 and t + 1).
                 const auto lo = min(obits(old), obits(nv));
-                auto dep = [&](Real vn, Aux tn) { return depends_on<KIND>(lo, nv, t0, vn, tn); };
+                auto dep = [&](Real vn, Aux tn) { return depends_on<KIND>(lo, old, nv, t0, vn, tn); };
                 if (lkf == 0 && dep(zu, Tzu)) m_zu = true;
                 if (lkf == ek - 1 && dep(zd, Tzd)) m_zd = true;
                 if (lif == 0 && dep(yu, Tyu)) m_yu = true;

@@ -110,5 +110,32 @@ int main() {
         }
         report("adj_axis_any_time", n, wrong);
     }
+    {   // marking: a node that does not depend on a neighbour's change keeps every bit under it
+        const double vals[] = {0.0, -0.0, INFINITY, -(double)INFINITY, std::nan(""), 1.7e308, 1e300, 1e-310, 1.0, -2.5};
+        auto node = [&](double T0, const double* T, const double* L) {
+            double den = 0.0, num = 0.0;
+            for (int a = 0; a < 3; ++a) {
+                double de, ne;
+                axis_ref(T0, T[2 * a], T[2 * a + 1], L[2 * a], L[2 * a + 1], 20.0, de, ne);
+                den = a ? den + de : de;
+                num = a ? num + ne : ne;
+            }
+            return std::fabs(den) > 1e-9 ? num / den : 0.0;
+        };
+        long long n = 0, wrong = 0, skipped = 0;
+        for (int i = 0; i < 4000000; ++i) {
+            const double T0 = uni(0.0, 1.0);
+            double T[6], L[6];
+            for (double& t : T) t = rng() % 6 ? T0 + uni(-0.1, 0.1) : T0;
+            for (double& v : L) v = rng() % 3 ? uni(-30.0, 30.0) : vals[rng() % 10];
+            const int c = rng() % 6;
+            const double nv = rng() % 2 ? uni(-30.0, 30.0) : vals[rng() % 10], old = L[c];
+            const double before = node(T0, T, L);
+            L[c] = nv;
+            if (!adj_depends_exact(T[c], T0, before, old, nv)) wrong += !same(before, node(T0, T, L)), ++skipped;
+            ++n;
+        }
+        report("adj_marking", n, wrong + (skipped < n / 8));
+    }
     return bad ? 1 : 0;
 }

@@ -27,7 +27,7 @@ def check_lines(tmp_path_factory):
     return subprocess.run([exe], capture_output=True, text=True, timeout=300).stdout.splitlines()
 
 
-@pytest.mark.parametrize("name", ["eik3_slowness", "eik2_slowness", "adj_axis_any_time"])
+@pytest.mark.parametrize("name", ["eik3_slowness", "eik2_slowness", "adj_axis_any_time", "adj_marking"])
 def test_updates_match_the_expressions(check_lines, name):
     line = [x for x in check_lines if x.split()[1] == name]
     assert line and line[0].startswith("ok "), check_lines
