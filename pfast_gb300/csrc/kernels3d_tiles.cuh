@@ -31,7 +31,7 @@
 #include <type_traits>
 #include <cooperative_groups.h>
 #include "kernels.h"
-#include "dataflow3.h"
+#include "dataflow_queue.h"
 #include "tune_policy.h"
 
 namespace pfast {
@@ -1296,18 +1296,9 @@ __global__ void __launch_bounds__(kWarps3 * 32) sweep3d_kernel(const Sweep3Args 
 // progress for two seconds sets *err, records the instance as not converged and exits.
 // result[inst] = iterations | 1 << 30 when not converged.  A.iter is the first iteration's
 // number: a solve continued from per-diagonal iterations counts on from them.
-constexpr unsigned kSlotEmpty = 0xffffffffu;
 // shared-memory copy of a model's arguments (multi-grid launches)
 constexpr int kDfArgsBytes = (int)((sizeof(Sweep3Args) + 15) / 16 * 16);
 static_assert(sizeof(Sweep3Args) % 8 == 0 && sizeof(Sweep3Args) % 4 == 0, "argument copy by words");
-
-struct alignas(16) DataflowShared {
-    unsigned head, tail;   // ring positions: next to take / next to fill
-    int done;              // items completed in this outer iteration
-    int abort;
-    int item;
-    int flags[2];          // clusters, by iteration parity: bit 0 some tile moved, bit 1 some tile due
-};
 
 __device__ __forceinline__ unsigned long long global_ns() {
     unsigned long long t;
@@ -1315,105 +1306,30 @@ __device__ __forceinline__ unsigned long long global_ns() {
     return t;
 }
 
-// Orders this thread's earlier accesses before its later ones for the other warps of the block
-// (CL: of the cluster; the field then travels through L2 between SMs).
+// The queue's memory (dataflow_queue.h) for the warps of a block or (CL) of a cluster, whose field
+// then travels through L2 between SMs.
 template <bool CL>
-__device__ __forceinline__ void df_fence() {
-    if constexpr (CL) asm volatile("fence.acq_rel.cluster;" ::: "memory");
-    else __threadfence_block();
-}
-
-// The queue words of a block or cluster: the counters, the ring and its state (CL: in the shared
-// memory of the cluster's first block, reached through distributed shared memory).
-struct DataflowQueue {
-    unsigned* cnt;
-    unsigned* slots;
-    unsigned qmask;
-    DataflowShared* sh;
+struct DataflowMemory {
+    __device__ __forceinline__ unsigned add(unsigned* p, unsigned v) const { return atomicAdd(p, v); }
+    __device__ __forceinline__ unsigned sub(unsigned* p, unsigned v) const { return atomicSub(p, v); }
+    __device__ __forceinline__ unsigned cas(unsigned* p, unsigned want, unsigned v) const { return atomicCAS(p, want, v); }
+    __device__ __forceinline__ void fence() const {
+        if constexpr (CL) asm volatile("fence.acq_rel.cluster;" ::: "memory");
+        else __threadfence_block();
+    }
+    __device__ __forceinline__ bool stopped(const DataflowQueue& Q) const { return *(volatile int*)&Q.sh->abort != 0; }
+    __device__ __forceinline__ void stop(const DataflowQueue& Q) const { *(volatile int*)&Q.sh->abort = 1; }
 };
 
-__device__ __forceinline__ void df_push(const DataflowQueue& Q, unsigned e) {
-    const unsigned p = atomicAdd(&Q.sh->tail, 1u);
-    unsigned* slot = Q.slots + (p & Q.qmask);
-    // a slot still holds an earlier round's item only while that item's taker is about to
-    // exchange it out (at most ntiles <= ring size items are outstanding): wait for it
-    for (int spin = 0; atomicCAS(slot, kSlotEmpty, e) != kSlotEmpty; ++spin)
-        if (spin > (1 << 22) || *(volatile int*)&Q.sh->abort) { *(volatile int*)&Q.sh->abort = 1; return; }
-}
-
-// The k-th possible dependent of item (o, x), k < 13 (dataflow3.h: dependents()): -1, or the item
-// that has one missing dependency fewer.
-__device__ __forceinline__ int df_dependent(const TileGrid3& g, int o, int x, int k) {
-    if (k == 0) return o < 7 ? (x << 3) | (o + 1) : -1;
-    const int a = (k - 1) >> 2, s = ((k - 1) >> 1) & 1, later = (k - 1) & 1;
-    const int y = tile_neighbour(g, x, a, s);
-    if (y < 0) return -1;
-    if (!later) return side_upstream(o, a, 1 - s) ? (y << 3) | o : -1;
-    return o < 7 && !side_upstream(o + 1, a, 1 - s) ? (y << 3) | (o + 1) : -1;
-}
-
-// Item e has one missing dependency fewer; returns its count before.  A block keeps two 4-bit
-// counters per tile, four tiles per word; a cluster, whose completions would wait for the re-arming
-// of one, all eight orders' counters, one word per tile.
+// Completion of item (o, x) by a whole warp (df_complete_lane).
 template <bool CL>
-__device__ __forceinline__ unsigned df_notify(const DataflowQueue& Q, int e) {
-    const int y = e >> 3;
-    const unsigned shf = CL ? 4u * (unsigned)(e & 7) : 8u * (unsigned)(y & 3) + 4u * (unsigned)(e & 1);
-    return (atomicSub(Q.cnt + (CL ? y : y >> 2), 1u << shf) >> shf) & 15u;
-}
-
-// Re-arm x's counter of parity o for order o + 2 (it is zero: it fired for (o, x), and no
-// dependency of (o + 2, x) completes before (o, x) did).
-__device__ __forceinline__ void df_rearm(const TileGrid3& g, const DataflowQueue& Q, int o, int x) {
-    if (o + 2 < 8)
-        atomicAdd(Q.cnt + (x >> 2), (unsigned)dep_count(g, o + 2, x) << (8u * (unsigned)(x & 3) + 4u * (unsigned)(o & 1)));
-}
-
-// Completion of item (o, x) by one lane: re-arm, then notify the dependents (the notifications
-// are all in flight together).  Of the items that become ready, one is returned for the lane to
-// go on with; the others join the ring.
-template <bool CL>
-__device__ __forceinline__ unsigned df_complete(const TileGrid3& g, const DataflowQueue& Q, int o, int x) {
+__device__ __forceinline__ unsigned df_complete_warp(const DataflowMemory<CL>& m, const TileGrid3& g, const DataflowQueue& Q,
+                                                     int o, int x, int lane) {
     if constexpr (!CL) {
-        df_rearm(g, Q, o, x);
-        df_fence<CL>();
-    }
-    int dep[13];
-    unsigned old[13];
-#pragma unroll
-    for (int k = 0; k < 13; ++k) {
-        dep[k] = df_dependent(g, o, x, k);
-        old[k] = dep[k] >= 0 ? df_notify<CL>(Q, dep[k]) : 2u;
-    }
-    unsigned keep = kSlotEmpty;
-#pragma unroll
-    for (int k = 0; k < 13; ++k) {
-        if (old[k] == 1u) {
-            if (keep == kSlotEmpty) keep = (unsigned)dep[k];
-            else df_push(Q, (unsigned)dep[k]);
-        } else if (old[k] == 0u) {
-            *(volatile int*)&Q.sh->abort = 1;   // more completions than dependencies: stop
-        }
-    }
-    return keep;
-}
-
-// The same by a whole warp, one dependent per lane: each lane returns its dependent if that
-// became ready.
-template <bool CL>
-__device__ __forceinline__ unsigned df_complete_warp(const TileGrid3& g, const DataflowQueue& Q, int o, int x, int lane) {
-    if constexpr (!CL) {
-        if (lane == 0) df_rearm(g, Q, o, x);
+        if (lane == 0) df_rearm(m, g, Q, o, x);
     }
     __syncwarp();
-    unsigned keep = kSlotEmpty;
-    const int dep = lane < 13 ? df_dependent(g, o, x, lane) : -1;
-    if (dep >= 0) {
-        df_fence<CL>();   // what the warp wrote (seen by this lane through the warp barrier) first
-        const unsigned old = df_notify<CL>(Q, dep);
-        if (old == 1u) keep = (unsigned)dep;
-        else if (old == 0u) *(volatile int*)&Q.sh->abort = 1;
-    }
+    const unsigned keep = df_complete_lane<CL>(m, g, Q, o, x, lane);
     __syncwarp();
     return keep;
 }
@@ -1428,6 +1344,7 @@ __device__ __forceinline__ void df_iteration(const Sweep3Args& A, const int inst
     // polish 29.4 -> 27.9 ms); a block's put them into the ring, which keeps the oldest first (there
     // going on with the newest was 5 to 20 % slower).
     constexpr bool kKeep = CL;
+    const DataflowMemory<CL> m;
     const int total = 8 * A.ntiles;
     const int* dirty = A.dirty + (long long)inst * A.ntiles;
     int last_done = -1;
@@ -1475,10 +1392,10 @@ __device__ __forceinline__ void df_iteration(const Sweep3Args& A, const int inst
                 unsigned* slot = Q.slots + ((h + (unsigned)lane) & Q.qmask);
                 // the item's producer reserved this position before we took it: it is being written
                 for (int spin = 0; (e = atomicExch(slot, kSlotEmpty)) == kSlotEmpty; ++spin)
-                    if (spin > (1 << 22) || *(volatile int*)&Q.sh->abort) { *(volatile int*)&Q.sh->abort = 1; break; }
+                    if (spin > (1 << 22) || m.stopped(Q)) { m.stop(Q); break; }
+                m.fence();
             }
         }
-        df_fence<CL>();
         const bool have = e != kSlotEmpty;
         const int x = (int)(e >> 3), o = (int)(e & 7u);
         int dm = 0;
@@ -1492,21 +1409,22 @@ __device__ __forceinline__ void df_iteration(const Sweep3Args& A, const int inst
         unsigned next = kSlotEmpty;
         int ncomp = 0;
         if (have && !due) {   // locked in this order: nothing to compute
-            next = df_complete<CL>(g, Q, o, x);
+            next = df_complete<CL>(m, g, Q, o, x);
             ncomp = 1;
         }
         if (mine >= 0) {
             if (due && lane != mine) next = e;
-            if (next != kSlotEmpty) df_push(Q, next);   // for an idle warp
+            if (next != kSlotEmpty) df_push(m, Q, next);   // for an idle warp
             const int ex = __shfl_sync(0xffffffffu, x, mine), eo = __shfl_sync(0xffffffffu, o, mine);
             const int edm = __shfl_sync(0xffffffffu, dm, mine);
             const int tj = ex % g.nbj, ti = (ex / g.nbj) % g.nbi, tk = ex / (g.nbj * g.nbi);
+            __syncwarp();   // the other lanes behind lane `mine`, which took the item
             process_tile<KIND, true, FORM, SH>(A, inst, ex, tk, ti, tj, eo, iter, edm, wsm, lane);
-            next = df_complete_warp<CL>(g, Q, eo, ex, lane);
+            next = df_complete_warp<CL>(m, g, Q, eo, ex, lane);
             if (lane == 0) ++ncomp;
         }
         if constexpr (!kKeep) {
-            if (next != kSlotEmpty) df_push(Q, next);
+            if (next != kSlotEmpty) df_push(m, Q, next);
             next = kSlotEmpty;
         }
         e = next;
