@@ -13,6 +13,7 @@
 #include <algorithm>
 #include <type_traits>
 #include "kernels2d.h"
+#include "strip_sync.h"
 
 namespace pfast {
 
@@ -629,6 +630,31 @@ __device__ __forceinline__ unsigned long long strip_ns() {
     return t;
 }
 
+// A lane's view of its warp for strip_sync.h.
+struct StripWarp {
+    int lane;
+    int* abort;
+    __device__ __forceinline__ bool leader() const { return lane == 0; }
+    __device__ __forceinline__ void barrier() const { __syncwarp(); }
+    __device__ __forceinline__ void fence() const { __threadfence_block(); }
+    __device__ __forceinline__ void store(volatile int* p, int v) const { *p = v; }
+    __device__ __forceinline__ int broadcast(int v) const { return __shfl_sync(0xffffffffu, v, 0); }
+    // until *p >= want (a word of another warp of this block), two seconds at most; 0: given up
+    __device__ __forceinline__ int poll(volatile int* p, int want) const {
+        unsigned long long since = 0;
+        for (int spin = 0; *p < want; ++spin) {
+            if (*(volatile int*)abort) return 0;
+            if (spin > 16) __nanosleep(40);
+            if ((spin & 1023) == 1023) {
+                const unsigned long long now = strip_ns();
+                if (!since) since = now;
+                else if (now - since > 2000000000ull) { *(volatile int*)abort = 1; return 0; }
+            }
+        }
+        return 1;
+    }
+};
+
 // Traveltimes for the FP32 bulk adjoint, per instance: split parts, +inf where unreached.  An offset
 // from a tile's corner is then three FP32 operations per value; split in the step instead, the
 // sweep took 12.5 ms for 40 + 40 instances of 601 x 201 nodes.
@@ -672,25 +698,8 @@ __global__ void __launch_bounds__(kStripMax * 32) sweep2d_strips(const Sweep2Arg
     const int i0 = w * T2I, ei = min(T2I, nr - i0), last = ei - 1;
     const Real fill = ADJ ? Real(0) : Real(INFINITY);
     const float tabs_f = narrow_trunc(A.tol_abs), trel_f = narrow_trunc(A.tol_rel);
-    // wait until *p >= want (a word of another warp of this block); false: given up (warp-uniform)
-    auto wait_for = [&](volatile int* p, int want) -> bool {
-        int ok = 1;
-        if (lane == 0) {
-            unsigned long long since = 0;
-            for (int spin = 0; *p < want; ++spin) {
-                if (*(volatile int*)&s_abort) { ok = 0; break; }
-                if (spin > 16) __nanosleep(40);
-                if ((spin & 1023) == 1023) {
-                    const unsigned long long now = strip_ns();
-                    if (!since) since = now;
-                    else if (now - since > 2000000000ull) { *(volatile int*)&s_abort = 1; ok = 0; break; }
-                }
-            }
-        }
-        ok = __shfl_sync(0xffffffffu, ok, 0);
-        __threadfence_block();
-        return ok != 0;
-    };
+    const StripWarp warp{lane, &s_abort};
+    auto wait_for = [&](volatile int* p, int want) -> bool { return strip_wait(warp, p, want); };   // warp-uniform
     auto tile_end = [&](int cf, bool px) { return min(nc, px ? (cf + 1) * T2J : nc - (nbj - 1) * T2J + cf * T2J); };
 
     for (;;) {
@@ -759,11 +768,8 @@ __global__ void __launch_bounds__(kStripMax * 32) sweep2d_strips(const Sweep2Arg
                         if (hasU) ok = wait_for(s_tdone + strip_tile(us, cf), o + 1);
                         if (!ok) break;
                         if (!due(word(tile_at(cf)))) {   // locked in this order
-                            __syncwarp();
-                            if (lane == 0) {
-                                s_prog[w] = pbase + tile_end(cf, px);
-                                s_tdone[tile_at(cf)] = o + 1;
-                            }
+                            strip_publish(warp, s_prog + w, pbase + tile_end(cf, px));
+                            strip_publish(warp, s_tdone + tile_at(cf), o + 1);
                             ++cf;
                             continue;
                         }
@@ -1042,9 +1048,8 @@ __global__ void __launch_bounds__(kStripMax * 32) sweep2d_strips(const Sweep2Arg
                                     else if (f & kMoved) s_diff[tt] = 1;
                                 }
                                 *(volatile int*)(s_dirty + tt) = word_;
-                                __threadfence_block();
-                                s_tdone[tt] = o + 1;
                             }
+                            strip_publish(warp, s_tdone + tt, o + 1);
                             __syncwarp();
                             if (cB == cA) break;   // the stream ends here
                             cA = cB;
