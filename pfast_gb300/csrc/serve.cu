@@ -38,7 +38,6 @@ struct Model {
     double dx = 0, dy = 0, dz = 0;
     double* d_vp = nullptr;
     double* d_wr = nullptr;
-    cudaStream_t astream = nullptr;   // of the arrays
     size_t bytes = 0;
     int refs = 0;
     bool dropped = false;
@@ -69,15 +68,18 @@ struct Job {
     Clock::time_point t_submit, t_start, t_done;
 };
 
-void free_model(Model& m) {
-    if (m.d_vp) cudaFreeAsync(m.d_vp, m.astream);
-    if (m.d_wr) cudaFreeAsync(m.d_wr, m.astream);
+// Resident arrays go back to the device's memory pool in stream order (cudaFree would wait for the
+// sweeps of every request), on the stream of the caller's context; the pool hands them to the rest of the
+// process at that stream's next synchronisation, so every caller synchronises it, without the lock.
+void free_model(Model& m, cudaStream_t st) {
+    if (m.d_vp) cudaFreeAsync(m.d_vp, st);
+    if (m.d_wr) cudaFreeAsync(m.d_wr, st);
     m.d_vp = m.d_wr = nullptr;
 }
 
-void free_survey(Survey& s) {
-    if (s.sv3) pfast_survey3d_destroy(s.sv3);
-    if (s.sv2) pfast_survey2d_destroy(s.sv2);
+void free_survey(Survey& s, cudaStream_t st) {
+    if (s.sv3) { s.sv3->astream = st; pfast_survey3d_destroy(s.sv3); }
+    if (s.sv2) { s.sv2->astream = st; pfast_survey2d_destroy(s.sv2); }
     s.sv3 = nullptr;
     s.sv2 = nullptr;
 }
@@ -138,12 +140,12 @@ bool reserve_resident(pfast_server* srv, size_t bytes) {
         if (which == 0) {
             auto m = srv->models[id];
             srv->models.erase(id);
-            free_model(*m);
+            free_model(*m, srv->admin->own_stream);
             srv->policy->release(m->bytes);
         } else {
             auto s = srv->surveys[id];
             srv->surveys.erase(id);
-            free_survey(*s);
+            free_survey(*s, srv->admin->own_stream);
             srv->policy->release(s->bytes);
         }
     }
@@ -219,21 +221,17 @@ void worker_main(pfast_server* srv, int slot) {
         ctx_release_buffers(ctx);   // stream-ordered: the memory returns to the pool
         cudaStreamSynchronize(ctx->stream);
         lk.lock();
-        job->t_done = Clock::now();
-        job->status = st;
-        job->message = msg;
-        job->done = true;
         srv->policy->finish(job->bytes);
-        srv->completed += 1;
-        if (st != PFAST_OK) srv->failed += 1;
         job->model->refs -= 1;
         job->survey->refs -= 1;
         job->model->last_use = ++srv->clock;
         job->survey->last_use = srv->clock;
         // dropped entries go once unused
+        bool freed = false;
         for (auto it = srv->models.begin(); it != srv->models.end();) {
             if (it->second->dropped && it->second->refs == 0) {
-                free_model(*it->second);
+                free_model(*it->second, ctx->own_stream);
+                freed = true;
                 srv->policy->release(it->second->bytes);
                 it = srv->models.erase(it);
             } else {
@@ -242,7 +240,8 @@ void worker_main(pfast_server* srv, int slot) {
         }
         for (auto it = srv->surveys.begin(); it != srv->surveys.end();) {
             if (it->second->dropped && it->second->refs == 0) {
-                free_survey(*it->second);
+                free_survey(*it->second, ctx->own_stream);
+                freed = true;
                 srv->policy->release(it->second->bytes);
                 it = srv->surveys.erase(it);
             } else {
@@ -251,6 +250,17 @@ void worker_main(pfast_server* srv, int slot) {
         }
         job->model.reset();
         job->survey.reset();
+        if (freed) {
+            lk.unlock();
+            cudaStreamSynchronize(ctx->own_stream);
+            lk.lock();
+        }
+        job->t_done = Clock::now();
+        job->status = st;
+        job->message = msg;
+        job->done = true;
+        srv->completed += 1;
+        if (st != PFAST_OK) srv->failed += 1;
         srv->cv_done.notify_all();
         srv->cv_work.notify_all();
     }
@@ -300,8 +310,8 @@ pfast_status pfast_server_destroy(pfast_server* srv) {
     }
     srv->cv_work.notify_all();
     for (auto& t : srv->workers) t.join();
-    for (auto& kv : srv->models) free_model(*kv.second);
-    for (auto& kv : srv->surveys) free_survey(*kv.second);
+    for (auto& kv : srv->models) free_model(*kv.second, srv->admin->own_stream);
+    for (auto& kv : srv->surveys) free_survey(*kv.second, srv->admin->own_stream);
     for (pfast_ctx* c : srv->ctxs) pfast_ctx_destroy(c);
     if (srv->admin) pfast_ctx_destroy(srv->admin);
     delete srv;
@@ -319,54 +329,60 @@ pfast_status pfast_server_put_model(pfast_server* srv, long long model_id, int d
     m->dim = dim; m->nr = nrows; m->nc = ncols; m->nz = nz; m->dx = dx; m->dy = dy; m->dz = dz;
     const size_t N = (size_t)nz * nrows * ncols;
     m->bytes = N * 8 * (WR ? 2 : 1);
+    cudaStream_t st = srv->admin->own_stream;
+    bool fits = false;
     {
         std::lock_guard<std::mutex> g(srv->mu);
         auto it = srv->models.find(model_id);
         if (it != srv->models.end()) {
             if (it->second->refs > 0) { set_last_error("put_model: model %lld is in use", model_id); return PFAST_ERR_INVALID; }
-            free_model(*it->second);
+            free_model(*it->second, st);
             srv->policy->release(it->second->bytes);
             srv->models.erase(it);
         }
-        if (!reserve_resident(srv, m->bytes)) {
-            set_last_error("put_model: %zu bytes do not fit the HBM budget", m->bytes);
-            return PFAST_ERR_NOMEM;
-        }
+        fits = reserve_resident(srv, m->bytes);
     }
     PFAST_CUDA_TRY(cudaSetDevice(srv->cfg.device));
-    m->astream = srv->admin->own_stream;
-    cudaError_t e = cudaMallocAsync(&m->d_vp, N * 8, m->astream);
-    if (e == cudaSuccess && WR) e = cudaMallocAsync(&m->d_wr, N * 8, m->astream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(m->d_vp, vp, N * 8, cudaMemcpyHostToDevice, m->astream);
-    if (e == cudaSuccess && WR) e = cudaMemcpyAsync(m->d_wr, WR, N * 8, cudaMemcpyHostToDevice, m->astream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(m->astream);
-    std::lock_guard<std::mutex> g(srv->mu);
+    if (!fits) {
+        cudaStreamSynchronize(st);
+        set_last_error("put_model: %zu bytes do not fit the HBM budget", m->bytes);
+        return PFAST_ERR_NOMEM;
+    }
+    cudaError_t e = cudaMallocAsync(&m->d_vp, N * 8, st);
+    if (e == cudaSuccess && WR) e = cudaMallocAsync(&m->d_wr, N * 8, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(m->d_vp, vp, N * 8, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess && WR) e = cudaMemcpyAsync(m->d_wr, WR, N * 8, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) {
-        free_model(*m);
+        free_model(*m, st);
+        cudaStreamSynchronize(st);
+        std::lock_guard<std::mutex> g(srv->mu);
         srv->policy->release(m->bytes);
         return cuda_fail(e, "put_model", __FILE__, __LINE__);
     }
+    std::lock_guard<std::mutex> g(srv->mu);
     m->last_use = ++srv->clock;
     srv->models[model_id] = m;
     srv->cv_work.notify_all();
     return PFAST_OK;
 }
 
-static pfast_status put_survey(pfast_server* srv, long long survey_id, std::shared_ptr<Survey> s) {
+static pfast_status put_survey_locked(pfast_server* srv, long long survey_id, std::shared_ptr<Survey> s) {
+    cudaStream_t st = srv->admin->own_stream;
     std::lock_guard<std::mutex> g(srv->mu);
     auto it = srv->surveys.find(survey_id);
     if (it != srv->surveys.end()) {
         if (it->second->refs > 0) {
-            free_survey(*s);
+            free_survey(*s, st);
             set_last_error("put_survey: survey %lld is in use", survey_id);
             return PFAST_ERR_INVALID;
         }
-        free_survey(*it->second);
+        free_survey(*it->second, st);
         srv->policy->release(it->second->bytes);
         srv->surveys.erase(it);
     }
     if (!reserve_resident(srv, s->bytes)) {
-        free_survey(*s);
+        free_survey(*s, st);
         set_last_error("put_survey: %zu bytes do not fit the HBM budget", s->bytes);
         return PFAST_ERR_NOMEM;
     }
@@ -374,6 +390,12 @@ static pfast_status put_survey(pfast_server* srv, long long survey_id, std::shar
     srv->surveys[survey_id] = s;
     srv->cv_work.notify_all();
     return PFAST_OK;
+}
+
+static pfast_status put_survey(pfast_server* srv, long long survey_id, std::shared_ptr<Survey> s) {
+    const pfast_status r = put_survey_locked(srv, survey_id, s);
+    cudaStreamSynchronize(srv->admin->own_stream);   // what it replaced, evicted or refused
+    return r;
 }
 
 pfast_status pfast_server_put_survey3d(pfast_server* srv, long long survey_id, int nrows, int ncols, int nz, double dx,
@@ -403,14 +425,14 @@ pfast_status pfast_server_put_survey2d(pfast_server* srv, long long survey_id, i
     return put_survey(srv, survey_id, s);
 }
 
-pfast_status pfast_server_drop(pfast_server* srv, int what, long long id) {
-    if (!srv) { set_last_error("null server"); return PFAST_ERR_INVALID; }
+static pfast_status drop_locked(pfast_server* srv, int what, long long id) {
+    cudaStream_t st = srv->admin->own_stream;
     std::lock_guard<std::mutex> g(srv->mu);
     if (what == 0) {
         auto it = srv->models.find(id);
         if (it == srv->models.end()) { set_last_error("drop: no model %lld", id); return PFAST_ERR_INVALID; }
         if (it->second->refs == 0) {
-            free_model(*it->second);
+            free_model(*it->second, st);
             srv->policy->release(it->second->bytes);
             srv->models.erase(it);
         } else {
@@ -420,7 +442,7 @@ pfast_status pfast_server_drop(pfast_server* srv, int what, long long id) {
         auto it = srv->surveys.find(id);
         if (it == srv->surveys.end()) { set_last_error("drop: no survey %lld", id); return PFAST_ERR_INVALID; }
         if (it->second->refs == 0) {
-            free_survey(*it->second);
+            free_survey(*it->second, st);
             srv->policy->release(it->second->bytes);
             srv->surveys.erase(it);
         } else {
@@ -428,6 +450,13 @@ pfast_status pfast_server_drop(pfast_server* srv, int what, long long id) {
         }
     }
     return PFAST_OK;
+}
+
+pfast_status pfast_server_drop(pfast_server* srv, int what, long long id) {
+    if (!srv) { set_last_error("null server"); return PFAST_ERR_INVALID; }
+    const pfast_status r = drop_locked(srv, what, id);
+    if (r == PFAST_OK) cudaStreamSynchronize(srv->admin->own_stream);
+    return r;
 }
 
 pfast_status pfast_server_submit(pfast_server* srv, const pfast_request* req, long long* ticket) {
