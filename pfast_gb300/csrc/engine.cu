@@ -160,27 +160,10 @@ Spacing3 make_spacing(double dx, double dy, double dz) {
 
 // Run outer iterations of `kind` over the active batch instances until each one
 // converges or reaches maxiter.  iters[b] receives the iteration count of instance b.
-// Autotuner, per (device, sweep kind, grid, active instances): the phase times of each
-// (schedule, tile shape) candidate, measured by pfast_survey3d_autotune, which runs the same
-// evaluation once with each; the choice itself is tune_policy.h.
-static std::mutex g_tune_mu;
-static std::map<std::tuple<int, int, int, int, int, int>, TuneEntry> g_tune;
-
-// The fastest allowed candidate once all are timed; -1 before that.
-static int tuned_candidate(const std::tuple<int, int, int, int, int, int>& key, unsigned allowed, int sms) {
-    std::lock_guard<std::mutex> g(g_tune_mu);
-    auto it = g_tune.find(key);
-    if (it == g_tune.end() || !tune_complete(&it->second, allowed)) return -1;
-    return tune_pick(&it->second, allowed, std::get<5>(key), sms);
-}
-
-static void tune_record(const std::tuple<int, int, int, int, int, int>& key, int which, double ms) {
-    if (!(ms > 0.0)) return;
-    std::lock_guard<std::mutex> g(g_tune_mu);
-    TuneEntry& e = g_tune[key];
-    e.ms[which] += ms;
-    e.n[which] += 1;
-}
+// Autotuner: the phase times of each (schedule, tile shape) candidate, measured by
+// pfast_survey3d_autotune, which runs the same evaluation once with each; the choice itself is
+// tune_policy.h.
+static TuneTable g_tune;
 
 // One outer iteration of a per-diagonal phase as a CUDA graph: the diff reset, the 8 x ndiag
 // sweep launches and the per-instance reduction, captured once per (kind, launch arguments,
@@ -262,8 +245,9 @@ pfast_status run_sweeps3(pfast_ctx* ctx, Sweep3Args a, int kind, int nb, std::ve
     int dev = 0, sms = 1;
     PFAST_CUDA_TRY(cudaGetDevice(&dev));
     PFAST_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const auto tkey = std::make_tuple(dev, kind, a.nz, a.nr, a.nc, (int)active.size());
-    const int load = (int)active.size() * SweepScope::count(dev);
+    const TuneTable::Phase phase = {dev, kind, a.nz, a.nr, a.nc, (int)active.size()};
+    const int under_way = SweepScope::count(dev);
+    const int load = (int)active.size() * under_way;
     DataflowShape dshape[kTileShapes];
     bool fits[kTileShapes] = {};
     for (int shape = 0; shape < kTileShapes; ++shape) {
@@ -275,7 +259,8 @@ pfast_status run_sweeps3(pfast_ctx* ctx, Sweep3Args a, int kind, int nb, std::ve
         fits[shape] = dshape[shape].warps > 0;
     }
     const unsigned allowed = tune_allowed(ctx->schedule, ctx->tile_shape, fits);
-    int cand = tuned_candidate(tkey, allowed, sms);
+    const int clusters[kTileShapes] = {dshape[0].cluster, dshape[1].cluster};
+    int cand = g_tune.pick(phase, under_way == 1, allowed, clusters, sms);
     if (cand < 0) {
         const int shape = ctx->tile_shape == PFAST_TILE_AUTO ? 0 : ctx->tile_shape - 1;
         DiagTable3* t = nullptr;
@@ -436,7 +421,7 @@ pfast_status run_sweeps3(pfast_ctx* ctx, Sweep3Args a, int kind, int nb, std::ve
     double ms = 0.0;
     add_elapsed(ctx->ev[0], ctx->ev[1], &ms);
     if (ms_acc) *ms_acc += ms;
-    if (ctx->tuning) tune_record(tkey, cand, ms);
+    if (ctx->tuning) g_tune.record(phase, under_way == 1 && SweepScope::count(dev) == 1, cand, clusters, ms);
     return PFAST_OK;
 }
 

@@ -5,7 +5,14 @@
 // (one launch per phase), 2 hybrid (first outer iteration per diagonal, then dataflow); shape
 // 0 = 4x8x32 tiles, 1 = 8x4x32.  pfast_survey3d_autotune records each candidate's phase times
 // per (device, sweep kind, grid, active instances); a phase then takes the fastest allowed one.
+// A dataflow or hybrid time belongs to the cluster size it was measured with (below), which depends
+// on the evaluations under way beside it.
 #pragma once
+
+#include <array>
+#include <map>
+#include <mutex>
+#include <tuple>
 
 namespace pfast {
 
@@ -32,10 +39,10 @@ inline unsigned tune_allowed(int schedule_opt, int shape_opt, const bool dataflo
     return allowed;
 }
 
-// The candidate of a phase: once every allowed candidate has been timed (e non-null), the one
-// with the smallest mean phase time (the first of equal ones); before that, the dataflow kernel
-// with 4x8x32 tiles from two active instances per SM, else one launch per tile diagonal
-// (falling back to the lowest allowed candidate).  The sweeps ask untuned_pick below until then.
+// The candidate of a phase once every allowed candidate has been timed: the one with the smallest
+// mean phase time (the first of equal ones).  Before that (which no sweep asks: they take untuned_pick
+// below until TuneTable has every time) the dataflow kernel with 4x8x32 tiles from two active
+// instances per SM, else one launch per tile diagonal, else the lowest allowed candidate.
 inline int tune_pick(const TuneEntry* e, unsigned allowed, int nact, int sms) {
     if (e) {
         int best = -1;
@@ -117,5 +124,44 @@ inline bool tune_complete(const TuneEntry* e, unsigned allowed) {
         if ((allowed >> c & 1) && e->n[c] == 0) return false;
     return true;
 }
+
+// The phase times of all candidates, from every thread.  With 16 blocks per source for 9 sources alone and
+// one when eight threads evaluate side by side, the time of a dataflow candidate says nothing about
+// the other case: a phase asks for the times of the cluster sizes it would launch with, measured as
+// it runs (alone or beside other evaluations) or else in the other way.
+class TuneTable {
+public:
+    using Phase = std::array<int, 6>;   // device, sweep kind, nz, nr, nc, active instances
+
+    void record(const Phase& p, bool alone, int c, const int cluster[2], double ms) {
+        if (!(ms > 0.0)) return;
+        std::lock_guard<std::mutex> g(mu_);
+        Time& t = times_[std::make_tuple(p, alone, c, blocks(c, cluster))];
+        t.ms += ms;
+        t.n += 1;
+    }
+
+    // The fastest allowed candidate once all are timed with these cluster sizes; -1 before that.
+    int pick(const Phase& p, bool alone, unsigned allowed, const int cluster[2], int sms) const {
+        std::lock_guard<std::mutex> g(mu_);
+        for (const bool how : {alone, !alone}) {
+            TuneEntry e;
+            for (int c = 0; c < kTuneCandidates; ++c) {
+                auto it = times_.find(std::make_tuple(p, how, c, blocks(c, cluster)));
+                if (it == times_.end()) continue;
+                e.ms[c] = it->second.ms;
+                e.n[c] = it->second.n;
+            }
+            if (tune_complete(&e, allowed)) return tune_pick(&e, allowed, p[5], sms);
+        }
+        return -1;
+    }
+
+private:
+    struct Time { double ms = 0.0; int n = 0; };
+    static int blocks(int c, const int cluster[2]) { return c < 2 ? 0 : cluster[c & 1]; }   // per diagonal: none
+    mutable std::mutex mu_;
+    std::map<std::tuple<Phase, bool, int, int>, Time> times_;
+};
 
 }  // namespace pfast
