@@ -446,15 +446,16 @@ pfast_status prepare_slowness(pfast_ctx* ctx, const double* vp, long long N, boo
         PFAST_TRY(ctx->s32.ensure(sizeof(float) * N));
         PFAST_TRY(ctx->sq64.ensure(sizeof(double) * N));
     }
-    PFAST_TRY(ctx->need.ensure(sizeof(int) * 4));
-    PFAST_CUDA_TRY(cudaMemsetAsync(ctx->need.p, 0, sizeof(int), ctx->stream));
+    PFAST_TRY(ctx->need.ensure(sizeof(VelocityCheck)));
+    PFAST_CUDA_TRY(cudaMemsetAsync(ctx->need.p, 0, sizeof(VelocityCheck), ctx->stream));
     PFAST_LAUNCH(ctx, launch_slowness(vp, ctx->s64.as<double>(), mixed ? ctx->s32.as<float>() : nullptr,
-                                      mixed ? ctx->sq64.as<double>() : nullptr, sq_scale, ctx->need.as<int>(), N,
+                                      mixed ? ctx->sq64.as<double>() : nullptr, sq_scale, ctx->need.as<VelocityCheck>(), N,
                                       ctx->stream));
-    int bad = 0;
-    PFAST_CUDA_TRY(cudaMemcpyAsync(&bad, ctx->need.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    VelocityCheck check;
+    PFAST_CUDA_TRY(cudaMemcpyAsync(&check, ctx->need.p, sizeof(check), cudaMemcpyDeviceToHost, ctx->stream));
     PFAST_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-    if (bad) {
+    ctx->vmax = check.largest();
+    if (check.bad) {
         set_last_error("the velocity model holds a value that is not a positive finite number");
         return PFAST_ERR_INVALID;
     }
@@ -472,6 +473,7 @@ pfast_status forward3d_batch(pfast_ctx* ctx, const pfast_survey3d* sv, int b0, i
     a.fstride = N;
     a.src_kij = sv->d_src_kij + 3 * b0;
     a.src_r2 = ctx->near_radius * ctx->near_radius;
+    a.prune_limit = forward_prune_limit(a.sp.d, ctx->vmax);
     const long long* src_lin = sv->d_src_lin + b0;
     int dummy_nc = 0;
     int* nc_ptr = st ? &st->not_converged : &dummy_nc;

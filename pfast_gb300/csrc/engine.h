@@ -81,6 +81,7 @@ struct pfast_ctx {
     int tile_shape = PFAST_TILE_AUTO;           // of the current 3D evaluation (pfast_options)
     int candidates = 0;                         // per sweep kind: 1 + candidate of its last phase (pfast_stats)
     int near_radius = 0;                        // of the current 3D evaluation (pfast_options)
+    double vmax = 0.0;                          // largest velocity of the current model
     // request server: the stream on which arrays of surveys created on this context are allocated and
     // freed, as cudaMalloc and cudaFree wait for the sweeps of every other stream
     cudaStream_t resident_stream = nullptr;

@@ -42,6 +42,7 @@ struct Sweep3Args {
                               // adjoint: relative to 1 + |lambda|)
     unsigned long long* work; // per instance: nodes of the tiles processed (executed node updates); may be null
     int shape;                // tile shape: 0 = 4x8x32, 1 = 8x4x32 (common.cuh: TileShape)
+    int prune_limit;          // plain forward: forward_prune_limit (exact_arith.h) of the grid and the model
     int vec_rows;             // rows of the field (and of the FP32 adjoint's traveltime) start on 16-byte
                               // boundaries: nc a multiple of 16 / element size, 16-byte aligned fields;
                               // tiles then move in 16-byte vectors
@@ -121,10 +122,15 @@ extern template struct ShapeLaunchers<Shape48>;
 extern template struct ShapeLaunchers<Shape84>;
 
 // Small 3D kernels.
-// s64 = 1.0/vp, s32 = (float)s64 (if non-null), sq64 = s64*s64*sq_scale (if non-null); *bad is set
-// when some vp is not a positive finite number.
-pfast_status launch_slowness(const double* vp, double* s64, float* s32, double* sq64, double sq_scale, int* bad, long long n,
-                             cudaStream_t st);
+// s64 = 1.0/vp, s32 = (float)s64 (if non-null), sq64 = s64*s64*sq_scale (if non-null); *check (device
+// memory, zeroed by the caller) tells whether some vp is not a positive finite number, and the largest.
+struct VelocityCheck {
+    int bad, pad;
+    unsigned long long vmax;   // bits of an FP64 number
+    double largest() const { double v; std::memcpy(&v, &vmax, sizeof(v)); return v; }
+};
+pfast_status launch_slowness(const double* vp, double* s64, float* s32, double* sq64, double sq_scale, VelocityCheck* check,
+                             long long n, cudaStream_t st);
 // Opt-in near-source start: nodes within `radius` nodes (Euclidean) of each instance's source get
 // 0.5*(s_src + s_node)*distance.  field: FP32 (is_fp32) or FP64 fields, fstride apart.
 pfast_status launch_near_source3(void* field, int is_fp32, long long fstride, const int* src_kij, const double* s64,

@@ -478,6 +478,8 @@ __global__ void __launch_bounds__(kWarps2 * 32) sweep2d_kernel(const Sweep2Args 
                         box[c] = nv;
                         chg = true;
                         note_move(old, nv, dstep);
+                        // (plain: as forward_depends_exact without a limit, since a discriminant that rounds
+                        // below 0 gives the unreached value here, and no third neighbour comes in)
                         auto dep = [&](int n) {
                             constexpr long long kMargin = KIND == kFwdPlain64 ? 1ll << 33 : 0;
                             return min(obits2(old), obits2(nv)) < obits2(box[n]) + kMargin;

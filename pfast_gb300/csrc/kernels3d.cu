@@ -152,15 +152,19 @@ inline unsigned grid_for(long long n) {
 }
 
 __global__ void slowness_kernel(const double* __restrict__ vp, double* __restrict__ s64, float* __restrict__ s32,
-                                double* __restrict__ sq64, int* __restrict__ bad, long long n, double sq_scale) {
+                                double* __restrict__ sq64, VelocityCheck* __restrict__ check, long long n, double sq_scale) {
+    unsigned long long vmax = 0;
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
         const double v = vp[t];
-        if (!(v > 0.0 && v < INFINITY)) *bad = 1;
+        if (!(v > 0.0 && v < INFINITY)) check->bad = 1;
+        else vmax = max(vmax, (unsigned long long)dbits(v));
         const double s = 1.0 / v;   // s = 1.0/vp, src/T_pfsm3d.h:75
         s64[t] = s;
         if (s32) s32[t] = (float)s;
         if (sq64) sq64[t] = (s * s) * sq_scale;
     }
+    for (int k = 16; k; k >>= 1) vmax = max(vmax, __shfl_xor_sync(0xffffffffu, vmax, k));
+    if (threadIdx.x % 32 == 0 && vmax > *(volatile unsigned long long*)&check->vmax) atomicMax(&check->vmax, vmax);
 }
 
 template <typename Real>
@@ -316,9 +320,9 @@ __global__ void gather3_kernel(const double* __restrict__ T, long long fstride, 
         if (e__ != cudaSuccess) return cuda_fail(e__, "kernel launch", __FILE__, __LINE__);    \
     } while (0)
 
-pfast_status launch_slowness(const double* vp, double* s64, float* s32, double* sq64, double sq_scale, int* bad, long long n,
-                             cudaStream_t st) {
-    slowness_kernel<<<grid_for(n), kThreads, 0, st>>>(vp, s64, s32, sq64, bad, n, sq_scale);
+pfast_status launch_slowness(const double* vp, double* s64, float* s32, double* sq64, double sq_scale, VelocityCheck* check,
+                             long long n, cudaStream_t st) {
+    slowness_kernel<<<grid_for(n), kThreads, 0, st>>>(vp, s64, s32, sq64, check, n, sq_scale);
     PFAST_LAUNCH_CHECK();
     return PFAST_OK;
 }

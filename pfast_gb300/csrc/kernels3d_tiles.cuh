@@ -685,18 +685,15 @@ __device__ __forceinline__ long long obits(double x) { return __double_as_longlo
 __device__ __forceinline__ int obits(float x) { return __float_as_int(x); }
 
 // Whether the update of a neighbour (value vn, traveltime tn) can depend on a node that changed
-// from old to nv; lo: the smaller of the node's old and new value (ordered bits), t0: its traveltime.
+// from old to nv; lo: the smaller of the node's old and new value (ordered bits; plain forward:
+// forward_change), t0: its traveltime.
 // Forward: the Godunov update and its Newton form exclude neighbours above the node's value.
 // Adjoint: lambda at a node weighs its neighbours with max(T_neighbour - T_node, 0).
 // The plain kinds skip tiles only where that leaves every bit as it is:
-//   forward: the reference's formula is the exact solution to within sqrt(8 eps) = 4e-8 relative at
-//   worst (its discriminant cancels), so a neighbour value more than 2^-20 relative above the
-//   node's can neither lower the minimum of the node's value and the formula's nor take part in
-//   it; closer values count as a dependency;
-//   adjoint: adj_depends_exact (exact_arith.h).
+// forward_depends_exact and adj_depends_exact (exact_arith.h).
 template <int KIND, typename B, typename Real, typename Aux>
 __device__ __forceinline__ bool depends_on(B lo, Real old, Real nv, Aux t0, Real vn, Aux tn) {
-    if constexpr (KIND == kFwdPlain64) return lo < obits(vn) + (1ll << 33);
+    if constexpr (KIND == kFwdPlain64) return forward_depends_exact(lo, vn);
     else if constexpr (KIND == kAdjPlain64) return adj_depends_exact(t0, tn, vn, old, nv);
     else if constexpr (Traits<KIND>::adj) return obits(t0) > obits(tn);
     else return lo < obits(vn);
@@ -1146,7 +1143,8 @@ __device__ __forceinline__ void process_tile(const Sweep3Args& A, const int inst
                 // does the neighbour across a face (value vn, traveltime tn) depend on this node?
                 // The neighbour values were read before this step's stores, none of which
                 // touches them (they lie on the hyperplanes t - 1 and t + 1).
-                const auto lo = min(obits(old), obits(nv));
+                auto lo = min(obits(old), obits(nv));
+                if constexpr (KIND == kFwdPlain64) lo = forward_change(old, nv, A.prune_limit);
                 auto dep = [&](Real vn, Aux tn) { return depends_on<KIND>(lo, old, nv, t0, vn, tn); };
                 if (lkf == 0 && dep(zu, Tzu)) m_zu = true;
                 if (lkf == ek - 1 && dep(zd, Tzd)) m_zd = true;

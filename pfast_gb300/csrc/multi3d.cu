@@ -34,7 +34,8 @@ struct Model {
     double *s64 = nullptr, *sq64 = nullptr, *T64 = nullptr, *L64 = nullptr, *scr = nullptr, *ee = nullptr;
     float *s32 = nullptr, *T32 = nullptr;
     unsigned* mask = nullptr;
-    int *tflags = nullptr, *act = nullptr, *changed = nullptr, *need = nullptr, *bad = nullptr;
+    int *tflags = nullptr, *act = nullptr, *changed = nullptr, *need = nullptr;
+    VelocityCheck* check = nullptr;
     unsigned long long* work = nullptr;
     // host
     std::vector<int> active, iters;
@@ -66,7 +67,7 @@ void carve(Model& m, unsigned char*& p, bool mixed) {
     m.need = (int*)take(4 * ns);
     m.ee = (double*)take(8 * ns);
     m.work = (unsigned long long*)take(8 * ns);
-    m.bad = (int*)take(4);
+    m.check = (VelocityCheck*)take(sizeof(VelocityCheck));
     if (mixed) {
         m.s32 = (float*)take(4 * N);
         m.sq64 = (double*)take(8 * N);
@@ -193,17 +194,17 @@ pfast_status eval_group(pfast_ctx* ctx, std::vector<Model>& ms, const pfast_opti
     // ---- slowness of every model; reject a model with a velocity that is not positive
     for (Model& M : ms) {
         const double hsq = (M.sv->dx == M.sv->dy && M.sv->dy == M.sv->dz) ? M.sv->dx * M.sv->dx : 1.0;
-        PFAST_CUDA_TRY(cudaMemsetAsync(M.bad, 0, sizeof(int), st));
-        PFAST_LAUNCH(ctx, launch_slowness(M.vp, M.s64, mixed ? M.s32 : nullptr, mixed ? M.sq64 : nullptr, hsq, M.bad,
-                                          M.N, st));
+        PFAST_CUDA_TRY(cudaMemsetAsync(M.check, 0, sizeof(VelocityCheck), st));
+        PFAST_LAUNCH(ctx, launch_slowness(M.vp, M.s64, mixed ? M.s32 : nullptr, mixed ? M.sq64 : nullptr, hsq,
+                                          M.check, M.N, st));
         PFAST_CUDA_TRY(cudaMemsetAsync(M.grad, 0, sizeof(double) * M.N, st));
     }
-    std::vector<int> bad(nm, 0);
+    std::vector<VelocityCheck> check(nm);
     for (int m = 0; m < nm; ++m)
-        PFAST_CUDA_TRY(cudaMemcpyAsync(&bad[m], ms[m].bad, sizeof(int), cudaMemcpyDeviceToHost, st));
+        PFAST_CUDA_TRY(cudaMemcpyAsync(&check[m], ms[m].check, sizeof(VelocityCheck), cudaMemcpyDeviceToHost, st));
     PFAST_CUDA_TRY(cudaStreamSynchronize(st));
     for (int m = 0; m < nm; ++m)
-        if (bad[m]) {
+        if (check[m].bad) {
             set_last_error("model %d holds a velocity that is not a positive finite number", m);
             return PFAST_ERR_INVALID;
         }
@@ -211,6 +212,7 @@ pfast_status eval_group(pfast_ctx* ctx, std::vector<Model>& ms, const pfast_opti
     auto base = [&](int m) {
         Sweep3Args a = survey_sweep_args(ms[m].sv);
         a.fstride = ms[m].N;
+        a.prune_limit = forward_prune_limit(a.sp.d, check[m].largest());
         return a;
     };
     auto all_active = [&]() {

@@ -48,7 +48,7 @@ constexpr size_t kOffDiag = align256(kOffTiles + 4 * (size_t)kMaxTiles);    // i
 constexpr size_t kOffFlags = align256(kOffDiag + 4 * (size_t)(kMaxDiag + 1));   // int[3*kMaxTiles]: dirty, stamp, diff
 constexpr size_t kOffWords = align256(kOffFlags + 12 * (size_t)kMaxTiles);
 // words: [0..1] source linear index (long long), [2..4] source (k,i,j), [5] active id,
-//        [6] changed flag, [7] bad-velocity flag
+//        [6] changed flag, [8..11] velocity check
 constexpr size_t kScratchBytes = align256(kOffWords + 64);
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
@@ -131,11 +131,11 @@ extern "C" pfast_status pfast_fsm3d_noalloc(const double* vp, double* U, int src
     int* d_src_kij = words + 2;
     int* d_act = words + 5;
     int* d_changed = words + 6;
-    int* d_bad = words + 7;
+    VelocityCheck* d_check = reinterpret_cast<VelocityCheck*>(words + 8);
     int* d_dirty = reinterpret_cast<int*>(base + kOffFlags);
     const int ntiles = nbk * nbi * nbj;
 
-    int hw[8];
+    int hw[12];
     const long long lin = (long long)src_z * nrows * ncols + (long long)src_row * ncols + src_col;
     std::memcpy(hw, &lin, sizeof(lin));
     hw[2] = src_z;
@@ -144,16 +144,17 @@ extern "C" pfast_status pfast_fsm3d_noalloc(const double* vp, double* U, int src
     hw[5] = 0;   // the single instance
     hw[6] = 0;
     hw[7] = 0;
+    hw[8] = hw[9] = hw[10] = hw[11] = 0;
     PFAST_CUDA_TRY(cudaMemcpyAsync(words, hw, sizeof(hw), cudaMemcpyHostToDevice, s));
     PFAST_CUDA_TRY(cudaMemcpyAsync(d_tiles, tiles.data(), sizeof(unsigned) * tiles.size(), cudaMemcpyHostToDevice, s));
     PFAST_CUDA_TRY(cudaMemcpyAsync(d_off, off.data(), sizeof(int) * off.size(), cudaMemcpyHostToDevice, s));
 
-    pfast_status r = launch_slowness(vp, slow, nullptr, nullptr, 1.0, d_bad, N, s);
+    pfast_status r = launch_slowness(vp, slow, nullptr, nullptr, 1.0, d_check, N, s);
     if (r) return r;
-    int bad = 0;
-    PFAST_CUDA_TRY(cudaMemcpyAsync(&bad, d_bad, sizeof(int), cudaMemcpyDeviceToHost, s));
+    VelocityCheck check;
+    PFAST_CUDA_TRY(cudaMemcpyAsync(&check, d_check, sizeof(check), cudaMemcpyDeviceToHost, s));
     PFAST_CUDA_TRY(cudaStreamSynchronize(s));
-    if (bad) {
+    if (check.bad) {
         set_last_error("the velocity model holds a value that is not a positive finite number");
         return PFAST_ERR_INVALID;
     }
@@ -184,6 +185,7 @@ extern "C" pfast_status pfast_fsm3d_noalloc(const double* vp, double* U, int src
         a.sp.inv2[k] = 1.0 / dd[k] / dd[k];
     }
     a.sp.ex = exact_grid3(dd);
+    a.prune_limit = forward_prune_limit(dd, check.largest());
     a.tol_abs = kConvTol;
     a.ntiles = ntiles;
     a.dirty = d_dirty;

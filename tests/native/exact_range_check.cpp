@@ -137,5 +137,36 @@ int main() {
         }
         report("adj_marking", n, wrong + (skipped < n / 8));
     }
+    {   // marking, 3D forward: the same for a neighbour's change (its axis' other neighbour may hide it),
+        // on grids of any spacing and far more steps from the source than a grid has
+        long long n = 0, wrong = 0, skipped = 0;
+        for (int i = 0; i < 6000000; ++i) {
+            double d[3];
+            const double h = std::pow(10.0, uni(-3.0, 3.0)), ratio = rng() % 2 ? 1.0 : std::pow(10.0, uni(0.0, 7.0));
+            for (double& x : d) x = ratio == 1.0 ? h : h * std::pow(ratio, uni(0.0, 1.0));
+            const double s = std::pow(10.0, uni(-5.0, 0.0)), vmax = (1.0 / s) * (rng() % 2 ? 1.0 : uni(1.0, 100.0));
+            const int limit = forward_prune_limit(d, vmax);
+            const double step = s * *std::min_element(d, d + 3), base = step * std::pow(10.0, rng() % 2 ? uni(0.0, 11.0) : uni(7.0, 9.0));
+            double v[3];
+            for (double& x : v) {
+                const unsigned c = rng() % 8;
+                x = c < 3 ? base * (1.0 + std::pow(10.0, uni(-7.0, 0.0))) : c == 3 ? kUnreached : base + step * uni(0.0, 2.0);
+            }
+            const int a = rng() % 3;
+            const double other = rng() % 2 ? kUnreached : v[a] * uni(0.99999, 1.01);
+            const double x0 = v[a], x1 = rng() % 2 ? x0 * uni(0.9, 1.1) : x0 + step * uni(-2.0, 2.0);
+            v[a] = std::min(x0, other);
+            double vn = eik3_ref(v[0], v[1], v[2], s, d);
+            if (rng() % 4 == 0) vn *= uni(0.9, 1.0);
+            vn = std::min(vn, kUnreached);
+            v[a] = std::min(x1, other);
+            const double q = eik3_ref(v[0], v[1], v[2], s, d);
+            if (x0 >= 0.0 && x1 >= 0.0 && vn >= 0.0 && !forward_depends_exact(forward_change(x0, x1, limit), vn))
+                wrong += !same(std::min(vn, q), vn), ++skipped;
+            ++n;
+        }
+        report("fwd_marking", n, wrong + (skipped < n / 50));
+        std::printf("%lld of %lld without a dependency\n", skipped, n);
+    }
     return bad ? 1 : 0;
 }

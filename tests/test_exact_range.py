@@ -27,7 +27,7 @@ def check_lines(tmp_path_factory):
     return subprocess.run([exe], capture_output=True, text=True, timeout=300).stdout.splitlines()
 
 
-@pytest.mark.parametrize("name", ["eik3_slowness", "eik2_slowness", "adj_axis_any_time", "adj_marking"])
+@pytest.mark.parametrize("name", ["eik3_slowness", "eik2_slowness", "adj_axis_any_time", "adj_marking", "fwd_marking"])
 def test_updates_match_the_expressions(check_lines, name):
     line = [x for x in check_lines if x.split()[1] == name]
     assert line and line[0].startswith("ok "), check_lines
@@ -102,3 +102,26 @@ def test_adjoints_of_fields_with_any_time(v):
     L = np.empty(T2.shape)
     e = pg.Tadjoint_fsm2d(L, T2, tobs, rec, n2, src, srnum, 0, 40, 20.0, 16.7, *T2.shape)
     assert same_or_nan(L, L0) and e == e0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("d,v0,contrast", [((19000.0, 17.5, 0.0027), 1e-175, 1.0), ((0.0027, 17.5, 19000.0), 1e-175, 1.0),
+                                           ((20.0, 20.0, 20.0), None, 1e8), ((5.0, 100.0, 20.0), None, 1e6)])
+def test_solves_far_from_the_source_in_steps(d, v0, contrast):
+    """Uneven spacings and contrasts at which times are 1e7 steps and more: which tiles are skipped must
+    still not show in the bits."""
+    import pfast_gb300 as pg
+    from oracle import port
+    rng = np.random.default_rng(941)
+    shape = nz, nr, nc = 36, 30, 41
+    vp = 1500.0 + 2500.0 * rng.random(shape) if v0 else 1000.0 * np.exp(rng.uniform(0.0, np.log(contrast), shape))
+    if v0:
+        vp[rng.random(shape) < 0.05] = v0
+    else:
+        vp[rng.random(shape) < 0.3] = 1.0     # slow bodies around fast nodes
+    src = np.stack([rng.integers(0, n, 20) for n in (nr, nc, nz)], 1).astype(np.int32)
+    for s in range(len(src)):
+        U0, _ = port.fsm3d(vp, src, s, 100, *d)
+        U = np.empty_like(vp)
+        pg.fsm3d(vp, U, src, s, 100, *d, nr, nc, nz)
+        assert bits_equal(U, U0), s
