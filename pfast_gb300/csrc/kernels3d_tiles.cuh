@@ -166,11 +166,11 @@ __device__ __forceinline__ float eik3_fast(float a, float b, float c, float s, c
     return q1 <= b ? q1 : (q2 <= a ? q2 : q3);
 }
 
-// Square root by the hardware approximation (PTX sqrt.approx.ftz.f32, a few ulps): the FP32 bulk
+// Square root by the hardware approximation (PTX sqrt.approx.f32, a few ulps): the FP32 bulk
 // result is only the starting point of the FP64 polish.
 __device__ __forceinline__ float sqrt_approx(float x) {
     float r;
-    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
 
