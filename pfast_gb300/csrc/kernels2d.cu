@@ -96,7 +96,9 @@ __device__ __forceinline__ double adj2_plain(double T0, double Txp, double Txm, 
     const long long inf = dbits(kInf);   // T >= INF on the bit patterns (T >= 0)
     if (dbits(Txp) >= inf || dbits(T0) >= inf || dbits(Txm) >= inf || dbits(Tzp) >= inf || dbits(Tzm) >= inf)
         return 0.0;
-    if (K.ex.quick) {
+    const unsigned most = most_of(most_of(upper_of(T0), upper_of(Txp)),
+                                  most_of(upper_of(Txm), most_of(upper_of(Tzp), upper_of(Tzm))));
+    if (K.ex.quick && adj_ordinary(most)) {
         double ex, ez, nx, nz;
         adj_axis_exact(T0, Txp, Txm, Lxp, Lxm, K.ex.x, ex, nx);
         adj_axis_exact(T0, Tzp, Tzm, Lzp, Lzm, K.ex.z, ez, nz);

@@ -265,7 +265,9 @@ __device__ __forceinline__ double adj3_plain(double T0, double Txp, double Txm, 
                                              double Tzp, double Tzm, double Lxp, double Lxm, double Lyp,
                                              double Lym, double Lzp, double Lzm, const Spacing3& sp) {
     if (unreached64(T0, Txp, Txm, Typ, Tym, Tzp, Tzm)) return 0.0;
-    if (sp.ex.quick) {
+    const unsigned most = most_of(most_of(most_of(upper_of(T0), upper_of(Txp)), most_of(upper_of(Txm), upper_of(Typ))),
+                                  most_of(upper_of(Tym), most_of(upper_of(Tzp), upper_of(Tzm))));
+    if (sp.ex.quick && adj_ordinary(most)) {
         double ex, ey, ez, nx, ny, nz;
         adj_axis_exact(T0, Txp, Txm, Lxp, Lxm, sp.ex.axis[0], ex, nx);
         adj_axis_exact(T0, Typ, Tym, Lyp, Lym, sp.ex.axis[1], ey, ny);
@@ -1272,26 +1274,27 @@ __global__ void __launch_bounds__(kWarps3 * 32) sweep3d_kernel(const Sweep3Args 
 }
 
 // ----------------------------------------------------------- dataflow schedule
-// One launch per phase.  Each block takes instances (sources) from a queue and runs the
-// whole solve of one instance: outer iterations of eight sweep orders until the instance's
+// One launch per phase.  Each block or cluster of blocks takes instances (sources) from a queue and
+// runs the whole solve of one instance: outer iterations of eight sweep orders until the instance's
 // convergence test passes or maxiter iterations ran.  Within an outer iteration the items
 // (sweep order o, tile x) form the dataflow graph of dataflow3.h: an item is ready once the
 // items it reads from are done, so the sweeps of different orders overlap and no barrier
-// separates tile diagonals or orders.  Per tile, two 4-bit counters in shared memory (one
-// per order parity, four tiles per word) count the item's missing dependencies; a ring of
-// ready items in shared memory feeds the block's warps.
+// separates tile diagonals or orders.  Counters in shared memory hold the items' missing
+// dependencies, and a ring of ready items there feeds the warps (dataflow_queue.h; a cluster's lie in
+// the shared memory of its first block).
 //   A warp takes about its share of the ready items (1 to 32, one per lane) and reads their
 //   lock words.  A tile that is not due in the item's order (tile locking) completes at once,
 //   lane by lane; of the due items the warp processes one (process_tile) and returns the
 //   others to the ring for idle warps.  Completing (o, x) re-arms x's counter of parity o for
 //   order o + 2 (clusters keep all eight orders' counters instead) and decrements its dependents'
-//   counters; those that reach zero join the ring.
-//   The iteration ends when all 8 x ntiles items completed; the block then tests convergence
-//   as the per-diagonal schedule's reduction does (any tile moved / any tile still due).
+//   counters; those that reach zero join the ring or stay with the lane.
+//   The iteration ends when all 8 x ntiles items completed; the block or cluster then tests
+//   convergence as the per-diagonal schedule's reduction does (any tile moved / any tile still due).
 // Every tile processing sees exactly the neighbour values and lock words it sees in the
-// per-diagonal schedule, so both schedules give the same bits.  All waits are on this block's
-// own shared memory (no block waits for another) and are bounded: a block that sees no
-// progress for two seconds sets *err, records the instance as not converged and exits.
+// per-diagonal schedule, so both schedules give the same bits.  All waits are on the shared memory
+// of the own block or of the own cluster's first block (the blocks of a cluster run at the same time;
+// no block or cluster waits for another) and are bounded: one that sees no progress for two seconds
+// sets queue[1], records the instance as not converged and exits.
 // result[inst] = iterations | 1 << 30 when not converged.  A.iter is the first iteration's
 // number: a solve continued from per-diagonal iterations counts on from them.
 // shared-memory copy of a model's arguments (multi-grid launches)
