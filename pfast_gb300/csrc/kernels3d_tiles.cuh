@@ -61,8 +61,9 @@ template <> struct Traits<kAdjPolish64>  { using Real = double; using Aux = doub
 //                 or 16 (adjoint) warps instead of 11, at more instructions a step (ncu, first
 //                 version: 355 / 442 warp instructions per tile and step against 247 / 400).  For the
 //                 forward with one block per source on large grids, whose many ready tiles keep 24 warps
-//                 busy (256 sources of 256 x 256 x 128, 8192 tiles: 303 ms against 317 with boxes; 152
-//                 sources of 128 x 128 x 100, 1600 tiles: 35.1 against 30.9); for the adjoint with one
+//                 busy (256 sources of 256 x 256 x 128, 8192 tiles: 307 ms against 323 with boxes; 152
+//                 sources of 4900 tiles: 117.5 / 120.2, 3500 tiles: 82.9 / 82.3, 3000 tiles: 70.2 / 64.3,
+//                 128 x 128 x 100, 1600 tiles: 35.5 / 31.0); for the adjoint with one
 //                 block per source (the 256 sources: 243 against 292 with a field box) or up to three on
 //                 grids of 1024 tiles or more.
 //   kFormBoxes    (adjoint polish in clusters otherwise) field and traveltime in boxes.

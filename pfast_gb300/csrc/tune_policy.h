@@ -66,13 +66,13 @@ inline int tune_pick(const TuneEntry* e, unsigned allowed, int nact, int sms) {
 // share its queue, where the instances alone would leave SMs idle.  A cluster size is wanted
 // while the clusters need about one block per SM (the hardware packs the blocks of a cluster
 // densely, so beyond that some SMs hold several and others none) and the grid has tiles for them.
-// Measured (ms of a mixed gradient of 128 x 128 x 64 nodes, blocks per source): 64 sources 95 (1), 81
-// (2); 40 sources 71 (2), 70 (4); 100 sources 99 (1), 103 (2); plain, 96 x 96 x 48: 16 sources 602
-// (1), 331 (2), 202 (4), 175 (8), 287 (16); 40 sources 331 (2), 299 (4).
+// Measured (gradients on smooth random models, ms, blocks per source in brackets; runs differ by up to 7 %
+// with where the hardware places the clusters): mixed, 128 x 128 x 64 nodes: 64 sources 82 (1), 65 (2); 40
+// sources 57 (2), 51 (3), 59 (4); plain, 96 x 96 x 48: 16 sources 494 (1), 327 (2), 186 (4), 137 (8);
+// 40 sources 338 (2), 239 (3), 236 (4).
 // Any size, not powers of two alone, which left up to half of the SMs idle just above a step
-// (plain gradient of 128 x 128 x 100: 21 sources 628 ms with 4 blocks, 395 with 7; 96 x 96 x 48: 42
-// sources 314 (2), 223 (3); mixed, 128 x 128 x 100: 13 sources 53 (8), 46 (15)).  Sizes of 9 to 15 only on
-// grids of 100 tiles a block: 12 sources of 96 x 96 x 48 (432 tiles) took 126 ms with 8 blocks, 162 with 13.
+// (plain, 128 x 128 x 100: 21 sources 640 ms (4), 409 (7); 96 x 96 x 48: 42 sources 321 (2), 228 (3)).
+// Sizes of 9 to 15 only on grids of 100 tiles a block: 12 sources of 96 x 96 x 48 (432 tiles) 130 (8), 145 (12).
 constexpr int kMaxCluster = 16;
 
 inline bool cluster_wanted(int cs, bool plain, int nact, int ntiles, int sms) {
@@ -82,28 +82,31 @@ inline bool cluster_wanted(int cs, bool plain, int nact, int ntiles, int sms) {
 // Warps per block of a cluster.  Few: the ready tiles of a source are few as well, and what
 // bounds them is the latency of one tile, so they should lie on different SM sub-partitions, and
 // idle warps only poll the queue.  The plain kinds saturate a sub-partition's FP64 pipe with one warp.
-// Measured (ms; warps per block): one shot of 128 x 128 x 64 nodes, plain, 16 blocks: 117 (2),
-// 88 (4), 102 (6), 171 (11, all that fit); 16 sources of 96 x 96 x 48, plain gradient, 8 blocks: 208
-// (2), 175 (4), 235 (6), 361 (11); 24 sources of 155 x 75 x 101, mixed forward, 8 blocks: 72 (2),
-// 49 (4), 48 (6), 54 (8); 9 sources of 90 x 71 x 53, mixed gradient, 16 blocks: 40.1 (2), 39.9 (4),
-// 41.3 (6); 64 sources of 128 x 128 x 64, mixed gradient, 2 blocks: 97 (8), 83 (12), 81 (24).
+// Measured (ms, warps per block in brackets): one shot of 128 x 128 x 64 nodes, plain, 16 blocks: 88 (2),
+// 67 (4), 73 (6), 119 (11, all that fit); 16 sources of 96 x 96 x 48, plain gradient, 8 blocks: 179 (2),
+// 138 (4), 194 (6); 24 sources of 155 x 75 x 101, mixed forward, 6 blocks: 49 (2), 32 (4), 35 (6); 9 sources
+// of 90 x 71 x 53, mixed gradient, 16 blocks: 22 (2), 25 (4), 25 (6); 30 sources of 128 x 128 x 64, mixed
+// gradient, 5 blocks: 61 (4), 55 (6); 64 sources, 2 blocks: 109 (4), 89 (6), 75 (8), 64 (12).
 inline int cluster_warps(int cs, bool plain) {
     if (plain || cs >= 8) return 4;
     return cs >= 4 ? 6 : 12;
 }
 
 // The candidate of a phase that has not been timed, among `allowed` (tune_allowed): the dataflow
-// kernel, except where one launch per tile diagonal is ahead:
+// kernel, except where one launch per tile diagonal is ahead (the tile counts of both lines are those
+// measured on 152 SMs):
 // - the plain kinds, whose FP64 pipe needs one warp per SM sub-partition only, with at most three
 //   blocks per instance that leave SMs idle, where a diagonal holds enough tiles for all SMs.
-//   Gradients, ms per diagonal / dataflow (tiles a diagonal): 84 sources of 96 x 96 x 48 393 / 552
-//   (1450), 61 of 226 x 35 x 68 723 / 924 (1480), 49 of 100 x 171 x 47 738 / 790-880 (1440), 64 of
-//   96 x 96 x 48 352 / 333 (1110), 84 of 64 x 64 x 32 165 / 151 (670); one block each from three
-//   quarters of the SMs on: 119 of 67 x 137 x 26 504 / 427 (2100), 123 of 104 x 125 x 25 579 / 493
-//   (2200); two or three each from all SMs on: forward of 79 of 37 x 126 x 108 575 / 472 (1590);
-// - the FP32 bulk kinds with one block per instance where a diagonal holds many tiles (256 sources
-//   of 256 x 256 x 128, 30,000 tiles a diagonal: forward 165 / 176, adjoint 242 / 250; 256
-//   sources of 96 x 96 x 48, 4,400: 12.3 / 8.8, 14.6 / 11.6).
+//   Gradients, ms per diagonal / dataflow (tiles a diagonal): 84 sources of 96 x 96 x 48 404 / 562
+//   (1450), 61 of 226 x 35 x 68 744 / 953 (1480), 49 of 100 x 171 x 47 758 / 787 (1440), 64 of
+//   96 x 96 x 48 362 / 342 (1110), 84 of 64 x 64 x 32 170 / 154 (670); one block each from three
+//   quarters of the SMs on: 119 of 67 x 137 x 26 517 / 433 (1730), 123 of 104 x 125 x 25 593 / 500
+//   (2200); two or three each from all SMs on: forward of 79 of 37 x 126 x 108 320 / 291 (1590).  On
+//   rough models (every node at random) the per-diagonal launches stay ahead a little longer;
+// - the FP32 bulk kinds with one block per instance where a diagonal holds many tiles (256 sources,
+//   forward and adjoint ms per diagonal / dataflow: 256 x 256 x 128, 30,000 tiles a diagonal, 172 / 184 and
+//   245 / 250; 200 x 200 x 100, 20,400: 94 / 91, 127 / 127; 176 x 176 x 100, 16,600: 71 / 66, 90 / 85;
+//   128 x 128 x 64, 7,700: 24 / 20, 33 / 29).  The line lies at 16,384, a little below where the two meet.
 // cluster: blocks per instance of the dataflow kernel; plain / fp32: the phase's kind (neither: polish).
 inline int untuned_pick(unsigned allowed, bool plain, bool fp32, int cluster, int nact, long long ntiles, int ndiag,
                         int sms) {
