@@ -373,7 +373,7 @@ def main():
     # resident sources sharing the slowness / traveltime lines in L2.
     traffic_ratios = {("fwd64", "diagonal 4x8x32"): 1.09, ("fwd64", "persistent 4x8x32"): 0.75,
                       ("adj64", "persistent 4x8x32"): 0.92, ("fwd32", "diagonal 4x8x32"): 1.23,
-                      ("adj32", "diagonal 4x8x32"): 2.59}
+                      ("adj32", "diagonal 4x8x32"): 2.58}
     ratio = traffic_ratios.get((dom, cand))
     traffic = alg_bytes / launches_dom * ratio if (ratio and launches_dom) else None
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
