@@ -474,6 +474,7 @@ pfast_status forward3d_batch(pfast_ctx* ctx, const pfast_survey3d* sv, int b0, i
     a.src_kij = sv->d_src_kij + 3 * b0;
     a.src_r2 = ctx->near_radius * ctx->near_radius;
     a.prune_limit = forward_prune_limit(a.sp.d, ctx->vmax);
+    a.tiny_steps = has_tiny_steps(a.sp, ctx->vmax);
     const long long* src_lin = sv->d_src_lin + b0;
     int dummy_nc = 0;
     int* nc_ptr = st ? &st->not_converged : &dummy_nc;

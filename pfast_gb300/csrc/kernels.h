@@ -42,6 +42,7 @@ struct Sweep3Args {
                               // adjoint: relative to 1 + |lambda|)
     unsigned long long* work; // per instance: nodes of the tiles processed (executed node updates); may be null
     int shape;                // tile shape: 0 = 4x8x32, 1 = 8x4x32 (common.cuh: TileShape)
+    int tiny_steps;           // FP32 bulk forward: some step of the model is below 2^-37 s
     int prune_limit;          // plain forward: forward_prune_limit (exact_arith.h) of the grid and the model
     int vec_rows;             // rows of the field (and of the FP32 adjoint's traveltime) start on 16-byte
                               // boundaries: nc a multiple of 16 / element size, 16-byte aligned fields;
@@ -50,6 +51,9 @@ struct Sweep3Args {
                               // iteration (instead of iter), dyn[1] = active instances (blocks with
                               // blockIdx.y >= dyn[1] exit); null: iter and the grid
 };
+
+// Sweep3Args::tiny_steps of a model whose largest velocity is vmax (isotropic grids).
+inline int has_tiny_steps(const Spacing3& sp, double vmax) { return !(sp.d[0] / vmax >= 0x1p-37); }
 
 // Tile-diagonal table for a grid: tiles (bk, bi, bj) in flipped coordinates with
 // bk+bi+bj = d, packed bk | bi<<10 | bj<<20.

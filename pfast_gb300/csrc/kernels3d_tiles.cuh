@@ -168,10 +168,15 @@ __device__ __forceinline__ float eik3_fast(float a, float b, float c, float s, c
 }
 
 // Square root by the hardware approximation (PTX sqrt.approx.f32, a few ulps): the FP32 bulk
-// result is only the starting point of the FP64 polish.
+// result is only the starting point of the FP64 polish.  Arguments below the smallest normal number
+// occur only where some node's step is below 2^-37 s (Sweep3Args::tiny_steps: a discriminant that is
+// not 0 is at least 2^-48 of the step squared); elsewhere the form that flushes them gives the same bits
+// with fewer instructions (FP32 forward of 256 sources of 256 x 256 x 128, per diagonal: 91.8 and 89 ms).
+template <bool TINY>
 __device__ __forceinline__ float sqrt_approx(float x) {
     float r;
-    asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+    if constexpr (TINY) asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+    else asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
 
@@ -184,6 +189,7 @@ __device__ __forceinline__ float sqrt_approx(float x) {
 // union of the paths with divergence bookkeeping anyway.  The selected value is the same
 // expression as in the branching form, bit for bit (candidates from unreached neighbours may
 // be inf or NaN; they are never selected).
+template <bool TINY>
 __device__ __forceinline__ float eik3_fast_iso(float a, float b, float c, float sh) {
     const float lo = fminf(a, b), hi = fmaxf(a, b);
     const float c0 = fminf(lo, c), mid = fmaxf(lo, c);
@@ -191,10 +197,10 @@ __device__ __forceinline__ float eik3_fast_iso(float a, float b, float c, float 
     const float q1 = c0 + sh;
     const float B = b0 - c0;
     const float D = fmaf(2.0f * sh, sh, -B * B);
-    const float q2 = (D >= 0.f) ? fmaf(0.5f, B + sqrt_approx(D), c0) : (float)kInf;
+    const float q2 = (D >= 0.f) ? fmaf(0.5f, B + sqrt_approx<TINY>(D), c0) : (float)kInf;
     const float A = a0 - c0, AB = A - B;
     const float D3 = fmaf(3.0f * sh, sh, -fmaf(AB, AB, fmaf(A, A, B * B)));
-    const float q3 = (D3 >= 0.f) ? fmaf(1.0f / 3.0f, (A + B) + sqrt_approx(D3), c0) : (float)kInf;
+    const float q3 = (D3 >= 0.f) ? fmaf(1.0f / 3.0f, (A + B) + sqrt_approx<TINY>(D3), c0) : (float)kInf;
     return q1 <= b0 ? q1 : (q2 <= a0 ? q2 : q3);
 }
 
@@ -969,7 +975,9 @@ __device__ __forceinline__ void process_tile(const Sweep3Args& A, const int inst
                 }
                 // field values are >= +0 or +inf: fminf is the reference's MIN here
                 const float xa = fminf(xd, xu), yb = fminf(yd, yu), zc = fminf(zd, zu), s = sp_[t];
-                nv = fminf(old, A.sp.iso ? eik3_fast_iso(xa, yb, zc, s * A.sp.df[0]) : eik3_fast(xa, yb, zc, s, A.sp));
+                nv = fminf(old, !A.sp.iso      ? eik3_fast(xa, yb, zc, s, A.sp)
+                                : A.tiny_steps ? eik3_fast_iso<true>(xa, yb, zc, s * A.sp.df[0])
+                                               : eik3_fast_iso<false>(xa, yb, zc, s * A.sp.df[0]));
                 ch = upd & (nv < old);
                 feeds = nv < fmaxf(fmaxf(inK ? zu : 0.0f, inI ? yu : 0.0f), inJ ? xu : 0.0f);
             } else {

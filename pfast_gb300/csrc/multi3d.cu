@@ -213,6 +213,7 @@ pfast_status eval_group(pfast_ctx* ctx, std::vector<Model>& ms, const pfast_opti
         Sweep3Args a = survey_sweep_args(ms[m].sv);
         a.fstride = ms[m].N;
         a.prune_limit = forward_prune_limit(a.sp.d, check[m].largest());
+        a.tiny_steps = has_tiny_steps(a.sp, check[m].largest());
         return a;
     };
     auto all_active = [&]() {
