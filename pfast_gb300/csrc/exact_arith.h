@@ -233,10 +233,10 @@ inline ExactGrid3 exact_grid3(const double d[3]) {
 
 // |v| in [2^-34, 2^34]: traveltimes for which every quotient above stays in its range
 PFAST_HD bool in_range(double v) { return (unsigned)(exponent_of(v) - 989) <= 67u; }
-// Slownesses below 2^34 as well: the terms with s*s enter the same sums, and where they overflow (from
-// about 2^450 on, velocities below 1e-136 of an impermeable body) the one-step quotient of an infinite
-// numerator is NaN, where x / d is infinite and the minimum with the node's value drops it.
-PFAST_HD bool slow_in_range(double s) { return exponent_of(s) <= 1056; }
+// Slownesses below 2^58 as well (the root of the terms with s*s is then below 2^119): where those overflow
+// (from about 2^450 on, velocities below 1e-136 of an impermeable body) the one-step quotient of an
+// infinite numerator is NaN, where x / d is infinite and the minimum with the node's value drops it.
+PFAST_HD bool slow_in_range(double s) { return exponent_of(s) <= 1080; }
 
 // Magnitude of a value >= +0 as FP32 (truncated; +inf and beyond give a huge finite value).
 PFAST_HD float approx32(double v) {
@@ -277,7 +277,10 @@ PFAST_HD double eik3_tail_ref(double a, double b, double c, double da, double db
 // division: per warp at most 2 + 13 + 21 + 13 FP64 instructions (spacings of few bits), where the
 // expressions as they stand take about 185.  96 x 96 x 48 nodes, 16 sources, one launch per tile
 // diagonal: forward sweeps 210 -> 140 ms with FP64 tails and the library's root.
-template <bool ISO, bool FAST>
+// MIN: only the minimum with a node's value (at most the unreached one) counts, so that for a slowness
+// out of range, whose solutions are all 2^37 or more (spacings above 2^-20), any larger value does: a body
+// that lets nothing through does not run the expressions beside the other lanes' short form.
+template <bool ISO, bool FAST, bool MIN = false>
 PFAST_HD double eik3_exact(double x, double y, double z, double s, const ExactGrid3& g, const double* inv2) {
     double a = x, b = y, c = z, t;
     int ka = 0, kb = 1, kc = 2, k;
@@ -291,6 +294,7 @@ PFAST_HD double eik3_exact(double x, double y, double z, double s, const ExactGr
     const double db = pick(kb, g.axis[0].d, g.axis[1].d, g.axis[2].d);
     const bool ainf = bits_of(a) >= 0x7ff0000000000000ll;
     if (!(in_range(b) && (is_zero(c) || in_range(c)) && (ainf || in_range(a)) && slow_in_range(s))) {
+        if (MIN && !slow_in_range(s)) return INFINITY;
         const double da = pick(ka, g.axis[0].d, g.axis[1].d, g.axis[2].d);
         return eik3_tail_ref(a, b, c, da, db, dc, pick(ka, inv2[0], inv2[1], inv2[2]),
                              pick(kb, inv2[0], inv2[1], inv2[2]), pick(kc, inv2[0], inv2[1], inv2[2]), s);

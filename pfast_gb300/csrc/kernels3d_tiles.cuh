@@ -117,9 +117,9 @@ __host__ __device__ constexpr int warp_smem_bytes() {
 __device__ __forceinline__ double eik3_plain(double a, double b, double c, double s, const Spacing3& sp) {
     if (sp.ex.quick) {
         if (sp.ex.iso)
-            return sp.ex.fast ? eik3_exact<true, true>(a, b, c, s, sp.ex, sp.inv2)
-                              : eik3_exact<true, false>(a, b, c, s, sp.ex, sp.inv2);
-        return eik3_exact<false, false>(a, b, c, s, sp.ex, sp.inv2);
+            return sp.ex.fast ? eik3_exact<true, true, true>(a, b, c, s, sp.ex, sp.inv2)
+                              : eik3_exact<true, false, true>(a, b, c, s, sp.ex, sp.inv2);
+        return eik3_exact<false, false, true>(a, b, c, s, sp.ex, sp.inv2);
     }
     double da = sp.d[0], db = sp.d[1], dc = sp.d[2];
     double ia = sp.inv2[0], ib = sp.inv2[1], ic = sp.inv2[2];

@@ -33,8 +33,9 @@ def test_updates_match_the_expressions(check_lines, name):
     assert line and line[0].startswith("ok "), check_lines
 
 
-# velocities whose slowness squares to infinity, to just below it, and is itself infinite
-SLOW = [1e-130, 1e-140, 1e-152, 1e-160, 1e-300, 5e-324]
+# velocities whose slowness is on either side of 2^58, squares to infinity, to just below it, and is itself
+# infinite
+SLOW = [1e-9, 4e-18, 3e-18, 1e-60, 1e-130, 1e-140, 1e-152, 1e-160, 1e-300, 5e-324]
 
 
 @pytest.mark.gpu
