@@ -171,7 +171,7 @@ __device__ __forceinline__ float eik3_fast(float a, float b, float c, float s, c
 // result is only the starting point of the FP64 polish.  Arguments below the smallest normal number
 // occur only where some node's step is below 2^-37 s (Sweep3Args::tiny_steps: a discriminant that is
 // not 0 is at least 2^-48 of the step squared); elsewhere the form that flushes them gives the same bits
-// with fewer instructions (FP32 forward of 256 sources of 256 x 256 x 128, per diagonal: 91.8 and 89 ms).
+// with fewer instructions (FP32 forward of 256 sources of 256 x 256 x 128, per diagonal: 91.8 and 90.2 ms).
 template <bool TINY>
 __device__ __forceinline__ float sqrt_approx(float x) {
     float r;
